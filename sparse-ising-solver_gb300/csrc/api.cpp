@@ -423,8 +423,7 @@ int ensure_common(sbx_ctx *ctx, const SolveDims &d, int64_t total_steps, int32_t
     return SBX_OK;
 }
 
-constexpr int64_t kRandChunk = 31 * 32;   // outputs per init thread
-constexpr int kRandBits = 40;             // jump matrices kept: 2^40 threads
+constexpr int kRandBits = 44;   // jump matrices kept: 2^44 rounds of outputs
 
 // x, y of one or more instances from their seeds' glibc rand() streams
 // (src/ising.cu:91-95, src/ising_tsp.cu:55-59), one launch.  Padded agents
@@ -437,23 +436,32 @@ int init_instances(sbx_ctx *ctx, const SolveDims &d, std::vector<RandInst> &inst
     cudaStream_t s = ctx->stream;
     if (!w.rjump_ready) {
         std::vector<uint32_t> mats;
-        rand_jump_matrices(kRandChunk, kRandBits, mats);
+        rand_jump_matrices(rand_round(), kRandBits, mats);
         CK(grow(w.rjump, w.cap_rj, mats.size()));
         CK(cudaMemcpy(w.rjump, mats.data(), mats.size() * 4, cudaMemcpyHostToDevice));
         w.rjump_ready = true;
     }
+    int64_t all = 0;
+    bool padded = false;
+    for (auto &I : inst) {
+        all += I.n * I.A * (tsp ? 1 : 2);
+        padded |= I.A != d.Ap;
+    }
+    const int shift = rand_chunk_shift(all);
+    const int64_t chunk = rand_round() << shift;
     int64_t threads = 0;
     for (auto &I : inst) {
         I.thread_base = threads;
         const int64_t outputs = I.n * I.A * (tsp ? 1 : 2);
-        threads += (outputs + kRandChunk - 1) / kRandChunk;
+        threads += (outputs + chunk - 1) / chunk;
     }
     const size_t es = prec_bytes(d.prec), nst = (size_t)d.n * d.Ap;
-    CK(cudaMemsetAsync(w.x, 0, nst * es, s));
-    CK(cudaMemsetAsync(w.y, 0, nst * es, s));
+    // without padded agents the init writes every x (not TSP) and y
+    if (padded || tsp) CK(cudaMemsetAsync(w.x, 0, nst * es, s));
+    if (padded) CK(cudaMemsetAsync(w.y, 0, nst * es, s));
     CK(grow(w.rinst, w.cap_rinst, inst.size()));
     CK(cudaMemcpyAsync(w.rinst, inst.data(), sizeof(RandInst) * inst.size(), cudaMemcpyHostToDevice, s));
-    CK(launch_rand_init(d.prec, w.x, w.y, d.Ap, tsp, kRandChunk, w.rjump, w.rinst, (int)inst.size(),
+    CK(launch_rand_init(d.prec, w.x, w.y, d.Ap, tsp, shift, w.rjump, w.rinst, (int)inst.size(),
                         threads, slot, s));
     // the instance table must outlive the async copy
     CK(cudaStreamSynchronize(s));
