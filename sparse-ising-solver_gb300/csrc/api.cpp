@@ -778,6 +778,7 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
         return fail(ctx, SBX_ERR_UNSUPPORTED, "trace / target: streaming kernel only");
     int rc = ensure_common(ctx, d, total, p->J.nchunks);
     if (rc) return rc;
+    if (!p->J.integer) CK(grow(ctx->w.cutrow, ctx->w.cap_cutrow, (size_t)cut_scratch_rows(d, p->J) * d.Ap));
     if ((rc = upload_coef(ctx, d, total))) return rc;
     if ((rc = init_state(ctx, d, pr->seed, false))) return rc;
 
@@ -1838,7 +1839,7 @@ int sbx_destroy(sbx_ctx *ctx)
     void *ptrs[] = {w.x, w.y, w.x2, w.S[0], w.S[1], w.Wp, w.fin, w.chg, w.newmask, w.stab, w.bif,
                     w.prev, w.ctl, w.wincount, w.visits, w.ab, w.sched, w.eacc, w.cut, w.trace,
                     w.tours, w.valid, w.rjump, w.coef32, w.coef64, w.part, w.rinst, w.trace_t0,
-                    w.btrace, w.hcount, w.gbar, w.stats};
+                    w.btrace, w.hcount, w.gbar, w.stats, w.cutrow};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     free_batch(ctx);   // (destroys the cached graph when a batch was packed)

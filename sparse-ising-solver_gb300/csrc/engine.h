@@ -119,6 +119,7 @@ struct Work {
     unsigned long long *eacc = nullptr;   // per-agent cut accumulators
     double *cut = nullptr;                // per-agent cuts
     double *stats = nullptr;              // k_stats output, 7 per problem
+    double *cutrow = nullptr;             // non-integer cuts: a block of rows' halves [row][Ap]
     TraceRec *trace = nullptr;            // per-window records; trace_t0: loop start
     long long *trace_t0 = nullptr;
     double *btrace = nullptr;             // batched: best cut [window][instance]
@@ -130,7 +131,7 @@ struct Work {
     size_t cap_x = 0, cap_y = 0, cap_x2 = 0, cap_S0 = 0, cap_S1 = 0, cap_Wp = 0, cap_fin = 0,
            cap_chg = 0, cap_new = 0, cap_stab = 0, cap_bif = 0, cap_prev = 0, cap_ctl = 0,
            cap_win = 0, cap_visits = 0, cap_ab = 0, cap_sched = 0, cap_eacc = 0, cap_cut = 0,
-           cap_trace = 0, cap_t0 = 0, cap_btrace = 0, cap_tours = 0, cap_valid = 0, cap_rj = 0, cap_c32 = 0, cap_c64 = 0, cap_part = 0, cap_rinst = 0, cap_hcount = 0, cap_gbar = 0, cap_stats = 0;
+           cap_trace = 0, cap_t0 = 0, cap_btrace = 0, cap_tours = 0, cap_valid = 0, cap_rj = 0, cap_c32 = 0, cap_c64 = 0, cap_part = 0, cap_rinst = 0, cap_hcount = 0, cap_gbar = 0, cap_stats = 0, cap_cutrow = 0;
     bool rjump_ready = false;
 };
 
@@ -212,6 +213,8 @@ cudaError_t launch_chunk(const SolveDims &d, const DevCsr &J, Work &w, cudaStrea
                          int *launches, cudaEvent_t *evs = nullptr);
 cudaError_t launch_cut(const SolveDims &d, const DevCsr &J, Work &w, const uint32_t *plane,
                        cudaStream_t s, int *launches);
+// Rows of w.cutrow that launch_cut needs (0 for integer weights).
+int64_t cut_scratch_rows(const SolveDims &d, const DevCsr &J);
 // count plain (non-window) steps of the solve's kind at step 0: the
 // autotuner's timing runs.
 cudaError_t launch_plain_steps(const SolveDims &d, const DevCsr &J, Work &w, int count, cudaStream_t s);

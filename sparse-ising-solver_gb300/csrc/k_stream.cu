@@ -3,6 +3,7 @@
 // bookkeeping kernels and the exact cut.
 #include "k_step.cuh"
 
+#include <algorithm>
 #include <cfloat>
 
 namespace sbx {
@@ -304,12 +305,127 @@ cudaError_t launch_trace_start(Work &w, cudaStream_t s)
 
 namespace {
 
-// Integer weights: E_a = sum_r s_r sum_j J_rj s_j exactly (int64); the
-// reference's FP64 sum of halves (src/kernels.cu:360-400) equals 0.5*E_a
-// exactly, so the cut below is bit-identical to it.
+// +-1 weights: E_a = sum_r s_r sum_j J_rj s_j = nnz - 2 (entries whose term is
+// -1), exactly; the reference's FP64 sum of halves (src/kernels.cu:360-400)
+// equals 0.5 E_a exactly, so the cut below is bit-identical to it.  The
+// entries, not the rows, are shared out (an R-MAT row of thousands of entries
+// walked by one warp took 650 us whatever the rest): WL lanes hold the WL
+// words of an entry (a 32-byte sector of the gathered row at WL = 8), each
+// group of WL lanes walks its own run of entries, and a lane adds the 32
+// agents' terms (the entry's two sign words and its weight's sign XORed) into
+// eight bit planes with full adders, unpacked every 248 entries.  Latency
+// bound (row walk and gather from L2).
+__device__ __forceinline__ void planes_to_bytes(const uint32_t (&p)[8], int k, uint32_t &lo, uint32_t &hi)
+{
+    // byte k of every plane, then an 8x8 bit transpose: byte v of lo (hi) is
+    // the count of agent 8 k + v (8 k + 4 + v)
+    const uint32_t s01 = (uint32_t)k | (((uint32_t)k + 4) << 4);
+    lo = __byte_perm(__byte_perm(p[0], p[1], s01), __byte_perm(p[2], p[3], s01), 0x5410);
+    hi = __byte_perm(__byte_perm(p[4], p[5], s01), __byte_perm(p[6], p[7], s01), 0x5410);
+    uint32_t t;
+    t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
+    lo ^= t ^ (t << 7);
+    t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
+    hi ^= t ^ (t << 7);
+    t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
+    lo ^= t ^ (t << 14);
+    t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
+    hi ^= t ^ (t << 14);
+    t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
+    lo ^= t;
+    hi ^= t >> 4;
+}
+
+constexpr int kCutBatch = 248;   // entries a lane counts in eight planes
+
+template <int WL>
+__global__ void __launch_bounds__(256) k_cut_unit(const int32_t *__restrict__ rowptr,
+                                                  const uint32_t *__restrict__ colw,
+                                                  const uint32_t *__restrict__ plane, int32_t n, int32_t nnz,
+                                                  int32_t W, int32_t run, unsigned long long *eacc)
+{
+    constexpr int G = 32 / WL;
+    __shared__ int s_cnt[WL * 32];
+    for (int i = threadIdx.x; i < WL * 32; i += 256) s_cnt[i] = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ql = lane % WL, q = blockIdx.y * WL + ql;
+    const bool live = q < W;
+    const uint32_t *S = plane + (live ? q : 0);
+    const int64_t g0 = (int64_t)blockIdx.x * 8 * G;
+    const int64_t b0 = (g0 + warp * G + lane / WL) * run;
+    const int64_t e0 = min((int64_t)nnz, b0), e1 = min((int64_t)nnz, b0 + run);
+    if (e0 < e1) {
+        // the row holding entry e0
+        int32_t lo = 0, hi = n;
+        while (hi - lo > 1) {
+            const int32_t mid = (lo + hi) >> 1;
+            if (__ldg(&rowptr[mid]) <= e0) lo = mid;
+            else hi = mid;
+        }
+        int32_t r = lo, rend = __ldg(&rowptr[r + 1]);
+        uint32_t sr = __ldg(&S[(int64_t)r * W]);
+        for (int64_t eb = e0; eb < e1; eb += kCutBatch) {
+            const int64_t ee = min(e1, eb + kCutBatch);
+            uint32_t p[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) p[k] = 0;
+            for (int64_t e = eb; e < ee; e += 4) {
+                uint32_t d[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const uint32_t cw = e + j < ee ? __ldg(&colw[e + j]) : 0u;
+                    d[j] = __ldg(&S[(int64_t)(cw & 0x7fffffffu) * W]) ^ (uint32_t)((int32_t)cw >> 31);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if (e + j < ee) {
+                        if (e + j >= rend) {
+                            do rend = __ldg(&rowptr[++r + 1]);
+                            while (e + j >= rend);
+                            sr = __ldg(&S[(int64_t)r * W]);
+                        }
+                        d[j] ^= sr;
+                    } else {
+                        d[j] = 0u;
+                    }
+                }
+                const uint32_t a1 = fadd(p[0], d[0], d[1]), b1 = fadd(p[0], d[2], d[3]);
+                uint32_t c = fadd(p[1], a1, b1);
+#pragma unroll
+                for (int k = 2; k < 8; k++) {
+                    const uint32_t t = p[k] & c;
+                    p[k] ^= c;
+                    c = t;
+                }
+            }
+            if (live) {
+                // lanes of other groups hold the same agents: start apart
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    uint32_t cl, ch;
+                    planes_to_bytes(p, k, cl, ch);
+#pragma unroll
+                    for (int v = 0; v < 8; v++) {
+                        const int c = (int)(((v < 4 ? cl : ch) >> (8 * (v & 3))) & 0xffu);
+                        if (c) atomicAdd(&s_cnt[ql * 32 + 8 * k + v], c);
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const long long ne = min((int64_t)nnz, (g0 + 8 * G) * run) - min((int64_t)nnz, g0 * run);
+    for (int i = threadIdx.x; i < WL * 32; i += 256) {
+        const int qq = blockIdx.y * WL + i / 32;
+        if (qq < W && ne) atomicAdd(&eacc[qq * 32 + (i & 31)], (unsigned long long)(ne - 2ll * s_cnt[i]));
+    }
+}
+
+// Other integer weights: the same sum in int64, lane = agent.
 __global__ void __launch_bounds__(256) k_cut_int(const int32_t *__restrict__ rowptr,
                                                  const uint32_t *__restrict__ colw,
-                                                 const float *__restrict__ valf, int unit,
+                                                 const float *__restrict__ valf,
                                                  const uint32_t *__restrict__ plane, int64_t n,
                                                  int32_t W, unsigned long long *eacc)
 {
@@ -319,12 +435,10 @@ __global__ void __launch_bounds__(256) k_cut_int(const int32_t *__restrict__ row
     for (int64_t r = (int64_t)blockIdx.y * 8 + warp; r < n; r += (int64_t)gridDim.y * 8) {
         const int32_t e0 = rowptr[r], e1 = rowptr[r + 1];
         long long t = 0;
+#pragma unroll 4
         for (int32_t e = e0; e < e1; e++) {
-            const uint32_t cw = colw[e];
-            const uint32_t word = plane[(int64_t)(cw & 0x7fffffffu) * W + w];
-            const int neg = (word >> lane) & 1u;
-            if (unit) t += (((uint32_t)neg ^ (cw >> 31)) & 1u) ? -1 : 1;
-            else t += neg ? -(long long)valf[e] : (long long)valf[e];
+            const uint32_t word = plane[(int64_t)(colw[e] & 0x7fffffffu) * W + w];
+            t += ((word >> lane) & 1u) ? -(long long)valf[e] : (long long)valf[e];
         }
         const int sr = (plane[r * W + w] >> lane) & 1u;
         acc += sr ? -t : t;
@@ -383,27 +497,45 @@ __global__ void k_cut_finish(const unsigned long long *eacc, int32_t A, double w
     cut[a] = __dmul_rn(-0.5, __dsub_rn(tmp, wsum));
 }
 
-// Non-integer weights: the reference's FP64 order, one agent per thread:
-// row sums in CSR order, halves summed over rows ascending.
-__global__ void k_cut_ordered(const int32_t *__restrict__ rowptr, const uint32_t *__restrict__ colw,
-                              const double *__restrict__ vald, const uint32_t *__restrict__ plane,
-                              int64_t n, int32_t W, int32_t A, double wsum, double *cut)
+// Non-integer weights: the reference's FP64 order, row sums in CSR order,
+// halves summed over rows ascending.  The rows' halves are independent:
+// k_cut_rows computes those of a block of rows into a scratch [row][Ap]
+// (warp per row and 32 agents, the +-1 factors as sign flips), and k_cut_sum
+// adds them in row order, one agent per lane, so only one FP64 addition per
+// row is serial (one thread walking all rows and entries: 5.9 ms for 2,917
+// rows of degree 12).
+__global__ void __launch_bounds__(256) k_cut_rows(const int32_t *__restrict__ rowptr,
+                                                  const uint32_t *__restrict__ colw,
+                                                  const double *__restrict__ vald,
+                                                  const uint32_t *__restrict__ plane, int64_t row0, int64_t rows,
+                                                  int32_t W, double *__restrict__ half)
 {
-    pdl_wait();
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= A) return;
-    const int w = a >> 5, lane = a & 31;
-    double tmp = 0;
-    for (int64_t r = 0; r < n; r++) {
-        double rs = 0;
-        for (int32_t e = rowptr[r]; e < rowptr[r + 1]; e++) {
-            const uint32_t word = plane[(int64_t)(colw[e] & 0x7fffffffu) * W + w];
-            rs = __dadd_rn(rs, __dmul_rn(vald[e], ((word >> lane) & 1u) ? -1.0 : 1.0));
-        }
-        const double sr = ((plane[r * W + w] >> lane) & 1u) ? -1.0 : 1.0;
-        tmp = __dadd_rn(tmp, __dmul_rn(__dmul_rn(rs, sr), 0.5));
+    const int64_t gw = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (gw >= rows * W) return;
+    const int64_t i = gw / W, r = row0 + i;
+    const int w = (int)(gw - i * W);
+    double rs = 0;
+    const int32_t e1 = __ldg(&rowptr[r + 1]);
+#pragma unroll 4
+    for (int32_t e = __ldg(&rowptr[r]); e < e1; e++) {
+        const uint32_t word = __ldg(&plane[(int64_t)(__ldg(&colw[e]) & 0x7fffffffu) * W + w]);
+        const double v = __ldg(&vald[e]);
+        rs = __dadd_rn(rs, ((word >> lane) & 1u) ? -v : v);
     }
-    cut[a] = __dmul_rn(-0.5, __dsub_rn(tmp, wsum));
+    const uint32_t sr = (__ldg(&plane[r * W + w]) >> lane) & 1u;
+    half[gw * 32 + lane] = __dmul_rn(sr ? -rs : rs, 0.5);
+}
+
+__global__ void __launch_bounds__(32) k_cut_sum(const double *__restrict__ half, int64_t rows, int32_t Ap,
+                                                int32_t A, int first, int last, double wsum, double *cut)
+{
+    const int a = blockIdx.x * 32 + threadIdx.x;
+    if (a >= A) return;
+    double tmp = first ? 0.0 : cut[a];
+#pragma unroll 16
+    for (int64_t i = 0; i < rows; i++) tmp = __dadd_rn(tmp, half[i * Ap + a]);
+    cut[a] = last ? __dmul_rn(-0.5, __dsub_rn(tmp, wsum)) : tmp;
 }
 
 // The statistics line of src/ising.cu:238-265 over the A values v[i] = val(i),
@@ -413,9 +545,32 @@ __global__ void k_cut_ordered(const int32_t *__restrict__ rowptr, const uint32_t
 // them.  out: min, max, total, mean, sum of squared deviations, agents at max,
 // first agent at max.  The host takes the standard deviation
 // pow(sd / (A - 1), 0.5) and ps = n_max / A from these.
+// The serial sums read their terms from shared memory, a tile at a time, so
+// each costs one FP64 addition (from global memory, with the subtraction and
+// the product in the chain, 200 agents took 32 us).
+constexpr int kStatTile = 512;
+
+template <class F>
+__device__ __forceinline__ double ordered_sum(F term, int32_t A, double *tile)
+{
+    double total = 0;
+    for (int32_t i0 = 0; i0 < A; i0 += kStatTile) {
+        const int32_t m = min(A - i0, kStatTile);
+        __syncwarp();
+        for (int32_t i = threadIdx.x & 31; i < m; i += 32) tile[i] = term(i0 + i);
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) {
+#pragma unroll 8
+            for (int32_t i = 0; i < m; i++) total = __dadd_rn(total, tile[i]);
+        }
+    }
+    return __shfl_sync(FULL, total, 0);
+}
+
 template <class F>
 __device__ __forceinline__ void stats_warp(F val, int32_t A, double *out)
 {
+    __shared__ double tile[kStatTile];
     const int lane = threadIdx.x & 31;
     double mn = DBL_MAX, mx = -DBL_MAX;
     for (int32_t i = lane; i < A; i += 32) {
@@ -435,17 +590,15 @@ __device__ __forceinline__ void stats_warp(F val, int32_t A, double *out)
         }
     nmax = __reduce_add_sync(FULL, nmax);
     first = __reduce_min_sync(FULL, first);
-    if (lane == 0) {
-        double total = 0;
-#pragma unroll 8
-        for (int32_t i = 0; i < A; i++) total = __dadd_rn(total, val(i));
-        const double avg = __ddiv_rn(total, (double)A);
-        double sd = 0;
-#pragma unroll 8
-        for (int32_t i = 0; i < A; i++) {
+    const double total = ordered_sum(val, A, tile);
+    const double avg = __ddiv_rn(total, (double)A);
+    const double sd = ordered_sum(
+        [&](int32_t i) {
             const double dv = __dsub_rn(val(i), avg);
-            sd = __dadd_rn(sd, __dmul_rn(dv, dv));
-        }
+            return __dmul_rn(dv, dv);
+        },
+        A, tile);
+    if (lane == 0) {
         out[0] = mn;
         out[1] = mx;
         out[2] = total;
@@ -509,6 +662,30 @@ cudaError_t launch_cut_batch(const SolveDims &d, const DevCsr &J, const uint32_t
     return cudaGetLastError();
 }
 
+int64_t cut_scratch_rows(const SolveDims &d, const DevCsr &J)
+{
+    // 32 MB of halves at a time: launches of k_cut_rows that fill the GPU
+    return J.integer ? 0 : std::min<int64_t>(d.n, std::max<int64_t>(1, ((int64_t)32 << 20) / (8 * d.Ap)));
+}
+
+namespace {
+
+template <int WL>
+void cut_unit(const SolveDims &d, const DevCsr &J, const uint32_t *plane, unsigned long long *eacc, cudaStream_t s)
+{
+    // runs of 8 entries or more (a walked entry costs two or three L2 round
+    // trips: short runs in many groups), and no more groups than fill the GPU
+    const int nsm = std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
+    const int64_t per_block = 8 * (32 / WL), ny = (d.W + WL - 1) / WL;
+    const int64_t most = std::max<int64_t>(1, (int64_t)nsm * 8 / ny);
+    const int64_t blocks = std::max<int64_t>(1, std::min(most, J.nnz / (8 * per_block)));
+    const int64_t run = std::max<int64_t>(1, (J.nnz + blocks * per_block - 1) / (blocks * per_block));
+    k_cut_unit<WL><<<dim3((unsigned)blocks, (unsigned)ny), 256, 0, s>>>(J.rowptr, J.colw, plane, (int32_t)d.n,
+                                                                        (int32_t)J.nnz, d.W, (int32_t)run, eacc);
+}
+
+}  // namespace
+
 cudaError_t launch_cut(const SolveDims &d, const DevCsr &J, Work &w, const uint32_t *plane,
                        cudaStream_t s, int *launches)
 {
@@ -516,17 +693,30 @@ cudaError_t launch_cut(const SolveDims &d, const DevCsr &J, Work &w, const uint3
     if (J.integer) {
         e = cudaMemsetAsync(w.eacc, 0, sizeof(unsigned long long) * d.Ap, s);
         if (e != cudaSuccess) return e;
-        int gy = (int)((d.n + 7) / 8);
-        int cap = (152 * 8 + d.W - 1) / d.W;
-        if (gy > cap) gy = cap;
-        k_cut_int<<<dim3(d.W, gy), 256, 0, s>>>(J.rowptr, J.colw, J.valf, J.unit ? 1 : 0, plane,
-                                                d.n, d.W, w.eacc);
+        if (J.unit) {
+            // the widest group that the row's words fill
+            if (d.W >= 16) cut_unit<16>(d, J, plane, w.eacc, s);
+            else if (d.W >= 8) cut_unit<8>(d, J, plane, w.eacc, s);
+            else if (d.W >= 4) cut_unit<4>(d, J, plane, w.eacc, s);
+            else if (d.W >= 2) cut_unit<2>(d, J, plane, w.eacc, s);
+            else cut_unit<1>(d, J, plane, w.eacc, s);
+        } else {
+            int gy = (int)((d.n + 7) / 8);
+            int cap = (152 * 8 + d.W - 1) / d.W;
+            if (gy > cap) gy = cap;
+            k_cut_int<<<dim3(d.W, gy), 256, 0, s>>>(J.rowptr, J.colw, J.valf, plane, d.n, d.W, w.eacc);
+        }
         k_cut_finish<<<(d.A + 255) / 256, 256, 0, s>>>(w.eacc, d.A, J.wsum, w.cut);
         *launches += 2;
     } else {
-        k_cut_ordered<<<(d.A + 127) / 128, 128, 0, s>>>(J.rowptr, J.colw, J.vald, plane, d.n, d.W,
-                                                        d.A, J.wsum, w.cut);
-        *launches += 1;
+        const int64_t step = cut_scratch_rows(d, J);
+        for (int64_t r = 0; r < d.n; r += step) {
+            const int64_t rows = std::min(step, d.n - r);
+            k_cut_rows<<<(unsigned)((rows * d.W + 7) / 8), 256, 0, s>>>(J.rowptr, J.colw, J.vald, plane, r, rows,
+                                                                        d.W, w.cutrow);
+            k_cut_sum<<<d.W, 32, 0, s>>>(w.cutrow, rows, d.Ap, d.A, r == 0, r + rows >= d.n, J.wsum, w.cut);
+            *launches += 2;
+        }
     }
     return cudaGetLastError();
 }
