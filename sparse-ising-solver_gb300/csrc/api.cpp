@@ -153,12 +153,10 @@ void free_csr(DevCsr &J)
     cudaFree(J.rinst);
     cudaFree(J.iagents);
     cudaFree(J.iwsum);
-    cudaFree(J.rs_rowptr);
-    cudaFree(J.rs_colw);
-    cudaFree(J.rs_valf);
-    J.rs_rowptr = nullptr;
-    J.rs_colw = nullptr;
-    J.rs_valf = nullptr;
+    for (DevSell &L : J.sell) {
+        cudaFree(L.base);
+        L = DevSell();
+    }
     J.iagents = nullptr;
     J.iwsum = nullptr;
     J.ninst = 0;
@@ -742,7 +740,7 @@ int run_stream(sbx_ctx *ctx, const void *key_obj, const SolveDims &d, const DevC
     return SBX_OK;
 }
 
-int ensure_rs_csr(sbx_ctx *ctx, DevCsr &J);
+int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale);
 
 int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_result *res,
                  double *agent_values)
@@ -794,7 +792,9 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     if (pr->kernel == SBX_KERNEL_RESIDENT_SPLIT && !rs)
         return fail(ctx, SBX_ERR_UNSUPPORTED,
                     "split resident kernel: 16-bit fused state, degree <= 127 and fitting on chip only");
-    if (rs && (rc = ensure_rs_csr(ctx, const_cast<DevCsr &>(p->J)))) return rc;
+    DevCsr &Jm = const_cast<DevCsr &>(p->J);
+    if (ka == 8 && (rc = ensure_sell(ctx, Jm, Jm.sell[0], 4))) return rc;
+    if (rs && (rc = ensure_sell(ctx, Jm, Jm.sell[1], 1))) return rc;
     if (!ka && !rs) {
         bool timed = false;
         if ((rc = pick_tile(ctx, d, p->J, pr, &timed))) return rc;
@@ -1122,33 +1122,52 @@ int build_class(sbx_ctx *ctx, BatchClass &c)
     return SBX_OK;
 }
 
-// The matrix in perm order for the register + shared resident kernel: row s
-// is row perm[s], its columns renamed to their slots, entries in the original
-// order within the row (the FP32 sums of real weights keep their order).
-int ensure_rs_csr(sbx_ctx *ctx, DevCsr &J)
+// The sliced form of the matrix (engine.h, DevSell) with entries scaled by
+// scale; entries in the original order within each row (the FP32 sums of
+// real weights keep their order).
+int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
 {
-    if (J.rs_rowptr) return SBX_OK;
-    const int64_t n = J.n;
-    std::vector<int32_t> inv((size_t)n), rp((size_t)n + 1, 0);
+    if (L.base) return SBX_OK;
+    const int64_t n = J.n, nsl = (n + 31) / 32;
+    if (n * scale > 32767) return fail(ctx, SBX_ERR_UNSUPPORTED, "resident kernel: column offsets past 15 bits");
+    std::vector<int32_t> inv((size_t)n);
     for (int64_t s = 0; s < n; s++) inv[(size_t)J.hperm[(size_t)s]] = (int32_t)s;
-    std::vector<uint32_t> cw((size_t)std::max<int64_t>(J.nnz, 1));
-    std::vector<float> vf((size_t)std::max<int64_t>(J.nnz, 1));
-    int64_t e = 0;
+    auto degree = [&](int64_t s) {
+        const size_t r = (size_t)J.hperm[(size_t)s];
+        return J.hrowptr[r + 1] - J.hrowptr[r];
+    };
+    std::vector<int64_t> off((size_t)nsl + 1, 0);
+    for (int64_t k = 0; k < nsl; k++) off[(size_t)k + 1] = off[(size_t)k] + (degree(32 * k) + 3) / 4;   // slots fall in degree
+    const int64_t blocks = off[(size_t)nsl];
+    if (blocks * 32 > INT32_MAX) return fail(ctx, SBX_ERR_UNSUPPORTED, "resident kernel: matrix too large");
+    // one buffer: blocks' columns, blocks' weights, slice offsets, degrees
+    const size_t bcol = (size_t)blocks * 32 * 8, bval = J.unit ? 0 : (size_t)blocks * 32 * 16;
+    const size_t boff = ((size_t)(nsl + 1) * 4 + 15) / 16 * 16, bdeg = (size_t)n * 4;
+    std::vector<unsigned char> buf(bcol + bval + boff + bdeg, 0);
+    uint16_t *col = (uint16_t *)buf.data();
+    float *val = (float *)(buf.data() + bcol);
+    int32_t *ho = (int32_t *)(buf.data() + bcol + bval), *hd = (int32_t *)(buf.data() + bcol + bval + boff);
+    std::fill(col, col + blocks * 128, (uint16_t)(n * scale));
+    for (int64_t k = 0; k <= nsl; k++) ho[k] = (int32_t)off[(size_t)k];
     for (int64_t s = 0; s < n; s++) {
-        const int32_t r = J.hperm[(size_t)s];
-        for (int32_t k = J.hrowptr[(size_t)r]; k < J.hrowptr[(size_t)r + 1]; k++, e++) {
-            const double v = J.hval[(size_t)k];
-            cw[(size_t)e] = (uint32_t)inv[(size_t)J.hcol[(size_t)k]] | ((J.unit && v < 0) ? 0x80000000u : 0u);
-            vf[(size_t)e] = (float)v;
+        const size_t r = (size_t)J.hperm[(size_t)s];
+        hd[s] = degree(s);
+        for (int32_t j = 0; j < hd[s]; j++) {
+            const size_t e = (size_t)J.hrowptr[r] + (size_t)j;
+            const double v = J.hval[e];
+            const size_t at = ((size_t)(off[(size_t)(s / 32)] + j / 4) * 32 + (size_t)(s & 31)) * 4 + (size_t)(j & 3);
+            col[at] = (uint16_t)(inv[(size_t)J.hcol[e]] * scale) | (uint16_t)((J.unit && v < 0) ? 0x8000u : 0u);
+            if (!J.unit) val[at] = -(float)v;
         }
-        rp[(size_t)s + 1] = (int32_t)e;
     }
-    CK(cudaMalloc(&J.rs_rowptr, sizeof(int32_t) * (n + 1)));
-    CK(cudaMalloc(&J.rs_colw, sizeof(uint32_t) * cw.size()));
-    CK(cudaMalloc(&J.rs_valf, sizeof(float) * vf.size()));
-    CK(cudaMemcpy(J.rs_rowptr, rp.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(J.rs_colw, cw.data(), sizeof(uint32_t) * cw.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(J.rs_valf, vf.data(), sizeof(float) * vf.size(), cudaMemcpyHostToDevice));
+    unsigned char *dev = nullptr;
+    CK(cudaMalloc(&dev, std::max<size_t>(buf.size(), 16)));
+    L.base = dev;
+    CK(cudaMemcpy(dev, buf.data(), buf.size(), cudaMemcpyHostToDevice));
+    L.col = (const uint2 *)dev;
+    L.val = J.unit ? nullptr : (const float4 *)(dev + bcol);
+    L.off = (const int32_t *)(dev + bcol + bval);
+    L.deg = (const int32_t *)(dev + bcol + bval + boff);
     return SBX_OK;
 }
 

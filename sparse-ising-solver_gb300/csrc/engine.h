@@ -43,6 +43,23 @@ inline int dev_attr(cudaDeviceAttr a)
 
 struct DevBsm;
 
+// A matrix in sliced form for the resident kernels: row s is the row of slot
+// s (perm[s], decreasing degree), 32 consecutive slots a slice, a slice's
+// entries in blocks of four per row, blocks as long as its longest row needs.
+// Lane l of a warp reads its block as one 8-byte word next to its
+// neighbours' (a row-by-row layout cost a cache line per lane and entry).
+// An entry is its column's slot times `scale` (the byte offset of the slot in
+// the kernel's sign array), bit 15 the sign of a -1 weight; entries past a
+// row's end name slot n, whose signs are all zero.  val: the negated weights
+// of other matrices, zero past a row's end.
+struct DevSell {
+    void *base = nullptr;              // one allocation holding the arrays below
+    const int32_t *off = nullptr;      // [slices + 1] first block of each slice
+    const int32_t *deg = nullptr;      // [n] entries of each slot
+    const uint2 *col = nullptr;        // [blocks][32]
+    const float4 *val = nullptr;       // [blocks][32], null for +-1 weights
+};
+
 // MaxCut / QUBO matrix on the device.  colw holds the column index; when every
 // weight is +-1 ("unit"), bit 31 holds the weight's sign and no value array is
 // read by the step kernels.
@@ -78,14 +95,12 @@ struct DevCsr {
     int32_t max_deg = 0;
     std::vector<double> hval;   // host copy of values (xi0)
     std::vector<int32_t> hrowptr, hcol, hperm;
-    // The matrix relabelled into perm order (row and column s = perm slot s),
-    // built on first use by the register + shared resident kernel.
+    // The sliced forms of the resident kernels, built on first use: [0] entries
+    // scaled by 4 (sign words), [1] by 1 (sign bytes).
+    DevSell sell[2];
     // Batched: the plan of the shared-memory-plane step kernel, when the
     // solve uses it (k_batch_smem.cu)
     const DevBsm *bsm = nullptr;
-    int32_t *rs_rowptr = nullptr;
-    uint32_t *rs_colw = nullptr;
-    float *rs_valf = nullptr;
 };
 
 // Control words shared by the kernels of one solve.

@@ -5,15 +5,21 @@
 // memory.  The whole solve (or one window, in the update-window mode) is one
 // launch; agents never interact, so a CTA needs no other CTA and one
 // __syncthreads() per step gives the Jacobi order of the reference kernel
-// (src/kernels.cu:211-269).  The arithmetic is the streaming kernel's
-// (sb_update, exact byte-counter force), so the two give identical states.
+// (src/kernels.cu:211-269).  The arithmetic is the streaming kernel's (exact
+// force, sb_update's roundings), so the two give identical states.
 //
 // Thread t owns the slots s = i*NT + t of the degree-sorted row list (row
 // perm[s]): slots i < RR in registers, the others in shared memory.  The
-// kernel reads the matrix relabelled into slot order (rows and columns), so a
-// warp's row pointers are consecutive and sign bytes are indexed by slot;
-// perm maps slots back to rows only where the global state is read or
-// written.
+// kernel reads the matrix in sliced form (engine.h, DevSell), so a warp's
+// entries are coalesced; perm maps slots back to rows only where the global
+// state is read or written.
+//
+// Force for +-1 weights: a block's four neighbour bytes (8 agents each) are
+// put together in a word and XORed with the four weights' signs (one PRMT
+// makes the mask); the words add up in bit planes, full adders over four
+// byte lanes at once, as many planes as the row's blocks can fill; the lanes
+// are then summed plane by plane and the planes transposed into byte
+// counters.  Bound: issue.
 #include "k_step.cuh"
 
 namespace sbx {
@@ -21,10 +27,11 @@ namespace sbx {
 namespace {
 
 struct RsP {
-    const int32_t *__restrict__ rowptr;   // slot order
-    const uint32_t *__restrict__ colw;    // columns as slots, bit 31 the weight sign
-    const float *__restrict__ valf;
-    const int32_t *__restrict__ perm;     // slot -> row
+    const int32_t *__restrict__ off;    // sliced matrix (engine.h, DevSell)
+    const int32_t *__restrict__ deg;
+    const uint2 *__restrict__ col;
+    const float4 *__restrict__ val;
+    const int32_t *__restrict__ perm;   // slot -> row
     const float4 *__restrict__ coef;    // per step: k1, k2 (clamped), k1, k2 (raw)
     void *x, *y;                        // global [n][Ap]
     uint32_t *Wp, *fin;                 // global planes [n][W]
@@ -35,7 +42,7 @@ struct RsP {
     int32_t *gbar;                      // co-resident launch: CTAs past each window
     int32_t coop;                       // 1: all windows in one co-resident launch
     int32_t n, A, Ap, W, period, threshold, uw;
-    int32_t step0, nsteps, first, unit;
+    int32_t step0, nsteps, first, unit, allpos;
     float c0;
     int32_t giveup;                     // test only: the window barrier gives up at once
 };
@@ -50,61 +57,139 @@ __device__ __forceinline__ void plane_put8(uint32_t *p, uint32_t bits, int sh)
     atomicOr(p, (bits << sh) & m);
 }
 
-// One SB step of slot s's 8 agents held in xv, yv (16-bit, packed).
-template <class T>
-__device__ __forceinline__ uint32_t row_step(const RsP &P, int s, uint4 &xv, uint4 &yv, const uint8_t *Sin,
-                                             const float4 &c)
+// The four neighbour bytes of block b of a row (8 agents each, at shared
+// address S) as one word, signs of the weights applied.
+__device__ __forceinline__ uint32_t lds8(uint32_t a)
 {
-    const int32_t e0 = __ldg(&P.rowptr[s]), e1 = __ldg(&P.rowptr[s + 1]);
-    const int32_t deg = e1 - e0;
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t block_word(const uint2 &c, uint32_t S, bool neg)
+{
+    const uint32_t b0 = lds8(S + (c.x & 0x7fffu)), b1 = lds8(S + ((c.x >> 16) & 0x7fffu));
+    const uint32_t b2 = lds8(S + (c.y & 0x7fffu)), b3 = lds8(S + ((c.y >> 16) & 0x7fffu));
+    const uint32_t w = __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
+    return neg ? w ^ prmt<0xfdb9>(c.x, c.y) : w;
+}
+
+// p[0..N) += the same planes shifted down by SH bits; one plane more.
+template <int N, int SH> __device__ __forceinline__ void fold(uint32_t (&p)[8])
+{
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint32_t b = p[k] >> SH;
+        if (k == 0) {
+            c = p[0] & b;
+            p[0] ^= b;
+        } else {
+            c = fadd(p[k], b, c);
+        }
+    }
+    p[N] = c;
+}
+
+// Byte counters of 2 * count over nb blocks (fewer than 2^PL): agents 0..3 in lo,
+// 4..7 in hi.
+template <int PL>
+__device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32_t S, bool neg, uint32_t &lo,
+                                             uint32_t &hi)
+{
+    uint32_t p[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (PL == 1) {
+        p[0] = block_word(__ldg(cp), S, neg);
+    } else {
+        for (int32_t b = 0; b < nb; b += 2) {
+            const uint2 c0 = __ldg(cp + b * 32);
+            uint2 c1;
+            const bool two = b + 1 < nb;   // warp-uniform
+            if (two) c1 = __ldg(cp + (b + 1) * 32);
+            const uint32_t w0 = block_word(c0, S, neg), w1 = two ? block_word(c1, S, neg) : 0u;
+            uint32_t c = fadd(p[0], w0, w1);
+#pragma unroll
+            for (int k = 1; k < PL; k++) {
+                const uint32_t t = p[k] & c;
+                p[k] ^= c;
+                c = t;
+            }
+        }
+    }
+    fold<PL, 16>(p);
+    fold<PL + 1, 8>(p);   // the low byte of each plane: PL + 2 planes, counts of at most 127
+    // bytes shifted up one plane (which doubles the counts), then an 8x8 bit
+    // transpose of (lo, hi)
+    lo = __byte_perm(__byte_perm(0u, p[0], 0x0040), __byte_perm(p[1], p[2], 0x0040), 0x5410);
+    hi = PL == 1 ? 0u
+                 : PL == 2 ? p[3] & 0xffu
+                           : __byte_perm(__byte_perm(p[3], p[4], 0x0040), __byte_perm(p[5], p[6], 0x0040), 0x5410);
+    uint32_t t;
+    t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
+    lo ^= t ^ (t << 7);
+    t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
+    lo ^= t ^ (t << 14);
+    if (PL > 1) {
+        t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
+        hi ^= t ^ (t << 7);
+        t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
+        hi ^= t ^ (t << 14);
+    }
+    t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
+    lo ^= t;
+    hi ^= t >> 4;
+}
+
+// One SB step of slot s's 8 agents held in xv, yv (16-bit, packed); the new
+// signs as a byte.
+template <class T>
+__device__ __forceinline__ uint32_t row_step(const RsP &P, int s, uint4 &xv, uint4 &yv, uint32_t S, const float4 &c)
+{
+    const int sl = s >> 5, lane = s & 31;
+    const int32_t b0 = __ldg(&P.off[sl]), nb = __ldg(&P.off[sl + 1]) - b0;   // warp-uniform
+    const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
     float tv[KA];
     if (P.unit) {
-        // byte counters of 2 * count (deg <= 127), as the streaming kernel
         uint32_t lo = 0, hi = 0;
-        auto add = [&](uint32_t cw) {
-            const uint32_t b = (uint32_t)Sin[cw & 0x7fffffffu] ^ (0u - (cw >> 31));
-            lo += spread2x(b & 0xfu);
-            hi += spread2x((b >> 4) & 0xfu);
-        };
-        if (deg == 4 && (e0 & 3) == 0) {
-            // four neighbours on a 16-byte boundary (lattices): one vector load
-            const uint4 c4 = __ldg((const uint4 *)(P.colw + e0));
-            add(c4.x);
-            add(c4.y);
-            add(c4.z);
-            add(c4.w);
-        } else {
-#pragma unroll 4
-            for (int32_t e = e0; e < e1; e++) add(__ldg(&P.colw[e]));
-        }
-        const float bias = 8388608.0f + (float)deg;
+        const bool neg = !P.allpos;
+        if (nb == 1) count_blocks<1>(cp, nb, S, neg, lo, hi);
+        else if (nb < 8) count_blocks<3>(cp, nb, S, neg, lo, hi);
+        else count_blocks<6>(cp, nb, S, neg, lo, hi);   // degree <= 127: at most 32 blocks
+        // PRMT builds the float 2^23 + 2 count; minus 2^23 + degree it is the
+        // force 2 count - degree, exactly
+        const float b = -(8388608.0f + (float)__ldg(&P.deg[s]));
+        const float2 bias = make_float2(b, b);
 #pragma unroll
-        for (int v = 0; v < KA; v++)
-            tv[v] = __uint_as_float(__byte_perm(v < 4 ? lo : hi, 0x4b000000u, 0x7440u + (v & 3))) - bias;
+        for (int v = 0; v < KA; v += 2) {
+            const uint32_t w = v < 4 ? lo : hi;
+            const float2 f = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + (v & 3))),
+                                                    __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7441u + (v & 3)))),
+                                        bias);
+            tv[v] = f.x;
+            tv[v + 1] = f.y;
+        }
     } else {
 #pragma unroll
         for (int v = 0; v < KA; v++) tv[v] = 0.0f;
-        for (int32_t e = e0; e < e1; e++) {
-            const uint32_t cw = __ldg(&P.colw[e]);
-            const float wv = __ldg(&P.valf[e]);
-            const uint32_t b = Sin[cw & 0x7fffffffu];
+        for (int32_t b = 0; b < nb; b++) {
+            const uint2 c4 = __ldg(cp + b * 32);
+            const float4 v4 = __ldg(P.val + ((int64_t)b0 + b) * 32 + lane);
+            const uint32_t o[4] = {c4.x & 0xffffu, c4.x >> 16, c4.y & 0xffffu, c4.y >> 16};
+            const float wv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-            for (int v = 0; v < KA; v++) tv[v] -= wv * (((b >> v) & 1u) ? -1.0f : 1.0f);
+            for (int j = 0; j < 4; j++) {
+                const uint32_t w = lds8(S + o[j]);
+                // wv is the negated weight; a set bit is spin -1
+#pragma unroll
+                for (int v = 0; v < KA; v++) tv[v] += ((w >> v) & 1u) ? -wv[j] : wv[j];
+            }
         }
     }
-    Raw<16> xr, yr;
-    xr.u = xv;
-    yr.u = yv;
-    float x[KA], y[KA];
-    to_vals<T, KA>(xr, x);
-    to_vals<T, KA>(yr, y);
-    sb_update<K_FUSED, false, KA>(x, y, tv, P.c0, c, c);
-    uint32_t nb = 0;
-#pragma unroll
-    for (int v = 0; v < KA; v++) nb |= sbit(x[v]) << v;
-    xv = from_vals<T, KA>(x).u;
-    yv = from_vals<T, KA>(y).u;
-    return nb;
+    uint32_t x[4] = {xv.x, xv.y, xv.z, xv.w}, y[4] = {yv.x, yv.y, yv.z, yv.w}, m0, m1;
+    sb_update16<T, K_FUSED, false, KA>(x, y, tv, P.c0, c, c);
+    xv = make_uint4(x[0], x[1], x[2], x[3]);
+    yv = make_uint4(y[0], y[1], y[2], y[3]);
+    sign_masks(x, m0, m1);
+    return sign_byte(m0, m1);
 }
 
 template <class T, int NT, int RR>
@@ -117,8 +202,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
     uint4 *xs = (uint4 *)smem;
     uint4 *ys = xs + ns;
     uint8_t *Sb0 = (uint8_t *)(ys + ns);
-    uint8_t *Sb1 = Sb0 + n;
-    uint8_t *Wb = Sb1 + n;
+    uint8_t *Sb1 = Sb0 + n + 1;   // one byte more each: the zero row
+    uint8_t *Wb = Sb1 + n + 1;
     __shared__ uint32_t s_chg, s_new, s_stop;
     __shared__ int32_t s_stab[KA];
     __shared__ uint8_t s_bif[KA], s_prev[KA];
@@ -137,6 +222,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
             if (P.wincount[widx] == P.A) s_stop = 1;
         }
         s_chg = 0;
+        Sb0[n] = 0;
+        Sb1[n] = 0;
     }
     if (tid < KA) {
         const int a = a0 + tid;
@@ -194,10 +281,11 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
     }
     __syncthreads();
 
+    const uint32_t sa0 = smem_u32(Sb0), sa1 = smem_u32(Sb1);
     int32_t nrun = P.nsteps;   // steps run (fewer at an update-window exit)
     for (int32_t it = 0; it < P.nsteps; it++) {
         const int32_t k = k0 + it;
-        const uint8_t *Sin = (k & 1) ? Sb1 : Sb0;
+        const uint32_t Sin = (k & 1) ? sa1 : sa0;
         uint8_t *Snx = (k & 1) ? Sb0 : Sb1;
         const bool win = ((k + 1) % P.period) == 0;
         const float4 ck = P.coef[k];
@@ -333,7 +421,7 @@ constexpr RsCfg kRsCfgs[] = {{1024, 0}, {1024, 2}, {1024, 4}};
 size_t rs_smem(int64_t n, const RsCfg &c)
 {
     const int64_t ns = n > (int64_t)c.rr * c.nt ? n - (int64_t)c.rr * c.nt : 0;
-    return (size_t)ns * 32 + (size_t)n * 3;
+    return (size_t)ns * 32 + (size_t)n * 3 + 2;
 }
 
 template <class T, int NT, int RR>
@@ -406,10 +494,12 @@ cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int
 {
     if (cfg < 1) return cudaErrorInvalidValue;
     RsP P;
-    if (!J.rs_rowptr) return cudaErrorInvalidValue;
-    P.rowptr = J.rs_rowptr;
-    P.colw = J.rs_colw;
-    P.valf = J.rs_valf;
+    if (!J.sell[1].base) return cudaErrorInvalidValue;
+    P.off = J.sell[1].off;
+    P.deg = J.sell[1].deg;
+    P.col = J.sell[1].col;
+    P.val = J.sell[1].val;
+    P.allpos = J.allpos ? 1 : 0;
     P.perm = J.perm;
     P.coef = (const float4 *)w.coef32;
     P.x = w.x;

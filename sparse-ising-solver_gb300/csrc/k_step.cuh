@@ -504,6 +504,102 @@ __device__ __forceinline__ void sb_update(double (&x)[V], double (&y)[V], const 
     }
 }
 
+// prmt with the selector's sign-replicate bit (0x8 of a nibble: the byte's
+// top bit in all of its bits), which __byte_perm does not reach.
+template <uint32_t SEL> __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "n"(SEL));
+    return d;
+}
+
+// Two 16-bit values at a time: x clamped to [-1, 1], and (k0, k1) zeroed
+// where that changed x.  |x| > 1 is exactly "the clamp moves x", the clamped
+// value is the reference's sign(x), NaN passes through as before.
+template <class T> __device__ __forceinline__ uint32_t wall2(uint32_t x, float &k0, float &k1);
+template <> __device__ __forceinline__ uint32_t wall2<__nv_bfloat16>(uint32_t x, float &k0, float &k1)
+{
+    uint32_t c;
+    asm("{\n\t.reg .pred p, q;\n\t"
+        "max.NaN.bf16x2 %0, %3, %4;\n\t"
+        "min.NaN.bf16x2 %0, %0, %5;\n\t"
+        "setp.ne.bf16x2 p|q, %0, %3;\n\t"
+        "selp.f32 %1, 0f00000000, %1, p;\n\t"
+        "selp.f32 %2, 0f00000000, %2, q;\n\t}"
+        : "=&r"(c), "+f"(k0), "+f"(k1)
+        : "r"(x), "r"(0xbf80bf80u), "r"(0x3f803f80u));
+    return c;
+}
+template <> __device__ __forceinline__ uint32_t wall2<__half>(uint32_t x, float &k0, float &k1)
+{
+    uint32_t c;
+    asm("{\n\t.reg .pred p, q;\n\t"
+        "max.NaN.f16x2 %0, %3, %4;\n\t"
+        "min.NaN.f16x2 %0, %0, %5;\n\t"
+        "setp.ne.f16x2 p|q, %0, %3;\n\t"
+        "selp.f32 %1, 0f00000000, %1, p;\n\t"
+        "selp.f32 %2, 0f00000000, %2, q;\n\t}"
+        : "=&r"(c), "+f"(k0), "+f"(k1)
+        : "r"(x), "r"(0xbc00bc00u), "r"(0x3c003c00u));
+    return c;
+}
+
+// sb_update of V agents on the packed 16-bit state: the same arithmetic
+// (packed FP32 FMAs, one rounding per store), the clamp and its test on the
+// packed x (two values an instruction).
+template <class T, int KIND, bool WIN, int V, class C4>
+__device__ __forceinline__ void sb_update16(uint32_t (&xw)[V / 2], uint32_t (&yw)[V / 2], const float (&tv)[V],
+                                            float c0, const C4 &c, const C4 &cn)
+{
+    const float2 c02 = make_float2(c0, c0);
+#pragma unroll
+    for (int i = 0; i < V / 2; i++) {
+        Raw<4> r;
+        float x[2], y[2];
+        r.u = yw[i];
+        to_vals<T, 2>(r, y);
+        float2 Y = __ffma2_rn(c02, make_float2(tv[2 * i], tv[2 * i + 1]), make_float2(y[0], y[1]));
+        r.u = wall2<T>(xw[i], Y.x, Y.y);
+        to_vals<T, 2>(r, x);
+        float2 X = make_float2(x[0], x[1]);
+        if (KIND == K_FUSED) {
+            X = __ffma2_rn(make_float2(c.x, c.x), Y, X);
+            Y = __ffma2_rn(make_float2(c.y, c.y), X, Y);
+        } else if (!WIN) {
+            Y = __ffma2_rn(make_float2(cn.w, cn.w), X, Y);
+            X = __ffma2_rn(make_float2(cn.z, cn.z), Y, X);
+        }
+        x[0] = X.x;
+        x[1] = X.y;
+        y[0] = Y.x;
+        y[1] = Y.y;
+        xw[i] = from_vals<T, 2>(x).u;
+        yw[i] = from_vals<T, 2>(y).u;
+    }
+}
+
+// Sign masks of eight values: byte j of m0 (m1) is 0xff where value j (4 + j)
+// is negative; packed 16-bit values or floats.
+__device__ __forceinline__ void sign_masks(const uint32_t (&xw)[4], uint32_t &m0, uint32_t &m1)
+{
+    m0 = prmt<0xfdb9>(xw[0], xw[1]);
+    m1 = prmt<0xfdb9>(xw[2], xw[3]);
+}
+__device__ __forceinline__ void sign_masks(const float (&x)[8], uint32_t &m0, uint32_t &m1)
+{
+    uint32_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) h[i] = prmt<0x00fb>(__float_as_uint(x[2 * i]), __float_as_uint(x[2 * i + 1]));
+    m0 = __byte_perm(h[0], h[1], 0x5410);
+    m1 = __byte_perm(h[2], h[3], 0x5410);
+}
+// The masks as a byte, bit v the sign of value v: two dot products with
+// -2^v (a mask byte is -1 or 0).
+__device__ __forceinline__ uint32_t sign_byte(uint32_t m0, uint32_t m1)
+{
+    return (uint32_t)__dp4a((int)m1, (int)0x80c0e0f0u, __dp4a((int)m0, (int)0xf8fcfeffu, 0));
+}
+
 // One SB step over every (row, agent).  Work item = (group of 32/LR rows,
 // segment of LR*V agents); lane l of a row owns V consecutive agents (one
 // vector load of x and of y).  Per neighbour j the lane reads the sign word
