@@ -1123,8 +1123,8 @@ int build_class(sbx_ctx *ctx, BatchClass &c)
 }
 
 // The sliced form of the matrix (engine.h, DevSell) with entries scaled by
-// scale; entries in the original order within each row (the FP32 sums of
-// real weights keep their order).
+// scale; real weights' entries in the original order within each row (their
+// FP32 sums keep it).
 int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
 {
     if (L.base) return SBX_OK;
@@ -1149,15 +1149,67 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
     int32_t *ho = (int32_t *)(buf.data() + bcol + bval), *hd = (int32_t *)(buf.data() + bcol + bval + boff);
     std::fill(col, col + blocks * 128, (uint16_t)(n * scale));
     for (int64_t k = 0; k <= nsl; k++) ho[k] = (int32_t)off[(size_t)k];
-    for (int64_t s = 0; s < n; s++) {
-        const size_t r = (size_t)J.hperm[(size_t)s];
-        hd[s] = degree(s);
-        for (int32_t j = 0; j < hd[s]; j++) {
-            const size_t e = (size_t)J.hrowptr[r] + (size_t)j;
-            const double v = J.hval[e];
-            const size_t at = ((size_t)(off[(size_t)(s / 32)] + j / 4) * 32 + (size_t)(s & 31)) * 4 + (size_t)(j & 3);
-            col[at] = (uint16_t)(inv[(size_t)J.hcol[e]] * scale) | (uint16_t)((J.unit && v < 0) ? 0x8000u : 0u);
-            if (!J.unit) val[at] = -(float)v;
+    // The kernels gather the 32 entries that a slice's rows hold at one
+    // position with one shared load, and random rows meet in a bank 2.7 deep
+    // (the gather's wavefronts bounded er800).  Neighbour counts of +-1
+    // weights do not depend on the order, so each position takes, row by row,
+    // an entry whose bank is still free there, or padding while the row has
+    // positions to spare.
+    auto place = [&](int64_t k, std::vector<uint16_t> &ent) {
+        const int64_t s0 = 32 * k, rows = std::min<int64_t>(32, n - s0), pos = 4 * (off[(size_t)k + 1] - off[(size_t)k]);
+        ent.resize((size_t)(32 * pos));
+        int64_t left[32];
+        for (int64_t l = 0; l < rows; l++) {
+            const size_t r = (size_t)J.hperm[(size_t)(s0 + l)];
+            uint16_t *v = &ent[(size_t)(l * pos)];
+            left[l] = J.hrowptr[r + 1] - J.hrowptr[r];
+            for (int32_t e = J.hrowptr[r]; e < J.hrowptr[r + 1]; e++)
+                *v++ = (uint16_t)((uint32_t)(inv[(size_t)J.hcol[(size_t)e]] * scale) |
+                                  (J.hval[(size_t)e] < 0 ? 0x8000u : 0u));
+        }
+        for (int64_t j = 0; j < pos; j++) {
+            int32_t word[32];   // the shared word each bank serves at this position
+            std::fill(word, word + 32, -1);
+            for (int64_t t = 0; t < rows; t++) {
+                const int64_t l = t + j % rows < rows ? t + j % rows : t + j % rows - rows;
+                uint16_t *v = &ent[(size_t)(l * pos)];
+                const int64_t m = left[l];
+                if (!m) continue;
+                int64_t pick = m;
+                for (int64_t c = m - 1; c >= 0 && m - c <= 24; c--) {
+                    const int32_t w = (v[c] & 0x7fff) >> 2;
+                    if (word[w & 31] == -1 || word[w & 31] == w) {
+                        pick = c;
+                        break;
+                    }
+                }
+                if (pick == m) {
+                    if (m < pos - j) continue;   // padding here, the entry later
+                    pick = m - 1;
+                }
+                const int32_t w = (v[pick] & 0x7fff) >> 2;
+                word[w & 31] = w;
+                col[(((size_t)off[(size_t)k] + (size_t)(j / 4)) * 32 + (size_t)l) * 4 + (size_t)(j & 3)] = v[pick];
+                v[pick] = v[m - 1];
+                left[l] = m - 1;
+            }
+        }
+    };
+    for (int64_t s = 0; s < n; s++) hd[s] = degree(s);
+    if (J.unit) {
+        parallel(J.nnz > (1 << 16) ? std::min(host_threads(), 8) : 1, [&](int t, int TT) {
+            std::vector<uint16_t> ent;
+            for (int64_t k = nsl * t / TT; k < nsl * (t + 1) / TT; k++) place(k, ent);
+        });
+    } else {
+        for (int64_t s = 0; s < n; s++) {
+            const size_t r = (size_t)J.hperm[(size_t)s];
+            for (int32_t j = 0; j < hd[s]; j++) {
+                const size_t e = (size_t)J.hrowptr[r] + (size_t)j;
+                const size_t at = ((size_t)(off[(size_t)(s / 32)] + j / 4) * 32 + (size_t)(s & 31)) * 4 + (size_t)(j & 3);
+                col[at] = (uint16_t)(inv[(size_t)J.hcol[e]] * scale);
+                val[at] = -(float)J.hval[e];
+            }
         }
     }
     unsigned char *dev = nullptr;
