@@ -780,7 +780,7 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     if ((rc = upload_coef(ctx, d, total))) return rc;
     if ((rc = init_state(ctx, d, pr->seed, false))) return rc;
 
-    // on-chip kernels first: shared-memory resident, then register + shared
+    // on-chip kernels first: shared-memory resident, then tensor memory + shared
     int ka = 0, rs = 0;
     if ((pr->kernel == SBX_KERNEL_AUTO || pr->kernel == SBX_KERNEL_RESIDENT) && !d.trace)
         ka = resident_pick_ka(d, p->J, pr->agents_per_block);
@@ -868,7 +868,7 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     res->windows_run = ctl[CTL_WINDOWS];
     for (uint8_t b : bif) res->bifurcated += b;
     res->kernel_used = ka ? SBX_KERNEL_RESIDENT : rs ? SBX_KERNEL_RESIDENT_SPLIT : SBX_KERNEL_STREAM;
-    res->agents_per_block = ka ? ka : rs ? 8 : 0;
+    res->agents_per_block = ka ? ka : rs;
     if (!ka && !rs) {
         res->lane_agents = d.tv ? d.tv : default_v(d);
         res->row_lanes = d.tlr;

@@ -267,13 +267,13 @@ cudaError_t launch_resident(const SolveDims &d, const DevCsr &J, Work &w, int ka
 int64_t resident_batch_max_rows();
 cudaError_t launch_resident_batch(const SolveDims &d, const DevRb &B, Work &w, cudaStream_t s);
 
-// Register + shared-memory resident kernel (k_resident_rs.cu), 8 agents per
-// CTA, 16-bit fused state: a configuration number > 0 when the shape fits.
+// Tensor-memory + shared-memory resident kernel (k_resident_rs.cu), fused
+// steps: its agents per CTA (8 of 16-bit state, 4 of FP32) when it is to run.
 int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced);
 // coop: the update-window mode's windows in one co-resident launch (a
 // bounded barrier per window); cudaErrorCooperativeLaunchTooLarge when the
 // CTAs cannot all be resident.
-cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int cfg, int32_t step0,
+cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int ka, int32_t step0,
                                int32_t nsteps, bool first, bool coop, cudaStream_t s);
 
 // TSP kernels (k_tsp.cu).

@@ -1,15 +1,18 @@
 // k_resident_rs.cu -- resident MaxCut SB kernel for state too large for one
-// SM's shared memory: a CTA owns 8 agents of every row and keeps their x, y
-// (16-bit storage) partly in registers -- RR rows per thread -- and the rest
-// in shared memory, with the rows' 8-bit sign words double-buffered in shared
-// memory.  The whole solve (or one window, in the update-window mode) is one
+// SM's shared memory: a CTA owns KA agents of every row (8 of 16-bit state, 4
+// of FP32: 32 bytes of x, y a row) and keeps 8,192 rows of them in tensor
+// memory -- all of its 256 KB, used as plain storage: a thread's rows are
+// eight columns each of its own lane -- and the rest in shared memory, with
+// the rows' sign bytes double-buffered in shared memory.  (Register rows
+// instead, 4 a thread, left 32 registers to count with: 48 spilled words a
+// warp and step, all L1 misses beside 219 KB of shared memory.)  The whole solve (or one window, in the update-window mode) is one
 // launch; agents never interact, so a CTA needs no other CTA and one
 // __syncthreads() per step gives the Jacobi order of the reference kernel
 // (src/kernels.cu:211-269).  The arithmetic is the streaming kernel's (exact
 // force, sb_update's roundings), so the two give identical states.
 //
 // Thread t owns the slots s = i*NT + t of the degree-sorted row list (row
-// perm[s]): slots i < RR in registers, the others in shared memory.  The
+// perm[s]): slots i < 8 in tensor memory, the others in shared memory.  The
 // kernel reads the matrix in sliced form (engine.h, DevSell), so a warp's
 // entries are coalesced; perm maps slots back to rows only where the global
 // state is read or written.
@@ -21,6 +24,8 @@
 // are then summed plane by plane and the planes transposed into byte
 // counters.  Bound: issue.
 #include "k_step.cuh"
+
+#include <algorithm>
 
 namespace sbx {
 
@@ -42,17 +47,40 @@ struct RsP {
     int32_t *gbar;                      // co-resident launch: CTAs past each window
     int32_t coop;                       // 1: all windows in one co-resident launch
     int32_t n, A, Ap, W, period, threshold, uw;
-    int32_t step0, nsteps, first, unit, allpos;
+    int32_t step0, nsteps, first;
     float c0;
     int32_t giveup;                     // test only: the window barrier gives up at once
 };
 
-constexpr int KA = 8;   // agents per CTA: one sign byte per row
+// agents per CTA: their x and y take 32 bytes a row, their signs a byte
+template <class T> constexpr int kAgents = sizeof(T) == 4 ? 4 : 8;
+constexpr int kTmRows = 8;     // rows of a thread in tensor memory: 512 columns / 8 warps a lane quarter / 8 words
+constexpr int kNT = 1024;
+// weights: real, all +1, or +-1
+enum { RS_REAL = 0, RS_POS = 1, RS_PM1 = 2 };
 
-// Merge the CTA's 8 bits (at bit offset sh) into a global plane word.
-__device__ __forceinline__ void plane_put8(uint32_t *p, uint32_t bits, int sh)
+// A row's eight state words (x then y) in tensor memory, one column each.
+// The load waits for its own data; stores are waited for once a step.
+__device__ __forceinline__ void tm_ld(uint32_t ta, uint4 &a, uint4 &b)
 {
-    const uint32_t m = 0xffu << sh;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "r"(ta)
+                 : "memory");
+}
+__device__ __forceinline__ void tm_st(uint32_t ta, const uint4 &a, const uint4 &b)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(ta), "r"(a.x),
+                 "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Merge the CTA's KA bits (at bit offset sh) into a global plane word.
+template <int KA> __device__ __forceinline__ void plane_put(uint32_t *p, uint32_t bits, int sh)
+{
+    const uint32_t m = ((1u << KA) - 1u) << sh;
     atomicAnd(p, ~m);
     atomicOr(p, (bits << sh) & m);
 }
@@ -139,24 +167,50 @@ __device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32
     hi ^= t >> 4;
 }
 
-// One SB step of slot s's 8 agents held in xv, yv (16-bit, packed); the new
-// signs as a byte.
+// The update of a row's agents; the new signs as a byte.
 template <class T>
-__device__ __forceinline__ uint32_t row_step(const RsP &P, int s, uint4 &xv, uint4 &yv, uint32_t S, const float4 &c)
+__device__ __forceinline__ uint32_t update_row(uint4 &xv, uint4 &yv, const float (&tv)[8], float c0, const float4 &c)
 {
+    uint32_t x[4] = {xv.x, xv.y, xv.z, xv.w}, y[4] = {yv.x, yv.y, yv.z, yv.w}, m0, m1;
+    sb_update16<T, K_FUSED, false, 8>(x, y, tv, c0, c, c);
+    xv = make_uint4(x[0], x[1], x[2], x[3]);
+    yv = make_uint4(y[0], y[1], y[2], y[3]);
+    sign_masks(x, m0, m1);
+    return sign_byte(m0, m1);
+}
+template <>
+__device__ __forceinline__ uint32_t update_row<float>(uint4 &xv, uint4 &yv, const float (&tv)[8], float c0,
+                                                      const float4 &c)
+{
+    float x[4], y[4];
+    const float t[4] = {tv[0], tv[1], tv[2], tv[3]};
+    memcpy(x, &xv, 16);
+    memcpy(y, &yv, 16);
+    sb_update<K_FUSED, false, 4>(x, y, t, c0, c, c);
+    memcpy(&xv, x, 16);
+    memcpy(&yv, y, 16);
+    const uint32_t m0 = __byte_perm(prmt<0x00fb>(xv.x, xv.y), prmt<0x00fb>(xv.z, xv.w), 0x5410);
+    return (uint32_t)__dp4a((int)m0, (int)0xf8fcfeffu, 0);
+}
+
+// Force totals of slot s's agents (s < n; a lane past the rows repeats the
+// last one's degree: its result is not kept).
+template <class T, int MODE>
+__device__ __forceinline__ void row_force(const RsP &P, int s, uint32_t S, float (&tv)[8])
+{
+    constexpr int KA = kAgents<T>;
     const int sl = s >> 5, lane = s & 31;
     const int32_t b0 = __ldg(&P.off[sl]), nb = __ldg(&P.off[sl + 1]) - b0;   // warp-uniform
     const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
-    float tv[KA];
-    if (P.unit) {
+    if (MODE != RS_REAL) {
         uint32_t lo = 0, hi = 0;
-        const bool neg = !P.allpos;
+        constexpr bool neg = MODE == RS_PM1;
         if (nb == 1) count_blocks<1>(cp, nb, S, neg, lo, hi);
         else if (nb < 8) count_blocks<3>(cp, nb, S, neg, lo, hi);
         else count_blocks<6>(cp, nb, S, neg, lo, hi);   // degree <= 127: at most 32 blocks
         // PRMT builds the float 2^23 + 2 count; minus 2^23 + degree it is the
         // force 2 count - degree, exactly
-        const float b = -(8388608.0f + (float)__ldg(&P.deg[s]));
+        const float b = -(8388608.0f + (float)__ldg(&P.deg[min(s, P.n - 1)]));
         const float2 bias = make_float2(b, b);
 #pragma unroll
         for (int v = 0; v < KA; v += 2) {
@@ -184,27 +238,22 @@ __device__ __forceinline__ uint32_t row_step(const RsP &P, int s, uint4 &xv, uin
             }
         }
     }
-    uint32_t x[4] = {xv.x, xv.y, xv.z, xv.w}, y[4] = {yv.x, yv.y, yv.z, yv.w}, m0, m1;
-    sb_update16<T, K_FUSED, false, KA>(x, y, tv, P.c0, c, c);
-    xv = make_uint4(x[0], x[1], x[2], x[3]);
-    yv = make_uint4(y[0], y[1], y[2], y[3]);
-    sign_masks(x, m0, m1);
-    return sign_byte(m0, m1);
 }
 
-template <class T, int NT, int RR>
-__global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
+template <class T, int MODE>
+__global__ void __launch_bounds__(kNT, 1) k_resident_rs(const RsP P)
 {
-    static_assert(sizeof(T) == 2, "16-bit state: 8 agents in 16 bytes");
+    constexpr int KA = kAgents<T>, NT = kNT;
+    constexpr uint32_t KM = (1u << KA) - 1u;
     extern __shared__ __align__(16) unsigned char smem[];
     const int n = P.n;
-    const int ns = n > RR * NT ? n - RR * NT : 0;   // rows kept in shared memory
+    const int ns = n > kTmRows * NT ? n - kTmRows * NT : 0;   // rows kept in shared memory
     uint4 *xs = (uint4 *)smem;
     uint4 *ys = xs + ns;
     uint8_t *Sb0 = (uint8_t *)(ys + ns);
     uint8_t *Sb1 = Sb0 + n + 1;   // one byte more each: the zero row
     uint8_t *Wb = Sb1 + n + 1;
-    __shared__ uint32_t s_chg, s_new, s_stop;
+    __shared__ uint32_t s_chg, s_new, s_stop, s_tmem;
     __shared__ int32_t s_stab[KA];
     __shared__ uint8_t s_bif[KA], s_prev[KA];
 
@@ -237,48 +286,76 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
         return;
     }
 
+    // All of the SM's tensor memory: 1,024 threads of 64 registers leave room
+    // for no second CTA that would wait for it.
+    const int warp = tid >> 5;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(512u));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    // this warp's lane quarter and columns
+    const uint32_t tw = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(8 * kTmRows * (warp >> 2));
+    // a row's state: tensor memory (whole warps), then shared memory
+    auto get_row = [&](int i, int s, uint4 &xv, uint4 &yv) {
+        if (i < kTmRows) {
+            tm_ld(tw + 8u * (uint32_t)i, xv, yv);
+        } else if (s < n) {
+            xv = xs[s - kTmRows * NT];
+            yv = ys[s - kTmRows * NT];
+        }
+    };
+    auto put_row = [&](int i, int s, const uint4 &xv, const uint4 &yv) {
+        if (i < kTmRows) {
+            tm_st(tw + 8u * (uint32_t)i, xv, yv);
+        } else if (s < n) {
+            xs[s - kTmRows * NT] = xv;
+            ys[s - kTmRows * NT] = yv;
+        }
+    };
+    // this warp's slots: i * NT + 32 * warp + lane while any is a row
+    const int w0 = 32 * warp;
+
     // Load the state (the pre-step Update_XY at step 0, src/ising.cu:188, as
     // the streaming pre-step computes it) and the sign words of step k0.
     const int32_t k0 = P.step0;
     uint8_t *Scur = (k0 & 1) ? Sb1 : Sb0;
-    uint4 xr[RR > 0 ? RR : 1], yr[RR > 0 ? RR : 1];
     const float4 c00 = P.coef[0];
-    auto load_row = [&](int s, uint4 &xv, uint4 &yv) {
-        const int r = __ldg(&P.perm[s]);
-        xv = *(const uint4 *)(xg + (int64_t)r * P.Ap + a0);
-        yv = *(const uint4 *)(yg + (int64_t)r * P.Ap + a0);
-        Raw<16> xw, yw;
-        xw.u = xv;
-        yw.u = yv;
-        float x[KA], y[KA];
-        to_vals<T, KA>(xw, x);
-        to_vals<T, KA>(yw, y);
-        if (P.first) {
-#pragma unroll
-            for (int v = 0; v < KA; v++) {
-                y[v] = fmaf(c00.w, x[v], y[v]);
-                x[v] = fmaf(c00.z, y[v], x[v]);
-            }
-            xv = from_vals<T, KA>(x).u;
-            yv = from_vals<T, KA>(y).u;
-        }
-        uint32_t bits = 0;
-#pragma unroll
-        for (int v = 0; v < KA; v++) bits |= sbit(x[v]) << v;
-        Scur[s] = (uint8_t)bits;
-        Wb[s] = (uint8_t)((P.Wp[(int64_t)r * P.W + wg] >> sh) & 0xffu);
-    };
-#pragma unroll
-    for (int i = 0; i < RR; i++) {
+    for (int i = 0; i * NT + w0 < n; i++) {
         const int s = i * NT + tid;
-        if (s < n) load_row(s, xr[i], yr[i]);
+        uint4 xv = make_uint4(0, 0, 0, 0), yv = xv;
+        if (s < n) {
+            const int r = __ldg(&P.perm[s]);
+            xv = *(const uint4 *)(xg + (int64_t)r * P.Ap + a0);
+            yv = *(const uint4 *)(yg + (int64_t)r * P.Ap + a0);
+            Raw<16> xw, yw;
+            xw.u = xv;
+            yw.u = yv;
+            float x[KA], y[KA];
+            to_vals<T, KA>(xw, x);
+            to_vals<T, KA>(yw, y);
+            if (P.first) {
+#pragma unroll
+                for (int v = 0; v < KA; v++) {
+                    y[v] = fmaf(c00.w, x[v], y[v]);
+                    x[v] = fmaf(c00.z, y[v], x[v]);
+                }
+                xv = from_vals<T, KA>(x).u;
+                yv = from_vals<T, KA>(y).u;
+            }
+            uint32_t bits = 0;
+#pragma unroll
+            for (int v = 0; v < KA; v++) bits |= sbit(x[v]) << v;
+            Scur[s] = (uint8_t)bits;
+            Wb[s] = (uint8_t)((P.Wp[(int64_t)r * P.W + wg] >> sh) & KM);
+        }
+        put_row(i, s, xv, yv);
     }
-    for (int s = RR * NT + tid; s < n; s += NT) {
-        uint4 xv, yv;
-        load_row(s, xv, yv);
-        xs[s - RR * NT] = xv;
-        ys[s - RR * NT] = yv;
-    }
+    tm_wait_st();
     __syncthreads();
 
     const uint32_t sa0 = smem_u32(Sb0), sa1 = smem_u32(Sb1);
@@ -290,11 +367,15 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
         const bool win = ((k + 1) % P.period) == 0;
         const float4 ck = P.coef[k];
         uint32_t chg = 0;
-#pragma unroll
-        for (int i = 0; i < RR; i++) {
+        for (int i = 0; i * NT + w0 < n; i++) {
             const int s = i * NT + tid;
+            float tv[8];
+            row_force<T, MODE>(P, s, Sin, tv);
+            uint4 xv = make_uint4(0, 0, 0, 0), yv = xv;
+            get_row(i, s, xv, yv);
+            const uint32_t nb = update_row<T>(xv, yv, tv, P.c0, ck);
+            put_row(i, s, xv, yv);
             if (s < n) {
-                const uint32_t nb = row_step<T>(P, s, xr[i], yr[i], Sin, ck);
                 Snx[s] = (uint8_t)nb;
                 if (win) {
                     chg |= nb ^ Wb[s];
@@ -302,17 +383,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
                 }
             }
         }
-        for (int s = RR * NT + tid; s < n; s += NT) {
-            uint4 xv = xs[s - RR * NT], yv = ys[s - RR * NT];
-            const uint32_t nb = row_step<T>(P, s, xv, yv, Sin, ck);
-            xs[s - RR * NT] = xv;
-            ys[s - RR * NT] = yv;
-            Snx[s] = (uint8_t)nb;
-            if (win) {
-                chg |= nb ^ Wb[s];
-                Wb[s] = (uint8_t)nb;
-            }
-        }
+        tm_wait_st();
         if (win) {
             // per-agent window bookkeeping inside the CTA, src/kernels.cu:46-79
             chg = __reduce_or_sync(FULL, chg);
@@ -330,8 +401,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
                 s_prev[tid] = b;
                 s_bif[tid] = b;
                 s_stab[tid] = st;
-                const uint32_t nm = __ballot_sync(0xffu, newb && a < P.A);
-                const uint32_t bm = __ballot_sync(0xffu, b && a < P.A);
+                const uint32_t nm = __ballot_sync(KM, newb && a < P.A);
+                const uint32_t bm = __ballot_sync(KM, b && a < P.A);
                 if (tid == 0) {
                     s_new = nm;
                     if (P.uw) atomicAdd(&P.wincount[(k + 1) / P.period - 1], __popc(bm));
@@ -383,21 +454,17 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
     }
 
     // write the state back (chunked runs continue from it; get_state reads it)
-#pragma unroll
-    for (int i = 0; i < RR; i++) {
+    for (int i = 0; i * NT + w0 < n; i++) {
         const int s = i * NT + tid;
+        uint4 xv = make_uint4(0, 0, 0, 0), yv = xv;
+        get_row(i, s, xv, yv);
         if (s < n) {
             const int r = __ldg(&P.perm[s]);
-            *(uint4 *)(xg + (int64_t)r * P.Ap + a0) = xr[i];
-            *(uint4 *)(yg + (int64_t)r * P.Ap + a0) = yr[i];
+            *(uint4 *)(xg + (int64_t)r * P.Ap + a0) = xv;
+            *(uint4 *)(yg + (int64_t)r * P.Ap + a0) = yv;
         }
     }
-    for (int s = RR * NT + tid; s < n; s += NT) {
-        const int r = __ldg(&P.perm[s]);
-        *(uint4 *)(xg + (int64_t)r * P.Ap + a0) = xs[s - RR * NT];
-        *(uint4 *)(yg + (int64_t)r * P.Ap + a0) = ys[s - RR * NT];
-    }
-    for (int s = tid; s < n; s += NT) plane_put8(&P.Wp[(int64_t)__ldg(&P.perm[s]) * P.W + wg], Wb[s], sh);
+    for (int s = tid; s < n; s += NT) plane_put<KA>(&P.Wp[(int64_t)__ldg(&P.perm[s]) * P.W + wg], Wb[s], sh);
     if (tid < KA) {
         const int a = a0 + tid;
         P.stab[a] = s_stab[tid];
@@ -409,42 +476,37 @@ __global__ void __launch_bounds__(NT, 1) k_resident_rs(const RsP P)
         P.ctl[CTL_WINDOWS] = (P.step0 + nrun) / P.period;
         if (s_stop == 2) P.ctl[CTL_STOP] = 1;
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
-// Configurations (threads per CTA, register rows per thread), fewest
-// registers first.
-struct RsCfg {
-    int nt, rr;
-};
-constexpr RsCfg kRsCfgs[] = {{1024, 0}, {1024, 2}, {1024, 4}};
-
-size_t rs_smem(int64_t n, const RsCfg &c)
+// shared memory of n rows: those past tensor memory's, and three bytes each
+size_t rs_smem(int64_t n)
 {
-    const int64_t ns = n > (int64_t)c.rr * c.nt ? n - (int64_t)c.rr * c.nt : 0;
+    const int64_t ns = n > (int64_t)kTmRows * kNT ? n - (int64_t)kTmRows * kNT : 0;
     return (size_t)ns * 32 + (size_t)n * 3 + 2;
 }
 
-template <class T, int NT, int RR>
-cudaError_t launch_rs_t(const RsP &P, size_t smem, int grid, cudaStream_t s, bool pdl)
+template <class T, int MODE>
+cudaError_t launch_rs_m(const RsP &P, size_t smem, int grid, cudaStream_t s, bool pdl)
 {
+    auto kern = k_resident_rs<T, MODE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
     if (P.coop) {
         // every CTA must be resident at once for the window barrier
-        int per_sm = 0, nsm = 0, dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaError_t e = cudaFuncSetAttribute(k_resident_rs<T, NT, RR>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident_rs<T, NT, RR>, NT, smem);
+        int per_sm = 0;
+        const int nsm = dev_attr(cudaDevAttrMultiProcessorCount);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kNT, smem);
         if (e != cudaSuccess) return e;
-        if ((int64_t)per_sm * nsm < grid) return cudaErrorCooperativeLaunchTooLarge;
+        // one CTA an SM: it holds all of the SM's tensor memory
+        if ((int64_t)std::min(per_sm, 1) * nsm < grid) return cudaErrorCooperativeLaunchTooLarge;
     }
-    cudaError_t e = cudaFuncSetAttribute(k_resident_rs<T, NT, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NT);
+    cfg.blockDim = dim3(kNT);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -457,49 +519,46 @@ cudaError_t launch_rs_t(const RsP &P, size_t smem, int grid, cudaStream_t s, boo
     }
     cfg.attrs = at;
     cfg.numAttrs = (pdl || P.coop) ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_resident_rs<T, NT, RR>, P);
+    return cudaLaunchKernelEx(&cfg, kern, P);
 }
 
 template <class T>
-cudaError_t launch_rs_cfg(int ci, const RsP &P, size_t smem, int grid, cudaStream_t s, bool pdl)
+cudaError_t launch_rs_t(const DevCsr &J, const RsP &P, size_t smem, cudaStream_t s, bool pdl)
 {
-    switch (ci) {
-    case 0: return launch_rs_t<T, 1024, 0>(P, smem, grid, s, pdl);
-    case 1: return launch_rs_t<T, 1024, 2>(P, smem, grid, s, pdl);
-    default: return launch_rs_t<T, 1024, 4>(P, smem, grid, s, pdl);
-    }
+    const int grid = (P.A + kAgents<T> - 1) / kAgents<T>;
+    if (!J.unit) return launch_rs_m<T, RS_REAL>(P, smem, grid, s, pdl);
+    if (J.allpos) return launch_rs_m<T, RS_POS>(P, smem, grid, s, pdl);
+    return launch_rs_m<T, RS_PM1>(P, smem, grid, s, pdl);
 }
 
 }  // namespace
 
 int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced)
 {
-    if (d.prec != P_BF16 && d.prec != P_F16) return 0;
+    const bool half = d.prec == P_BF16 || d.prec == P_F16;
+    if (!half && (forced || d.prec != P_F32)) return 0;
     if (!d.fused || d.n > (1 << 24)) return 0;
-    if (J.unit && J.max_deg > kHeavy) return 0;   // byte counters hold 127 neighbours
-    int dev = 0, smax = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (J.unit && J.max_deg > kHeavy) return 0;   // the planes hold 127 neighbours
+    const int nsm = dev_attr(cudaDevAttrMultiProcessorCount);
+    const int64_t budget = (int64_t)dev_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024;
+    // asked for: the rows that four a thread in registers and shared memory
+    // hold (what the entry point has always taken)
+    if (forced) return std::max<int64_t>(0, d.n - 4096) * 32 + d.n * 3 <= budget ? 8 : 0;
     // one CTA per SM: chosen by itself only when the agents fill half the SMs
-    if (!forced && (d.A + KA - 1) / KA < nsm / 2) return 0;
-    const size_t budget = (size_t)smax - 1024;
-    for (int i = 0; i < (int)(sizeof kRsCfgs / sizeof kRsCfgs[0]); i++)
-        if (rs_smem(d.n, kRsCfgs[i]) <= budget) return i + 1;
-    return 0;
+    const int ka = half ? 8 : 4;
+    if ((d.A + ka - 1) / ka < nsm / 2) return 0;
+    return (int64_t)rs_smem(d.n) <= budget ? ka : 0;
 }
 
-cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int cfg, int32_t step0,
+cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int ka, int32_t step0,
                                int32_t nsteps, bool first, bool coop, cudaStream_t s)
 {
-    if (cfg < 1) return cudaErrorInvalidValue;
     RsP P;
-    if (!J.sell[1].base) return cudaErrorInvalidValue;
+    if (ka < 1 || !J.sell[1].base) return cudaErrorInvalidValue;
     P.off = J.sell[1].off;
     P.deg = J.sell[1].deg;
     P.col = J.sell[1].col;
     P.val = J.sell[1].val;
-    P.allpos = J.allpos ? 1 : 0;
     P.perm = J.perm;
     P.coef = (const float4 *)w.coef32;
     P.x = w.x;
@@ -523,13 +582,13 @@ cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int
     P.step0 = step0;
     P.nsteps = nsteps;
     P.first = first ? 1 : 0;
-    P.unit = J.unit ? 1 : 0;
     P.c0 = (float)d.c0;
     P.giveup = d.giveup;
-    const size_t smem = rs_smem(d.n, kRsCfgs[cfg - 1]);
-    const int grid = (d.A + KA - 1) / KA;
-    if (d.prec == P_BF16) return launch_rs_cfg<__nv_bfloat16>(cfg - 1, P, smem, grid, s, d.pdl);
-    return launch_rs_cfg<__half>(cfg - 1, P, smem, grid, s, d.pdl);
+    const size_t smem = rs_smem(d.n);
+    if (d.prec == P_BF16) return launch_rs_t<__nv_bfloat16>(J, P, smem, s, d.pdl);
+    if (d.prec == P_F16) return launch_rs_t<__half>(J, P, smem, s, d.pdl);
+    if (d.prec == P_F32) return launch_rs_t<float>(J, P, smem, s, d.pdl);
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace sbx
