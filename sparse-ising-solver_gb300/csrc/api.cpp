@@ -517,17 +517,22 @@ bool state_exceeds_half_l2(const SolveDims &d)
 }
 
 // A tile the step kernels are built for (k_step.cuh, step_kw): whole-warp
-// rows take any vector width dividing the padded agents; 16, 8 or 4 lanes
-// per row take the two widest vectors and exactly the padded agents, and
-// rows with split heavy neighbour lists need whole-warp rows.
-bool tile_ok(const SolveDims &d, bool big, int v, int lr, int bt)
+// rows take any vector width; 16, 8 or 4 lanes per row take the two widest
+// vectors, and rows with split heavy neighbour lists need whole-warp rows.
+// exact (the caller names lane_agents or row_lanes): the row's lanes hold the
+// padded agents exactly.  Otherwise lanes of the two widest vectors may be left
+// over, fewer than half of them: an odd number of 32-agent words walked one agent a lane was three
+// to four times slower (torus 100x100, 608 agents, BF16: 42 us a step).
+bool tile_ok(const SolveDims &d, bool big, int v, int lr, int bt, bool exact)
 {
     const int vm = 16 / (int)prec_bytes(d.prec);
     if ((v != 1 && v != 2 && v != 4 && v != 8) || v > vm) return false;
     if (bt != 128 && bt != 256) return false;
-    if (lr == 32) return d.Ap % (32 * v) == 0;
+    const int width = lr * v, held = (d.Ap + width - 1) / width * width;
+    if (held != d.Ap && (exact || held >= 2 * d.Ap || v < 2 || v < vm / 2)) return false;
+    if (lr == 32) return true;
     if (lr != 16 && lr != 8 && lr != 4) return false;
-    return !big && (v == vm || v == vm / 2) && v * lr == d.Ap;
+    return !big && (v == vm || v == vm / 2) && held == width && width >= 32;
 }
 
 int default_v(const SolveDims &d)
@@ -561,7 +566,7 @@ int pick_tile(sbx_ctx *ctx, SolveDims &d, const DevCsr &J, const sbx_params *pr,
                     if ((fv && v != fv) || (flr && lr != flr) || (fbt && bt != fbt) || (fcm && cm != fcm - 1))
                         continue;
                     if (st_forced && lr != 32) continue;
-                    if (tile_ok(d, big, v, lr, bt)) cands.push_back(Tile{v, lr, bt, cm, st_forced});
+                    if (tile_ok(d, big, v, lr, bt, fv || flr || st_forced)) cands.push_back(Tile{v, lr, bt, cm, st_forced});
                 }
     if (cands.empty())
         return fail(ctx, SBX_ERR_ARG, "no streaming tile fits lane_agents / row_lanes / block_threads / count_mode");
@@ -620,7 +625,7 @@ int pick_tile(sbx_ctx *ctx, SolveDims &d, const DevCsr &J, const sbx_params *pr,
         if (best[i] < best[bi]) bi = i;
     Tile win = cands[bi];
     // staged rows: tried on the winning tile only, when the state streams
-    if (!fst && can_stage && win.lr == 32 && !win.st) {
+    if (!fst && can_stage && win.lr == 32 && !win.st && d.Ap % (32 * win.v) == 0) {
         Tile t = win;
         t.st = 1;
         float bs = 1e30f;

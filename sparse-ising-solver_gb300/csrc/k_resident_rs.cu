@@ -544,10 +544,24 @@ int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced)
     // asked for: the rows that four a thread in registers and shared memory
     // hold (what the entry point has always taken)
     if (forced) return std::max<int64_t>(0, d.n - 4096) * 32 + d.n * 3 <= budget ? 8 : 0;
-    // one CTA per SM: chosen by itself only when the agents fill half the SMs
     const int ka = half ? 8 : 4;
-    if ((d.A + ka - 1) / ka < nsm / 2) return 0;
-    return (int64_t)rs_smem(d.n) <= budget ? ka : 0;
+    if ((int64_t)rs_smem(d.n) > budget) return 0;
+    // Chosen by itself where its step (microseconds) is the shorter one.  Both
+    // sides fitted on GB300 over 5,900 to 9,900 rows, 200 to 1,024 agents and
+    // mean degrees 4 to 40: waves of one CTA an SM, each a cost per row that
+    // grows with the degree (FP32: 0.83 ns at degree 4, 1.65 at 16, 2.9 at
+    // 40), against the streaming step's cost per row and agent (FP32 2.1 to
+    // 3.2 ps, 16 bits 1.45 to 2.45) and its latency.  E.g. 6,000 rows, FP32,
+    // 1,024 agents: 9.8 us a step against 16.1 at degree 4, 24.8 against 21.1
+    // at degree 24.
+    const double n = (double)d.n, deg = (double)J.nnz / n;
+    const double waves = (double)(((d.A + ka - 1) / ka + nsm - 1) / nsm);
+    const double per_row = half ? (deg <= 4 ? 1.0 : 1.1 + 0.047 * deg) : (deg <= 4 ? 0.83 : 0.86 + 0.051 * deg);
+    const double more = deg > 24 ? deg - 24 : 0;
+    const double per_cell = half ? (deg <= 4 ? 1.45 : 2.0 + 0.03 * more) : (deg <= 4 ? 2.1 : 2.65 + 0.035 * more);
+    const double res = waves * (n * per_row * 1e-3 + 0.3);
+    const double str = (half ? 3.0 : 4.0) + n * ((d.A + 127) / 128 * 128) * per_cell * 1e-6;
+    return res < str ? ka : 0;
 }
 
 cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int ka, int32_t step0,

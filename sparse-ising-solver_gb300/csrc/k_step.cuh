@@ -619,12 +619,14 @@ __device__ __forceinline__ uint32_t sign_byte(uint32_t m0, uint32_t m1)
 // 4 for bit-plane counting without heavy rows (its loads in flight need
 // registers), 5 otherwise (heavy-row kernels: 6 spilled more and ran 2%
 // slower on R-MAT 2^20, 7 ran 11% slower).
-template <class T, int V, int KIND, bool WIN, int WM, bool BIG, int LR, int CM, int ST>
+// RAG: the lanes of a row's last segment hold more agents than the row has.
+template <class T, int V, int KIND, bool WIN, int WM, bool BIG, int LR, int CM, int ST, bool RAG>
 __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P, const int offset)
 {
     static_assert(LR == 32 || !BIG, "heavy rows are counted by whole warps");
     static_assert(!ST || (LR == 32 && !WIN && KIND != K_XY), "staged rows: whole-warp rows, plain steps");
     static_assert(LR * V >= 32, "a sign word belongs to one row's lanes");
+    static_assert(!RAG || (!ST && KIND != K_XY), "left-over lanes: direct steps");
     using A = typename St<T>::A;
     using R = typename std::conditional<WM == W_F64, double, float>::type;
     using RawT = Raw<V * sizeof(T)>;
@@ -652,7 +654,10 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
     constexpr int RW = 32 / LR; // rows per warp
     constexpr uint32_t VM = (V == 32) ? 0xffffffffu : ((1u << V) - 1u);
     const int rw = lane / LR, sl = lane & (LR - 1);   // row of the warp, lane of the row
-    const int nit = P.Ap / (LR * V);                  // segments per row (1 when LR < 32)
+    // segments per row (1 when LR < 32); RAG: lanes past the row's agents in
+    // its last segment repeat its last vector (no extra sectors) and store
+    // nothing.  (A variant of its own: the test costs full tiles 3 to 5%.)
+    const int nit = (P.Ap + LR * V - 1) / (LR * V);
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     const int64_t w0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 
@@ -712,7 +717,7 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             const int32_t h0 = __ldg(&P.hchunk[r]);
             const int32_t rb = __ldg(&P.rowptr[r]), re = __ldg(&P.rowptr[r + 1]);
             const int32_t e0 = rb + (ci - h0) * kHeavy;
-            const int a0 = it * 32 * V + lane * V;
+            const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
             const int q = a0 >> 5, off = a0 & 31;
             uint32_t lo = 0, hi = 0;
             count_bits<V, 32>(P, Scur + q, off, e0, min(re - e0, (int32_t)kHeavy), lane, lo, hi);
@@ -741,7 +746,7 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             if (WIN && (lane & (G - 1)) == 0) wp_old = P.Wp[r * P.W + q];
             const RawT xr = vload_s<T, V>(xp + base, cs);
             const RawT yr = vload_s<T, V>(yp + base, cs);
-            finish(r, q, off, base, true, xr, yr, tv, row_c0(r), wp_old);
+            finish(r, q, off, base, !RAG || a1 == a0, xr, yr, tv, row_c0(r), wp_old);
         }
     }
 
@@ -896,10 +901,11 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
         }
         // lanes of a group past the last row repeat the last row, store nothing
         const int32_t gi = g * RW + rw;
-        const bool live = RW == 1 || gi < nr32;
-        const int32_t ri = row0 + (live ? gi : nr32 - 1);
+        const bool row = RW == 1 || gi < nr32;
+        const int32_t ri = row0 + (row ? gi : nr32 - 1);
         const int32_t r = P.order ? __ldg(&P.order[ri]) : ri;
-        const int a0 = it * LR * V + sl * V;
+        const int a1 = it * LR * V + sl * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
+        const bool live = row && (!RAG || a1 == a0);
         const int q = a0 >> 5, off = a0 & 31;
         const int64_t base = (int64_t)r * P.Ap + a0;
         uint32_t wp_old = 0;   // window steps: the previous window's word, fetched early
@@ -962,14 +968,15 @@ cudaError_t launch_grid(K kern, const SolveDims &d, int64_t items, int bt, size_
     return launch(kern, dim3((unsigned)blocks), dim3(bt), smem, s, d.pdl, P, offset);
 }
 
-// One step with V agents per lane and LR lanes per row.
-template <class T, int V, int LR, int KIND, bool WIN>
-cudaError_t step_vl(const SolveDims &d, const DevCsr &J, const StepP &P, int offset, cudaStream_t s)
+// One step with V agents per lane and LR lanes per row (RAG: more than the
+// row's agents).
+template <class T, int V, int LR, int KIND, bool WIN, bool RAG>
+cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int offset, cudaStream_t s)
 {
     constexpr int RW = 32 / LR;
     const size_t smem = WIN ? sizeof(uint32_t) * d.W : 0;
     const int bt = d.tbt;
-    const int nit = d.Ap / (LR * V);
+    const int nit = (d.Ap + LR * V - 1) / (LR * V);
     const bool big = J.unit && J.nchunks > 0 && KIND != K_XY;
     // Row order: heavy rows first (their chunk items), then the rest in
     // decreasing degree when rows differ much in length or share a warp.
@@ -990,40 +997,50 @@ cudaError_t step_vl(const SolveDims &d, const DevCsr &J, const StepP &P, int off
     // only); staged rows (x, y copied ahead into shared memory) for
     // whole-warp rows of plain steps
     const bool cm = d.tcm == 1;
-    constexpr bool can_st = LR == 32 && !WIN && KIND != K_XY;
+    constexpr bool can_st = LR == 32 && !WIN && KIND != K_XY && !RAG;
     const bool st = can_st && d.tst != 0 && J.unit;
     const size_t smem_st = (size_t)(bt / 32) * 4 * 32 * V * sizeof(T);
     if constexpr (LR == 32) {
         if (big) {
             if constexpr (can_st) {
                 if (st) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 1>, d, items, bt, smem_st, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1>, d, items, bt, smem_st, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 1, false>, d, items, bt, smem_st, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1, false>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
-            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0>, d, items, bt, smem, s, Q, offset);
-            return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0>, d, items, bt, smem, s, Q, offset);
+            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG>, d, items, bt, smem, s, Q, offset);
+            return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
         }
     } else {
         if (big) return cudaErrorInvalidValue;
     }
-    if (KIND == K_XY) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0>, d, items, bt, smem, s, Q, offset);
+    if (KIND == K_XY) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
     if (J.unit) {
         if constexpr (KIND != K_XY) {
             if constexpr (can_st) {
                 if (st) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 1>, d, items, bt, smem_st, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 1>, d, items, bt, smem_st, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 1, false>, d, items, bt, smem_st, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 1, false>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
-            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 0>, d, items, bt, smem, s, Q, offset);
+            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 0, RAG>, d, items, bt, smem, s, Q, offset);
         }
-        return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
     }
     if constexpr (sizeof(T) == 8)
-        return launch_grid(k_row<T, V, KIND, WIN, W_F64, false, LR, 0, 0>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_F64, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
     else
-        return launch_grid(k_row<T, V, KIND, WIN, W_F32, false, LR, 0, 0>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_F32, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
+}
+
+template <class T, int V, int LR, int KIND, bool WIN>
+cudaError_t step_vl(const SolveDims &d, const DevCsr &J, const StepP &P, int offset, cudaStream_t s)
+{
+    // left-over lanes come with the two widest vectors (tile_ok)
+    if constexpr (KIND != K_XY && V >= 2 && V * (int)sizeof(T) >= 8)
+        if (d.Ap % (LR * V)) return step_vlr<T, V, LR, KIND, WIN, true>(d, J, P, offset, s);
+    if (d.Ap % (LR * V)) return cudaErrorInvalidValue;
+    return step_vlr<T, V, LR, KIND, WIN, false>(d, J, P, offset, s);
 }
 
 // Agents per lane by default: a 16-byte vector when the padded agent count
@@ -1036,9 +1053,9 @@ template <class T> int pick_v(int Ap)
 }
 
 // The tile (d.tv agents per lane, d.tlr lanes per row) picks the kernel.
-// Whole-warp rows take any V that divides the padded agent count; fewer
-// lanes per row are built for the two widest vectors (VM, VM/2) and need
-// LR*V = Ap.  The host validates tiles (tile_ok) before they get here.
+// Whole-warp rows take any V; fewer lanes per row are built for the two widest
+// vectors (VM, VM/2) and need LR*V >= Ap.  The host validates tiles (tile_ok)
+// before they get here.
 template <class T, int KIND, bool WIN>
 cudaError_t step_kw(const SolveDims &d, const DevCsr &J, const StepP &P, int offset, cudaStream_t s)
 {
