@@ -8,10 +8,17 @@
 //   (J x)[i][k] = C/4 colsum[k] + B/4 rowsum[i] + A/8 sum_l d_kl (x[i-1][l] + x[i+1][l])
 // (the diagonal cancels the self terms of the two penalty sums; for N = 2 the
 // two neighbours are one position).  A CTA owns KA agents and keeps their x in
-// shared memory for the whole run: per step each thread (position i, agent a)
-// gathers the two neighbouring rows, one pass computes every row and column
-// sum, and the 30x30 distance product runs from shared memory on the FP32
-// pipes.  No CTA talks to another, so the whole solve is one launch.
+// shared memory for the whole run.  H threads share a (position i, agent a)
+// row's cities: each reads the two neighbouring rows and multiplies them with
+// its cities' distances, while one part also sums its row and one its
+// column; after a barrier each updates its cities.  The distances are
+// constant operands of the multiply-adds (a kernel parameter, addressed at
+// compile time: warp w takes part w mod H, so a scheduler's warps share one
+// part's kilobyte).  No CTA talks to another, so the whole solve is one
+// launch.  Bound: issue (5 FP32 operations per 4 products).  29 cities x 1,000
+// agents: 6.0 us a step with one thread a row, 4.2 with four and the distances
+// in shared memory (a 16-byte shared load takes four cycles even when all
+// lanes share its address).
 //
 // Streaming kernel.  The CSR form of the same QUBO, one launch per step, x
 // double-buffered (Jacobi); used in FP64 (which it reproduces operation by
@@ -24,7 +31,6 @@ namespace sbx {
 namespace {
 
 struct TspP {
-    const float *__restrict__ D;      // [N][N] distances, zero diagonal
     const float *__restrict__ I2;     // [N] linear field per city
     const float2 *__restrict__ sched; // per step: b_t, dt*-(1-a_t)
     void *x, *y;                      // global [n][Ap], n = N*N, row = i*N + k
@@ -40,40 +46,68 @@ struct TspP {
 
 template <class T> __device__ __forceinline__ float rnd(float v) { return St<T>::ld(St<T>::st(v)); }
 
-template <class T, int NP>
-__global__ void __launch_bounds__(512) k_tsp_resident(const TspP P, const int KA)
+template <int NP> struct TspD {
+    float d[NP * NP];   // distances, zero past the cities
+};
+
+// Cities [K0, K0 + CPT) of the distance product of a row's two neighbours.
+template <int NP, int CPT, int K0>
+__device__ __forceinline__ void dist_product(const TspD<NP> &D, const float *rm, const float *rp, bool two,
+                                             float (&dk)[CPT])
+{
+#pragma unroll
+    for (int j = 0; j < CPT; j++) dk[j] = 0.f;
+#pragma unroll
+    for (int l = 0; l < NP; l += 4) {
+        const float4 m4 = *(const float4 *)&rm[l];
+        const float4 p4 = two ? *(const float4 *)&rp[l] : make_float4(0, 0, 0, 0);
+        const float nb[4] = {m4.x + p4.x, m4.y + p4.y, m4.z + p4.z, m4.w + p4.w};
+#pragma unroll
+        for (int j = 0; j < CPT; j++) {
+            const float *d = &D.d[(K0 + j) * NP + l];
+            dk[j] += d[0] * nb[0] + d[1] * nb[1] + d[2] * nb[2] + d[3] * nb[3];
+        }
+    }
+}
+
+// H parts of a row's NP cities.
+template <class T, int NP, int H>
+__global__ void __launch_bounds__(H == 1 ? 512 : 1024) k_tsp_resident(const TspP P,
+                                                                      const __grid_constant__ TspD<NP> D,
+                                                                      const int KA)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NPS = NP + 4;       // padded row: spreads rows over banks
-    const int N = P.N;
+    constexpr int CPT = NP / H;       // cities of a thread
+    const int N = P.N, rows = N * KA;
     float *xs = (float *)smem;                          // [N][KA][NPS]
-    float *Ds = xs + (size_t)N * KA * NPS;              // [NP][NP]
-    float *colsum = Ds + NP * NP;                       // [NP][KA]
-    uint32_t *rowbits = (uint32_t *)(colsum + NP * KA); // [N][KA]
-    uint32_t *prevbits = rowbits + N * KA;              // [N][KA]
-    int *aflag = (int *)(prevbits + N * KA);            // [KA] valid, [KA] changed
+    float *colsum = xs + (size_t)rows * NPS;            // [KA][NPS]
+    float *rsum = colsum + KA * NPS;                    // [N][KA]
+    uint32_t *rowbits = (uint32_t *)(rsum + rows);      // [N][KA]
+    uint32_t *prevbits = rowbits + rows;                // [N][KA]
+    int *aflag = (int *)(prevbits + rows);              // [KA] valid, [KA] changed
     __shared__ float s_I2[NP];
 
     pdl_wait();
-    const int tid = threadIdx.x;
-    const int i = tid / KA, a = tid - (tid / KA) * KA;  // position, local agent
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int h = warp % H, m = 32 * (warp / H) + (tid & 31);   // part, row
+    const int i = m / KA, a = m - (m / KA) * KA;        // position, local agent
+    const int k0 = CPT * h;                             // first city of this thread
     const int ag = blockIdx.x * KA + a;                 // global agent
-    const bool active = i < N;
+    const bool active = m < rows;
     const bool real = ag < P.A;                         // padded agents compute on zeros
     T *xg = (T *)P.x, *yg = (T *)P.y;
 
-    for (int t = tid; t < NP * NP; t += blockDim.x) {
-        const int k = t / NP, l = t % NP;
-        Ds[t] = (k < N && l < N) ? P.D[k * N + l] : 0.f;
-    }
     for (int t = tid; t < NP; t += blockDim.x) s_I2[t] = t < N ? P.I2[t] : 0.f;
+    for (int t = tid; t < KA * NPS; t += blockDim.x) colsum[t] = 0.f;
 
     // Initial state (x = 0, y from the init stream) and the pre-step
     // Update_XY at step 0 (src/ising_tsp.cu:155).
-    float yr[NP], xo[NP];
-    uint32_t bits0 = 0;
+    float yr[CPT], xo[CPT];
+    float *xrow = &xs[(size_t)m * NPS + k0];
 #pragma unroll
-    for (int k = 0; k < NP; k++) {
+    for (int j = 0; j < CPT; j++) {
+        const int k = k0 + j;
         float x = 0.f, y = 0.f;
         if (active && k < N && real) {
             const int64_t gi = (int64_t)(i * N + k) * P.Ap + ag;
@@ -81,104 +115,137 @@ __global__ void __launch_bounds__(512) k_tsp_resident(const TspP P, const int KA
             y = St<T>::ld(yg[gi]);
             y = rnd<T>(y + P.k2u * x);
             x = rnd<T>(x + P.k1u * y);
-            bits0 |= sbit(x) << k;
         }
-        yr[k] = y;
-        xo[k] = x;
-        if (active) xs[(i * KA + a) * NPS + k] = x;
+        yr[j] = y;
+        xo[j] = x;
+        if (active) xrow[j] = x;
     }
-    if (active) prevbits[i * KA + a] = 0xffffffffu;   // current_spins = -1
+    if (active && h == 0) {
+        prevbits[m] = 0xffffffffu;   // current_spins = -1
+        rowbits[m] = 0;
+    }
     int stab = 0;
     bool bif = false, prv = false;
-    if (active && i == 0 && real) {
+    if (active && i == 0 && h == 0 && real) {
         stab = P.stab[ag];
         bif = P.bif[ag];
         prv = P.prev[ag];
     }
-    (void)bits0;
     __syncthreads();
+    float i2r[CPT];   // the linear field of this thread's cities
+#pragma unroll
+    for (int j = 0; j < CPT; j++) i2r[j] = s_I2[k0 + j];
 
+    const bool whole = k0 + CPT <= N;   // warp-uniform: no city past N
+    // the parts that sum this row and its column: another for the next warp
+    // of rows, so that the schedulers (warp mod 4) share the sums
+    const int hrow = (warp / H) % H, hcol = (warp / H + H / 2) % H;
+    const int im = i == 0 ? N - 1 : i - 1, ip = i + 1 >= N ? 0 : i + 1;
+    const float *rm = &xs[(size_t)(im * KA + a) * NPS], *rp = &xs[(size_t)(ip * KA + a) * NPS];
     const int nwin = P.nwin;
     const uint32_t maskN = N == 32 ? 0xffffffffu : ((1u << N) - 1u);
     int k_step = 0;
     for (int wdx = 0; wdx < nwin; wdx++) {
         for (int it = 0; it < P.period; it++, k_step++) {
             const float2 sc = P.sched[k_step];
-            // Phase 1: read neighbours, row sum, one column sum.
-            float nb[NP];
-            float rs = 0.f;
+            // Phase 1: the distance product of this thread's cities; the sum
+            // of its row and that of city i's column each by one of its parts.
+            float dk[CPT];
             if (active) {
-                const int im = (i + N - 1) % N, ip = (i + 1) % N;
-                const float *rm = &xs[(im * KA + a) * NPS];
-                const float *rp = &xs[(ip * KA + a) * NPS];
+                if (h == 0) dist_product<NP, CPT, 0>(D, rm, rp, N > 2, dk);
+                else if (h == 1) dist_product<NP, CPT, CPT % NP>(D, rm, rp, N > 2, dk);
+                else if (h == 2) dist_product<NP, CPT, 2 * CPT % NP>(D, rm, rp, N > 2, dk);
+                else dist_product<NP, CPT, 3 * CPT % NP>(D, rm, rp, N > 2, dk);
+                if (h == hrow) {
+                    const float *r = &xs[(size_t)m * NPS];
+                    float rs = 0.f;
 #pragma unroll
-                for (int l = 0; l < NP; l += 4) {
-                    const float4 m4 = *(const float4 *)&rm[l];
-                    const float4 p4 = N > 2 ? *(const float4 *)&rp[l] : make_float4(0, 0, 0, 0);
-                    nb[l] = m4.x + p4.x;
-                    nb[l + 1] = m4.y + p4.y;
-                    nb[l + 2] = m4.z + p4.z;
-                    nb[l + 3] = m4.w + p4.w;
+                    for (int l = 0; l < NP; l += 4) {
+                        const float4 x4 = *(const float4 *)&r[l];
+                        rs += x4.x;
+                        rs += x4.y;
+                        rs += x4.z;
+                        rs += x4.w;
+                    }
+                    rsum[m] = rs;
                 }
-#pragma unroll
-                for (int l = 0; l < NP; l++) rs += xo[l];
-                float cs = 0.f;   // column (city) i over all positions
-                for (int p = 0; p < N; p++) cs += xs[(p * KA + a) * NPS + i];
-                colsum[i * KA + a] = cs;
+                if (h == hcol) {
+                    const float *c = &xs[(size_t)a * NPS + i];   // column (city) i over all positions
+                    float cs = 0.f;
+#pragma unroll 8
+                    for (int p = 0; p < N; p++) cs += c[p * KA * NPS];
+                    colsum[a * NPS + i] = cs;
+                }
             }
             __syncthreads();
-            // Phase 2: forces and the bSB update of this thread's N spins.
+            // Phase 2: forces and the bSB update of this thread's spins, two
+            // cities at a time in packed FP32 (per component the roundings of
+            // the scalar operations), both clamp branches computed and
+            // selected; cities past N stay zero.
             if (active) {
+                const float rs = rsum[m];
+                const float2 qc = make_float2(P.qc4, P.qc4), qb = make_float2(P.qb4, P.qb4);
+                const float2 qa = make_float2(P.qa8, P.qa8), rs2 = make_float2(rs, rs);
+                const float2 m1005 = make_float2(-1.005f, -1.005f), two = make_float2(2.f, 2.f);
+                const float2 bt = make_float2(sc.x, sc.x), cxi = make_float2(P.dtxi0, P.dtxi0);
+                const float2 cdt = make_float2(P.dt, P.dt), cy = make_float2(sc.y, sc.y);
 #pragma unroll
-                for (int k = 0; k < NP; k++) {
-                    if (k < N) {
-                        float dk = 0.f;
+                for (int j = 0; j < CPT; j += 4) {
+                    const float4 c4 = *(const float4 *)&colsum[a * NPS + k0 + j];
 #pragma unroll
-                        for (int l = 0; l < NP; l += 4) {
-                            const float4 d4 = *(const float4 *)&Ds[k * NP + l];
-                            dk += d4.x * nb[l] + d4.y * nb[l + 1] + d4.z * nb[l + 2] + d4.w * nb[l + 3];
+                    for (int e = 0; e < 4; e += 2) {
+                        const int q = j + e;
+                        const float2 cs2 = e ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+                        const float2 jx = __ffma2_rn(qa, make_float2(dk[q], dk[q + 1]),
+                                                     __ffma2_rn(qc, cs2, __fmul2_rn(qb, rs2)));
+                        const float2 i1 = __fmul2_rn(m1005, jx);
+                        const float2 x0 = make_float2(xo[q], xo[q + 1]), y0 = make_float2(yr[q], yr[q + 1]);
+                        float2 y = __ffma2_rn(cxi, __ffma2_rn(bt, make_float2(i2r[q], i2r[q + 1]),
+                                                              __fmul2_rn(two, i1)), y0);
+                        y = make_float2(rnd<T>(y.x), rnd<T>(y.y));
+                        float2 x = __ffma2_rn(cdt, y, x0);
+                        x = make_float2(rnd<T>(x.x), rnd<T>(x.y));
+                        y = __ffma2_rn(cy, x, y);
+                        y = make_float2(rnd<T>(y.x), rnd<T>(y.y));
+                        const bool w0 = fabsf(x0.x) > 1.f, w1 = fabsf(x0.y) > 1.f;
+                        if (whole || k0 + q < N) {
+                            xo[q] = w0 ? spin_of(x0.x) : x.x;
+                            yr[q] = w0 ? 0.f : y.x;
                         }
-                        const float jx = P.qc4 * colsum[k * KA + a] + P.qb4 * rs + P.qa8 * dk;
-                        float x = xo[k], y = yr[k];
-                        if (fabsf(x) > 1.f) {
-                            x = spin_of(x);
-                            y = 0.f;
-                        } else {
-                            const float i1 = -1.005f * jx;
-                            y = rnd<T>(y + P.dtxi0 * (2.f * i1 + sc.x * s_I2[k]));
-                            x = rnd<T>(x + P.dt * y);
-                            y = rnd<T>(y + sc.y * x);
+                        if (whole || k0 + q + 1 < N) {
+                            xo[q + 1] = w1 ? spin_of(x0.y) : x.y;
+                            yr[q + 1] = w1 ? 0.f : y.y;
                         }
-                        xo[k] = x;
-                        yr[k] = y;
                     }
                 }
 #pragma unroll
-                for (int l = 0; l < NP; l += 4)
-                    *(float4 *)&xs[(i * KA + a) * NPS + l] = make_float4(xo[l], xo[l + 1], xo[l + 2], xo[l + 3]);
+                for (int l = 0; l < CPT; l += 4)
+                    *(float4 *)&xrow[l] = make_float4(xo[l], xo[l + 1], xo[l + 2], xo[l + 3]);
             }
             __syncthreads();
         }
         // Window: validity (one +1 per city and per position), stability,
-        // tour snapshot of valid agents (src/kernels.cu:473-531).
-        uint32_t bits = 0;
+        // tour snapshot of valid agents (src/kernels.cu:473-531); each part
+        // adds its cities' sign bits, part 0 of the row decides.
         if (active) {
+            uint32_t part = 0;
 #pragma unroll
-            for (int k = 0; k < NP; k++)
-                if (k < N) bits |= sbit(xo[k]) << k;
-            rowbits[i * KA + a] = bits;
+            for (int j = 0; j < CPT; j++)
+                if (k0 + j < N) part |= sbit(xo[j]) << (k0 + j);
+            if (part) atomicOr(&rowbits[m], part);
         }
         if (tid < 2 * KA) aflag[tid] = tid < KA ? 1 : 0;
         __syncthreads();
-        if (active) {
+        const uint32_t bits = active ? rowbits[m] : 0u;
+        if (active && h == 0) {
             const int order_cnt = __popc(~bits & maskN);
             int city_cnt = 0;
             for (int p = 0; p < N; p++) city_cnt += (~rowbits[p * KA + a] >> i) & 1u;
             if (order_cnt != 1 || city_cnt != 1) atomicAnd(&aflag[a], 0);
-            if (bits != (prevbits[i * KA + a] & maskN)) atomicOr(&aflag[KA + a], 1);
+            if (bits != (prevbits[m] & maskN)) atomicOr(&aflag[KA + a], 1);
         }
         __syncthreads();
-        if (active) {
+        if (active && h == 0) {
             const bool valid = aflag[a] != 0;
             if (valid && real) {
                 P.tours[(int64_t)ag * N + i] = __ffs(~bits & maskN) - 1;
@@ -192,7 +259,8 @@ __global__ void __launch_bounds__(512) k_tsp_resident(const TspP P, const int KA
                 bif = (stab == P.threshold - 1);
                 prv = bif;
             }
-            prevbits[i * KA + a] = bits;
+            prevbits[m] = bits;
+            rowbits[m] = 0;
         }
         __syncthreads();
     }
@@ -200,21 +268,21 @@ __global__ void __launch_bounds__(512) k_tsp_resident(const TspP P, const int KA
     // State back to global memory (get_state) and the window spins.
     if (active && real) {
 #pragma unroll
-        for (int k = 0; k < NP; k++)
-            if (k < N) {
-                const int64_t gi = (int64_t)(i * N + k) * P.Ap + ag;
-                xg[gi] = St<T>::st(xo[k]);
-                yg[gi] = St<T>::st(yr[k]);
+        for (int j = 0; j < CPT; j++)
+            if (k0 + j < N) {
+                const int64_t gi = (int64_t)(i * N + k0 + j) * P.Ap + ag;
+                xg[gi] = St<T>::st(xo[j]);
+                yg[gi] = St<T>::st(yr[j]);
             }
-        const uint32_t bits = prevbits[i * KA + a];
-        for (int k = 0; k < N; k++) {
+        const uint32_t bits = prevbits[m];
+        for (int k = k0; k < k0 + CPT && k < N; k++) {
             const int64_t r = i * N + k;
             const uint32_t bit = (bits >> k) & 1u;
             uint32_t *p = &P.Wp[r * P.W + (ag >> 5)];
             if (bit) atomicOr(p, 1u << (ag & 31));
             else atomicAnd(p, ~(1u << (ag & 31)));
         }
-        if (i == 0) {
+        if (i == 0 && h == 0) {
             P.stab[ag] = stab;
             P.bif[ag] = bif;
             P.prev[ag] = prv;
@@ -226,20 +294,22 @@ __global__ void __launch_bounds__(512) k_tsp_resident(const TspP P, const int KA
     }
 }
 
-template <class T, int NP>
-cudaError_t launch_res(const TspP &P, int ka, cudaStream_t s, bool pdl)
+// Threads of a part: the rows, whole warps.
+int part_threads(int N, int ka) { return (N * ka + 31) / 32 * 32; }
+
+template <class T, int NP, int H>
+cudaError_t launch_res(const TspP &P, const DevTsp &t, int ka, cudaStream_t s, bool pdl)
 {
     constexpr int NPS = NP + 4;
     const int N = P.N;
-    const size_t smem = sizeof(float) * ((size_t)N * ka * NPS + NP * NP + NP * ka) +
+    const size_t smem = sizeof(float) * ((size_t)N * ka * NPS + (size_t)ka * NPS + N * ka) +
                         sizeof(uint32_t) * 2 * N * ka + sizeof(int) * 2 * ka;
-    cudaError_t e = cudaFuncSetAttribute(k_tsp_resident<T, NP>,
+    cudaError_t e = cudaFuncSetAttribute(k_tsp_resident<T, NP, H>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int threads = (N * ka + 31) / 32 * 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((P.A + ka - 1) / ka);
-    cfg.blockDim = dim3(threads);
+    cfg.blockDim = dim3(part_threads(N, ka) * H);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -247,14 +317,26 @@ cudaError_t launch_res(const TspP &P, int ka, cudaStream_t s, bool pdl)
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_tsp_resident<T, NP>, P, ka);
+    TspD<NP> D = {};
+    size_t pair = 0;   // packed: pairs c1 < c2 in order
+    for (int c1 = 0; c1 < N; c1++)
+        for (int c2 = c1 + 1; c2 < N; c2++, pair++) D.d[c1 * NP + c2] = D.d[c2 * NP + c1] = (float)t.packed[pair];
+    return cudaLaunchKernelEx(&cfg, k_tsp_resident<T, NP, H>, P, D, ka);
 }
 
+// Eight cities a thread (four parts of 32, two of 16) where the CTA's threads
+// allow it; more agents a CTA (only when asked for) take fewer parts.
 template <class T>
-cudaError_t launch_np(const TspP &P, int ka, cudaStream_t s, bool pdl)
+cudaError_t launch_np(const TspP &P, const DevTsp &t, int ka, cudaStream_t s, bool pdl)
 {
-    if (P.N <= 16) return launch_res<T, 16>(P, ka, s, pdl);
-    return launch_res<T, 32>(P, ka, s, pdl);
+    const int R = part_threads(P.N, ka);
+    if (P.N <= 16) {
+        if (2 * R <= 1024) return launch_res<T, 16, 2>(P, t, ka, s, pdl);
+        return launch_res<T, 16, 1>(P, t, ka, s, pdl);
+    }
+    if (4 * R <= 1024) return launch_res<T, 32, 4>(P, t, ka, s, pdl);
+    if (2 * R <= 1024) return launch_res<T, 32, 2>(P, t, ka, s, pdl);
+    return launch_res<T, 32, 1>(P, t, ka, s, pdl);
 }
 
 }  // namespace
@@ -262,15 +344,14 @@ cudaError_t launch_np(const TspP &P, int ka, cudaStream_t s, bool pdl)
 int tsp_pick_ka(const SolveDims &d, const DevTsp &t, int requested)
 {
     if (d.prec == P_F64 || t.N > 32 || t.N < 2) return 0;
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int nsm = dev_attr(cudaDevAttrMultiProcessorCount);
     const int kmax = 512 / t.N;   // registers: <= 512 threads of ~128 registers
     if (kmax < 1) return 0;
     if (requested > 0) return requested <= kmax ? requested : 0;
+    // one CTA an SM, as long as its rows can be split in eight-city parts
     int ka = (d.A + nsm - 1) / nsm;
     if (ka < 1) ka = 1;
-    if (ka > kmax) ka = kmax;
+    while (ka > 1 && (t.N <= 16 ? 2 : 4) * part_threads(t.N, ka) > 1024) ka--;
     return ka;
 }
 
@@ -278,7 +359,6 @@ cudaError_t launch_tsp_resident(const SolveDims &d, const DevTsp &t, Work &w, in
                                 cudaStream_t s)
 {
     TspP P;
-    P.D = t.D;
     P.I2 = t.I2;
     P.sched = w.sched;
     P.x = w.x;
@@ -306,9 +386,9 @@ cudaError_t launch_tsp_resident(const SolveDims &d, const DevTsp &t, Work &w, in
     P.k1u = (float)(d.dt * (p0 + 1));
     P.k2u = (float)(d.dt * (p0 - 1));
     switch (d.prec) {
-    case P_F32: return launch_np<float>(P, ka, s, d.pdl);
-    case P_BF16: return launch_np<__nv_bfloat16>(P, ka, s, d.pdl);
-    case P_F16: return launch_np<__half>(P, ka, s, d.pdl);
+    case P_F32: return launch_np<float>(P, t, ka, s, d.pdl);
+    case P_BF16: return launch_np<__nv_bfloat16>(P, t, ka, s, d.pdl);
+    case P_F16: return launch_np<__half>(P, t, ka, s, d.pdl);
     default: return cudaErrorInvalidValue;
     }
 }
