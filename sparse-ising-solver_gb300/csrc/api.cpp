@@ -54,6 +54,7 @@ struct BatchClass {
     DevRb rb;                             // packed for the resident batch kernel (on first use)
     int64_t rb_max = 0;                   // bin capacity the packing was made for
     DevBsm bsm;                           // plan of the shared-memory-plane step (on first use)
+    DevBres bres;                         // packed for the on-chip batch kernel (on first use)
     std::vector<int32_t> agent_off;       // instance i's cuts at [agent_off[i], agent_off[i + 1])
     int32_t *daoff = nullptr;             // the same on the device
     // Each instance's rows are renumbered by decreasing degree inside its
@@ -68,6 +69,8 @@ struct sbx_ctx {
     Work w;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evp[4] = {};
     int32_t *pinned = nullptr;   // stop-flag ring for the update-window poll
+    cudaStream_t side[3] = {};   // the on-chip batch kernel's cluster sizes, made on first use
+    cudaEvent_t fork = nullptr, join[3] = {};
     // graph cache for the streaming chunk
     cudaGraphExec_t gexec = nullptr;
     std::string gkey;
@@ -1270,6 +1273,161 @@ void free_bsm(DevBsm &M)
     M = DevBsm();
 }
 
+void free_bres(DevBres &B)
+{
+    void *ptrs[] = {B.bins, B.slot0, B.slice0, B.rows, B.off, B.col, B.cb, B.perm};
+    for (void *q : ptrs) cudaFree(q);
+    B = DevBres();
+}
+
+// Pack a class for the on-chip batch kernel; leaves bres.rows null when an
+// instance does not fit.  A bin's cluster is the smallest that holds it and,
+// when the class alone cannot fill the GPU, splits it down to an SM's share.
+int build_bres(sbx_ctx *ctx, BatchClass &c)
+{
+    DevBres &B = c.bres;
+    free_bres(B);
+    B.tried = true;
+    const DevCsr &J = c.J;
+    const size_t ni = c.probs.size();
+    int64_t cap[3];
+    for (int k = 0; k < 3; k++) cap[k] = batch_res_rows(1 << k);
+    const int nsm = std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
+    const int64_t share = std::max<int64_t>(512, J.n * (c.Ap / 16) / nsm);   // rows a CTA would hold in one even wave
+    std::vector<size_t> ord(ni);
+    std::iota(ord.begin(), ord.end(), 0);
+    std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return c.probs[a]->J.n > c.probs[b]->J.n; });
+    struct Bin {
+        std::vector<int32_t> inst;
+        int64_t rows = 0;
+        int k = 0;   // cluster of 2^k CTAs
+    };
+    std::vector<Bin> bins;
+    const int64_t room = std::min(cap[0], std::max<int64_t>(1024, share / 2));   // small instances share bins up to this
+    size_t open = (size_t)-1;   // first one-CTA bin with room (instances come in decreasing size)
+    for (size_t i : ord) {
+        const int64_t n = c.probs[i]->J.n;
+        int k = 0;
+        while (k < 3 && (n > cap[k] || (k < 2 && n / (1 << k) > share))) k++;
+        if (k == 3) return SBX_OK;   // too large for a cluster
+        size_t at = bins.size();
+        if (k == 0) {
+            if (open == (size_t)-1) open = at;
+            while (open < bins.size() && bins[open].rows >= room - 32) open++;
+            for (size_t b = open; b < bins.size() && b < open + 64; b++)
+                if (bins[b].rows + n <= room) {
+                    at = b;
+                    break;
+                }
+        }
+        if (at == bins.size()) {
+            bins.emplace_back();
+            bins.back().k = k;
+        }
+        bins[at].inst.push_back((int32_t)i);
+        bins[at].rows += n;
+    }
+    std::stable_sort(bins.begin(), bins.end(),
+                     [](const Bin &a, const Bin &b) { return a.k != b.k ? a.k < b.k : a.rows > b.rows; });
+    const size_t nb = bins.size();
+    std::vector<int32_t> list(nb), slot0(nb), slice0(nb), rows(nb), perm((size_t)J.n);
+    B.hinst.assign((size_t)J.n, 0);
+    B.hdeg.assign((size_t)J.n, 0);
+    int64_t slots = 0, slices = 0;
+    for (size_t b = 0; b < nb; b++) {
+        list[b] = (int32_t)b;
+        slot0[b] = (int32_t)slots;
+        slice0[b] = (int32_t)slices;
+        rows[b] = (int32_t)bins[b].rows;
+        if (!B.nbins[bins[b].k]) B.bin0[bins[b].k] = (int32_t)b;
+        B.nbins[bins[b].k]++;
+        B.max_rows[bins[b].k] = std::max(B.max_rows[bins[b].k], bins[b].rows);
+        slots += bins[b].rows;
+        slices += (bins[b].rows + 31) / 32 + 1;
+    }
+    std::vector<int32_t> off((size_t)slices, 0);
+    std::vector<int64_t> blocks(nb, 0);
+    const int T = J.nnz > (1 << 18) ? host_threads() : 1;
+    // a bin's slots: its instances' rows by decreasing degree (<= 127), ties
+    // in row order; its slices' block counts
+    parallel(T, [&](int t, int TT) {
+        for (size_t b = (size_t)t; b < nb; b += (size_t)TT) {
+            int64_t at[129] = {0};
+            auto deg = [&](int64_t r) { return J.hrowptr[(size_t)r + 1] - J.hrowptr[(size_t)r]; };
+            for (int32_t i : bins[b].inst)
+                for (int64_t r = c.row_off[(size_t)i], e = r + c.probs[(size_t)i]->J.n; r < e; r++) at[128 - deg(r)]++;
+            for (int k = 1; k <= 128; k++) at[k] += at[k - 1];
+            for (int32_t i : bins[b].inst)
+                for (int64_t r = c.row_off[(size_t)i], e = r + c.probs[(size_t)i]->J.n; r < e; r++) {
+                    const size_t s = (size_t)slot0[b] + (size_t)at[127 - deg(r)]++;
+                    perm[s] = (int32_t)r;
+                    B.hinst[s] = i;
+                    B.hdeg[s] = deg(r);
+                }
+            int32_t *o = &off[(size_t)slice0[b]];
+            for (int64_t k = 0; 32 * k < rows[b]; k++) {
+                o[k] = (int32_t)blocks[b];
+                blocks[b] += (B.hdeg[(size_t)slot0[b] + (size_t)(32 * k)] + 3) / 4;
+            }
+            o[(rows[b] + 31) / 32] = (int32_t)blocks[b];
+        }
+    });
+    int64_t total = 0;
+    std::vector<int64_t> first(nb);
+    for (size_t b = 0; b < nb; b++) {
+        first[b] = total;
+        total += blocks[b];
+    }
+    if (total * 32 > INT32_MAX) return SBX_OK;
+    std::vector<uint16_t> col((size_t)std::max<int64_t>(total, 1) * 128);
+    std::vector<int32_t> inv((size_t)J.n);
+    parallel(T, [&](int t, int TT) {
+        for (size_t b = (size_t)t; b < nb; b += (size_t)TT) {
+            for (int64_t s = 0; s < rows[b]; s++) inv[(size_t)perm[(size_t)(slot0[b] + s)]] = (int32_t)s;
+            std::fill(col.begin() + (long)(first[b] * 128), col.begin() + (long)((first[b] + blocks[b]) * 128),
+                      (uint16_t)(2 * rows[b]));
+            int32_t *o = &off[(size_t)slice0[b]];
+            for (int64_t s = 0; s < rows[b]; s++) {
+                const size_t r = (size_t)perm[(size_t)(slot0[b] + s)];
+                uint16_t *row = &col[((size_t)(first[b] + o[s / 32]) * 32 + (size_t)(s & 31)) * 4];
+                for (int32_t e = J.hrowptr[r], j = 0; e < J.hrowptr[r + 1]; e++, j++)
+                    row[(size_t)(j / 4) * 128 + (size_t)(j & 3)] =
+                        (uint16_t)(2 * inv[(size_t)J.hcol[(size_t)e]] + (J.hval[(size_t)e] < 0 ? 1 : 0));
+            }
+            for (int64_t k = 0; k <= (rows[b] + 31) / 32; k++) o[k] += (int32_t)first[b];
+        }
+    });
+    auto put = [&](void **p, const void *src, size_t bytes) {
+        cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+        return e == cudaSuccess && bytes ? cudaMemcpy(*p, src, bytes, cudaMemcpyHostToDevice) : e;
+    };
+    CK(put((void **)&B.bins, list.data(), 4 * nb));
+    CK(put((void **)&B.slot0, slot0.data(), 4 * nb));
+    CK(put((void **)&B.slice0, slice0.data(), 4 * nb));
+    CK(put((void **)&B.off, off.data(), 4 * off.size()));
+    CK(put(&B.col, col.data(), 2 * col.size()));
+    CK(put((void **)&B.perm, perm.data(), 4 * perm.size()));
+    CK(cudaMalloc(&B.cb, sizeof(float) * 2 * std::max<int64_t>(J.n, 1)));
+    CK(put((void **)&B.rows, rows.data(), 4 * nb));   // last: the plan is complete
+    return SBX_OK;
+}
+
+// dt * xi0 of each slot's instance, and the bias that turns a byte counter's
+// float into the force.
+int upload_bres_cb(sbx_ctx *ctx, BatchClass &c, double dt)
+{
+    DevBres &B = c.bres;
+    if (B.dt == dt) return SBX_OK;
+    std::vector<float> cb(2 * B.hinst.size());
+    for (size_t s = 0; s < B.hinst.size(); s++) {
+        cb[2 * s] = (float)(dt * c.xi0[(size_t)B.hinst[s]]);
+        cb[2 * s + 1] = -(8388608.0f + (float)B.hdeg[s]);
+    }
+    CK(cudaMemcpy(B.cb, cb.data(), sizeof(float) * cb.size(), cudaMemcpyHostToDevice));
+    B.dt = dt;
+    return SBX_OK;
+}
+
 // Can the class run the shared-memory-plane step kernel: 16-bit state, +-1
 // weights, at most 127 neighbours per row (seven count planes), 32, 64 or 128
 // padded agents, instances of at most 32,767 rows (15-bit local columns), and
@@ -1490,6 +1648,7 @@ void free_batch(sbx_ctx *ctx)
         free_csr(c.J);
         free_rb(c.rb);
         free_bsm(c.bsm);
+        free_bres(c.bres);
         cudaFree(c.daoff);
         cudaFree(c.dslot);
     }
@@ -1619,8 +1778,24 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
                         "32/64/128 agents and instances whose plane fits in shared memory");
         const bool use_bsm = bsm_fit && !tile_pinned && pr->kernel != SBX_KERNEL_RESIDENT &&
                              pr->kernel != SBX_KERNEL_RESIDENT_SPLIT;
+        // the on-chip batch kernel: +-1 fused 16-bit classes whose instances
+        // fit a cluster, unless a tile, a count mode or a kernel is asked for
+        bool use_res = !use_rb && !tile_pinned && !bsm_threads && !pr->count_mode && pr->kernel == SBX_KERNEL_AUTO &&
+                       (d.prec == P_BF16 || d.prec == P_F16) && d.fused && !d.trace && nchunks > 0 && c.J.unit &&
+                       c.J.max_deg <= kHeavy;
+        if (use_res) {
+            if (!c.bres.tried && (rc = build_bres(ctx, c))) return rc;
+            use_res = c.bres.rows != nullptr;
+        }
         c.J.bsm = nullptr;
-        if (use_rb) {
+        if (use_res) {
+            if ((rc = upload_bres_cb(ctx, c, pr->dt))) return rc;
+            for (int k = 0; k < 3; k++) {
+                if (!ctx->side[k]) CK(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
+                if (!ctx->join[k]) CK(cudaEventCreateWithFlags(&ctx->join[k], cudaEventDisableTiming));
+            }
+            if (!ctx->fork) CK(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
+        } else if (use_rb) {
             if (!c.rb.rowptr || c.rb_max != rb_rows) {
                 if ((rc = build_rb(ctx, c, rb_rows))) return rc;
             }
@@ -1639,7 +1814,14 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         int launches = 0;
         double kms = 0;
         CK(cudaEventRecord(ctx->ev0, s));
-        if (use_rb) {
+        if (use_res) {
+            d.steps_run = (int32_t)total;
+            const cudaError_t e = launch_batch_res(d, c.bres, c.J.allpos, *std::max_element(c.agents.begin(), c.agents.end()),
+                                                   ctx->w, s, ctx->side, ctx->fork, ctx->join, &launches);
+            if (e != cudaSuccess)   // what was launched ends before the buffers are used again
+                for (cudaStream_t t : ctx->side) cudaStreamSynchronize(t);
+            CK(e);
+        } else if (use_rb) {
             d.steps_run = (int32_t)total;
             CK(launch_resident_batch(d, c.rb, ctx->w, s));
             launches = 1;
@@ -1688,7 +1870,13 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             memset(r, 0, sizeof *r);
             r->time_to_target_us = -1;
             r->steps_to_target = -1;
-            if (d.tbsm) {
+            if (use_res) {
+                r->lane_agents = 16;
+                r->row_lanes = 1;
+                r->block_threads = 1024;
+                r->count_mode = 4;
+                r->staging = 3;
+            } else if (d.tbsm) {
                 r->lane_agents = 32;
                 r->row_lanes = d.W;
                 r->block_threads = d.tbsm;
@@ -1714,9 +1902,9 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             r->steps_run = total;
             r->windows_run = nchunks;
             r->kernel_used = use_rb ? SBX_KERNEL_RESIDENT : SBX_KERNEL_STREAM;
-            r->agents_per_block = use_rb ? 4 : 0;
+            r->agents_per_block = use_rb ? 4 : use_res ? 16 : 0;
             r->kernel_launches = launches;
-            r->kernel_ms = use_rb ? (profile ? ms : 0.0) : kms;
+            r->kernel_ms = use_rb || use_res ? (profile ? ms : 0.0) : kms;
             r->gpu_launches = launches + 4;
             if (agent_values)
                 memcpy(agent_values + val_off[gi], &cutv[(size_t)c.agent_off[i]], sizeof(double) * c.agents[i]);
@@ -1911,6 +2099,11 @@ int sbx_destroy(sbx_ctx *ctx)
     if (!ctx) return SBX_ERR_ARG;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    for (int k = 0; k < 3; k++) {
+        if (ctx->side[k]) cudaStreamDestroy(ctx->side[k]);
+        if (ctx->join[k]) cudaEventDestroy(ctx->join[k]);
+    }
+    if (ctx->fork) cudaEventDestroy(ctx->fork);
     Work &w = ctx->w;
     void *ptrs[] = {w.x, w.y, w.x2, w.S[0], w.S[1], w.Wp, w.fin, w.chg, w.newmask, w.stab, w.bif,
                     w.prev, w.ctl, w.wincount, w.visits, w.ab, w.sched, w.eacc, w.cut, w.trace,

@@ -187,6 +187,21 @@ struct DevBsm {
     int64_t max_rows = 0;         // largest instance: the shared-memory plane's rows
 };
 
+// A batch class packed for the on-chip batch kernel (k_batch_res.cu): whole
+// instances in bins, a bin's rows by decreasing degree ("slots") in slices of
+// 32 (as DevSell); the bins listed by cluster size 1, 2, 4, largest first.
+struct DevBres {
+    bool tried = false;          // planned (rows is null when the class does not fit)
+    int32_t *bins = nullptr, *slot0 = nullptr, *slice0 = nullptr, *rows = nullptr, *off = nullptr;
+    void *col = nullptr;         // [blocks][32] of four entries 2 slot + sign
+    void *cb = nullptr;          // per slot: dt * xi0, -(2^23 + degree)
+    int32_t *perm = nullptr;     // slot -> class row
+    int32_t bin0[3] = {0, 0, 0}, nbins[3] = {0, 0, 0};
+    int64_t max_rows[3] = {0, 0, 0};
+    std::vector<int32_t> hinst, hdeg;   // per slot: instance, degree
+    double dt = -1;              // dt of the uploaded cb
+};
+
 // A batch class packed for the resident batch kernel (k_resident_batch.cu):
 // whole instances in bins, rows of a bin by decreasing degree ("slots"), the
 // matrix relabelled into slot order.
@@ -266,6 +281,14 @@ cudaError_t launch_resident(const SolveDims &d, const DevCsr &J, Work &w, int ka
 // rows; one launch runs d.steps_run fused steps of every instance.
 int64_t resident_batch_max_rows();
 cudaError_t launch_resident_batch(const SolveDims &d, const DevRb &B, Work &w, cudaStream_t s);
+
+// On-chip batch kernel (k_batch_res.cu): most rows of a bin on a cluster of C
+// CTAs; all d.steps_run fused steps of every bin, the cluster sizes on the
+// side streams between fork and join.  agents: the class's largest count.
+int64_t batch_res_rows(int C);
+cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, int32_t agents, Work &w,
+                             cudaStream_t s, cudaStream_t *side, cudaEvent_t fork, cudaEvent_t *join,
+                             int *launches);
 
 // Tensor-memory + shared-memory resident kernel (k_resident_rs.cu), fused
 // steps: its agents per CTA (8 of 16-bit state, 4 of FP32) when it is to run.

@@ -1,0 +1,466 @@
+// k_batch_res.cu -- batched MaxCut with the state on chip for the whole solve:
+// the instances are packed into bins (whole instances; a large one is a bin of
+// its own), and a cluster of C = 1, 2 or 4 CTAs owns 16 agents of every row of
+// one bin from the first step to the last.  Instances never interact and
+// neither do agents, so a cluster needs no other.  +-1 weights, degree <= 127,
+// 16-bit state, fused steps; the arithmetic is the streaming kernel's (exact
+// force, sb_update's roundings), so the results are identical.
+//
+// A step launched per kernel (k_bsm) reads and writes the whole state each
+// time and waits for it: at 20 warps an SM it took 234 us a step on 512
+// instances (1.9 M rows x 64 agents) with the issue slots 38% busy, and no
+// less per row when the state fitted in L2.  Here the loop touches only the
+// columns (L2) and shared and tensor memory.
+//
+// Rows.  A bin's rows are in decreasing degree ("slots"), in slices of 32;
+// CTA r of the cluster takes slices r, r + C, ...  A thread's rows are one of
+// each 1,024; x and y of 16 agents are 64 bytes: the first 4 rows of a thread
+// in tensor memory (16 columns each of its own lane), the rest in shared
+// memory.  Every CTA holds the signs of all the bin's rows, a 16-bit word a
+// row, double-buffered; a new word is stored to all CTAs of the cluster
+// (distributed shared memory), and one cluster barrier a step orders the
+// stores against the next step's gathers (Jacobi, src/kernels.cu:211-269).
+//
+// Force.  Columns are blocks of four 16-bit entries (2 slot + sign) per row,
+// one coalesced 8-byte load a lane.  Two neighbours' 16-bit words make one
+// 32-bit word (XORed with their weights' signs); the words add up in bit
+// planes with full adders, the halves are summed, and the planes transposed
+// into byte counters.  Sixteen agents a row because a gather and its adders
+// then serve twice the agents of eight; thirty-two would not leave a
+// 20,000-row instance on eight SMs.  Bound: issue and the ALU pipe.
+#include "k_step.cuh"
+
+#include <algorithm>
+
+namespace sbx {
+
+namespace {
+
+constexpr int kNT = 1024;
+constexpr int kTmRows = 4;   // rows of a thread in tensor memory: 512 columns / 8 warps a lane quarter / 16 words
+
+struct BresP {
+    const int32_t *__restrict__ bins;    // bins of this launch, largest first
+    const int32_t *__restrict__ slot0;   // per bin: first slot (of perm and cb), slots + 1 entries in all
+    const int32_t *__restrict__ slice0;  // per bin: first slice (of off)
+    const int32_t *__restrict__ rows;    // per bin: rows
+    const int32_t *__restrict__ off;     // per slice: first block, and the end after a bin's last slice
+    const uint2 *__restrict__ col;       // [blocks][32]
+    const float2 *__restrict__ cb;       // per slot: dt * xi0 of its instance, -(2^23 + degree)
+    const int32_t *__restrict__ perm;    // slot -> state row
+    const float4 *__restrict__ coef;
+    void *x, *y;                         // global [rows][Ap]
+    uint32_t *Wp;                        // global plane [rows][W]: signs of the last step
+    int32_t *ctl;
+    int32_t Ap, W, groups, nsteps, allpos;
+};
+
+struct Row16 {
+    uint32_t x[8], y[8];   // packed pairs of 16 agents
+};
+
+__device__ __forceinline__ uint32_t lds16(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("{\n\t.reg .u16 h;\n\tld.shared.u16 h, [%1];\n\tcvt.u32.u16 %0, h;\n\t}" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void tm_ld16(uint32_t ta, Row16 &v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]),
+                   "=r"(v.x[6]), "=r"(v.x[7]), "=r"(v.y[0]), "=r"(v.y[1]), "=r"(v.y[2]), "=r"(v.y[3]),
+                   "=r"(v.y[4]), "=r"(v.y[5]), "=r"(v.y[6]), "=r"(v.y[7])
+                 : "r"(ta)
+                 : "memory");
+}
+__device__ __forceinline__ void tm_st16(uint32_t ta, const Row16 &v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                 "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta),
+                 "r"(v.x[0]), "r"(v.x[1]), "r"(v.x[2]), "r"(v.x[3]), "r"(v.x[4]), "r"(v.x[5]), "r"(v.x[6]),
+                 "r"(v.x[7]), "r"(v.y[0]), "r"(v.y[1]), "r"(v.y[2]), "r"(v.y[3]), "r"(v.y[4]), "r"(v.y[5]),
+                 "r"(v.y[6]), "r"(v.y[7])
+                 : "memory");
+}
+// Address of the same shared location in CTA `rank` of the cluster, and a
+// 16-bit store there.
+__device__ __forceinline__ uint32_t peer(uint32_t a, uint32_t rank)
+{
+    uint32_t d;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(rank));
+    return d;
+}
+__device__ __forceinline__ void st_peer16(uint32_t a, uint32_t v)
+{
+    asm volatile("{\n\t.reg .u16 h;\n\tcvt.u16.u32 h, %1;\n\tst.shared::cluster.u16 [%0], h;\n\t}" ::"r"(a), "r"(v)
+                 : "memory");
+}
+// All threads of the cluster's CTAs; orders their shared stores.
+template <int C> __device__ __forceinline__ void step_barrier()
+{
+    if (C == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+// A block's four neighbour words as two 32-bit words of two, the weights'
+// signs (bit 0 of an entry) applied.
+template <bool NEG> __device__ __forceinline__ void block_words(const uint2 &c, uint32_t S, uint32_t &w0, uint32_t &w1)
+{
+    const uint32_t u0 = NEG ? c.x & 0xfffefffeu : c.x, u1 = NEG ? c.y & 0xfffefffeu : c.y;
+    w0 = __byte_perm(lds16(S + (u0 & 0xffffu)), lds16(S + (u0 >> 16)), 0x5410);
+    w1 = __byte_perm(lds16(S + (u1 & 0xffffu)), lds16(S + (u1 >> 16)), 0x5410);
+    if (NEG) {   // 0 or 0xffff per half
+        w0 ^= (c.x & 0x00010001u) * 0xffffu;
+        w1 ^= (c.y & 0x00010001u) * 0xffffu;
+    }
+}
+
+// Byte counters of 2 * count over nb blocks: agents 8 h .. 8 h + 3 in
+// cnt[2 h], 8 h + 4 .. 8 h + 7 in cnt[2 h + 1].  PL planes hold the 2 nb
+// entries of a half word (2 nb < 2^PL).
+template <int PL, bool NEG>
+__device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32_t S, uint32_t (&cnt)[4])
+{
+    uint32_t p[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int32_t b = 0; b < nb; b += 2) {
+        const uint2 c0 = __ldg(cp + b * 32);
+        const bool two = b + 1 < nb;   // warp-uniform
+        uint2 c1;
+        if (two) c1 = __ldg(cp + (b + 1) * 32);
+        uint32_t w0, w1, w2 = 0u, w3 = 0u;
+        block_words<NEG>(c0, S, w0, w1);
+        if (two) block_words<NEG>(c1, S, w2, w3);
+        const uint32_t a = fadd(p[0], w0, w1), d = fadd(p[0], w2, w3);
+        uint32_t c = fadd(p[1], a, d);
+#pragma unroll
+        for (int k = 2; k < PL; k++) {
+            const uint32_t t = p[k] & c;
+            p[k] ^= c;
+            c = t;
+        }
+    }
+    // the halves together
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < PL; k++) {
+        const uint32_t b = p[k] >> 16;
+        if (k == 0) {
+            c = p[0] & b;
+            p[0] ^= b;
+        } else {
+            c = fadd(p[k], b, c);
+        }
+    }
+    if (PL < 7) p[PL] = c;   // counts are at most 127: seven planes
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        // byte h of each plane, shifted up a byte (which doubles the counts),
+        // then an 8x8 bit transpose
+        const uint32_t s01 = (uint32_t)h | (((uint32_t)h + 4) << 4);
+        uint32_t lo = __byte_perm(__byte_perm(0u, p[0], s01), __byte_perm(p[1], p[2], s01), 0x5410);
+        uint32_t hi = __byte_perm(__byte_perm(p[3], p[4], s01), __byte_perm(p[5], p[6], s01), 0x5410);
+        uint32_t t;
+        t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
+        lo ^= t ^ (t << 7);
+        t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
+        hi ^= t ^ (t << 7);
+        t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
+        lo ^= t ^ (t << 14);
+        t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
+        hi ^= t ^ (t << 14);
+        t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
+        cnt[2 * h] = lo ^ t;
+        cnt[2 * h + 1] = hi ^ (t >> 4);
+    }
+}
+
+template <class T, int C, bool NEG>
+__global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
+{
+    static_assert(sizeof(T) == 2, "16-bit state: 16 agents in 32 bytes");
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = C == 1 ? 0 : (int)(blockIdx.x % C);
+    const int unit = blockIdx.x / C;
+    const int bin = __ldg(&P.bins[unit / P.groups]);
+    const int a0 = (unit % P.groups) * 16;
+    const int R = __ldg(&P.rows[bin]), sl0 = __ldg(&P.slice0[bin]), s0 = __ldg(&P.slot0[bin]);
+    const int nsl = (R + 31) / 32, mine = (nsl - rank + C - 1) / C;   // the bin's slices, this CTA's
+    const int ns = max(0, 32 * mine - kTmRows * kNT);                 // rows kept in shared memory
+    const uint32_t pb = ((uint32_t)(R + 1) * 2 + 15) & ~15u;          // bytes of a sign plane
+    const uint32_t sb = smem_u32(smem);
+    uint4 *st = (uint4 *)(smem + 2 * pb);                             // [4 pieces][ns]
+    T *xg = (T *)P.x, *yg = (T *)P.y;
+
+    // All of the SM's tensor memory: 1,024 threads of 64 registers leave room
+    // for no second CTA that would wait for it.
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(512u));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {   // the zero row that padded entries read
+        ((uint16_t *)smem)[R] = 0;
+        ((uint16_t *)(smem + pb))[R] = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    step_barrier<C>();   // the cluster's CTAs are running: their shared memory may be written
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    const uint32_t tw = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(16 * kTmRows * (warp >> 2));
+
+    auto get_row = [&](int i, Row16 &v) {
+        if (i < kTmRows) {
+            tm_ld16(tw + 16u * (uint32_t)i, v);
+        } else {
+            const int r = (i - kTmRows) * kNT + tid;
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                const uint4 u = st[p * ns + r];
+                memcpy((unsigned char *)&v + 16 * p, &u, 16);
+            }
+        }
+    };
+    auto put_row = [&](int i, const Row16 &v) {
+        if (i < kTmRows) {
+            tm_st16(tw + 16u * (uint32_t)i, v);
+        } else {
+            const int r = (i - kTmRows) * kNT + tid;
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                uint4 u;
+                memcpy(&u, (const unsigned char *)&v + 16 * p, 16);
+                st[p * ns + r] = u;
+            }
+        }
+    };
+    uint32_t pk[C];   // the planes' base in every CTA of the cluster
+#pragma unroll
+    for (int c = 0; c < C; c++) pk[c] = C == 1 ? sb : peer(sb, (uint32_t)c);
+    auto put_sign = [&](uint32_t o, uint32_t w) {
+        if (C == 1) {
+            asm volatile("{\n\t.reg .u16 h;\n\tcvt.u16.u32 h, %1;\n\tst.shared.u16 [%0], h;\n\t}" ::"r"(sb + o), "r"(w)
+                         : "memory");
+        } else {
+#pragma unroll
+            for (int c = 0; c < C; c++) st_peer16(pk[c] + o, w);
+        }
+    };
+    // signs of a row's 16 agents, agent j in bit j
+    auto sign_word = [&](const Row16 &v) {
+        const uint32_t h0[4] = {v.x[0], v.x[1], v.x[2], v.x[3]}, h1[4] = {v.x[4], v.x[5], v.x[6], v.x[7]};
+        uint32_t m0, m1, m2, m3;
+        sign_masks(h0, m0, m1);
+        sign_masks(h1, m2, m3);
+        return sign_byte(m0, m1) | (sign_byte(m2, m3) << 8);
+    };
+
+    // The state after the pre-step Update_XY of step 0 (src/ising.cu:188),
+    // computed and rounded as the streaming pre-step does.
+    const float4 c00 = P.coef[0];
+    for (int i = 0; 32 * i + warp < mine; i++) {
+        const int s = 32 * ((32 * i + warp) * C + rank) + lane;   // slot of the bin
+        Row16 v = {};
+        if (s < R) {
+            const int64_t g = (int64_t)__ldg(&P.perm[s0 + s]) * P.Ap + a0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                Raw<16> xr, yr;
+                float x[8], y[8];
+                xr.u = *(const uint4 *)(xg + g + 8 * h);
+                yr.u = *(const uint4 *)(yg + g + 8 * h);
+                to_vals<T, 8>(xr, x);
+                to_vals<T, 8>(yr, y);
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    y[q] = fmaf(c00.w, x[q], y[q]);
+                    x[q] = fmaf(c00.z, y[q], x[q]);
+                }
+                xr = from_vals<T, 8>(x);
+                yr = from_vals<T, 8>(y);
+                memcpy(&v.x[4 * h], &xr.u, 16);
+                memcpy(&v.y[4 * h], &yr.u, 16);
+            }
+            put_sign(2u * (uint32_t)s, sign_word(v));   // step 0 reads plane 0
+        }
+        put_row(i, v);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    step_barrier<C>();
+
+    for (int32_t k = 0; k < P.nsteps; k++) {
+        const float4 ck = __ldg(&P.coef[k]);
+        const uint32_t Sin = sb + ((k & 1) ? pb : 0u), onx = (k & 1) ? 0u : pb;
+        for (int i = 0; 32 * i + warp < mine; i++) {
+            const int sl = (32 * i + warp) * C + rank, s = 32 * sl + lane;
+            const bool live = s < R;
+            const int32_t b0 = __ldg(&P.off[sl0 + sl]), nb = __ldg(&P.off[sl0 + sl + 1]) - b0;   // warp-uniform
+            const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
+            const float2 cb = __ldg(&P.cb[s0 + min(s, R - 1)]);
+            uint32_t cnt[4];
+            if (nb < 8) count_blocks<4, NEG>(cp, nb, Sin, cnt);
+            else count_blocks<7, NEG>(cp, nb, Sin, cnt);   // degree <= 127: at most 32 blocks
+            Row16 v;
+            get_row(i, v);
+            const float2 bias = make_float2(cb.y, cb.y);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float tv[8];
+#pragma unroll
+                for (int q = 0; q < 8; q += 2) {
+                    const uint32_t w = cnt[2 * h + (q >> 2)];
+                    const float2 t =
+                        __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + (q & 3))),
+                                               __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7441u + (q & 3)))),
+                                   bias);
+                    tv[q] = t.x;
+                    tv[q + 1] = t.y;
+                }
+                uint32_t x[4], y[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    x[q] = v.x[4 * h + q];
+                    y[q] = v.y[4 * h + q];
+                }
+                sb_update16<T, K_FUSED, false, 8>(x, y, tv, cb.x, ck, ck);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    v.x[4 * h + q] = x[q];
+                    v.y[4 * h + q] = y[q];
+                }
+            }
+            put_row(i, v);
+            if (live) put_sign(onx + 2u * (uint32_t)s, sign_word(v));
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        step_barrier<C>();
+    }
+
+    // the state and the signs of the last step back to global memory
+    for (int i = 0; 32 * i + warp < mine; i++) {
+        const int s = 32 * ((32 * i + warp) * C + rank) + lane;
+        Row16 v;
+        get_row(i, v);
+        if (s < R) {
+            const int64_t r = __ldg(&P.perm[s0 + s]), g = r * P.Ap + a0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                *(uint4 *)(xg + g + 8 * h) = make_uint4(v.x[4 * h], v.x[4 * h + 1], v.x[4 * h + 2], v.x[4 * h + 3]);
+                *(uint4 *)(yg + g + 8 * h) = make_uint4(v.y[4 * h], v.y[4 * h + 1], v.y[4 * h + 2], v.y[4 * h + 3]);
+            }
+            ((uint16_t *)P.Wp)[r * P.W * 2 + a0 / 16] = (uint16_t)sign_word(v);
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        P.ctl[CTL_STEP] = P.nsteps;
+        P.ctl[CTL_WINDOWS] = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+}
+
+// Dynamic shared memory of a bin of R rows on C CTAs.
+int64_t smem_bytes(int64_t R, int C)
+{
+    const int64_t nsl = (R + 31) / 32, mine = (nsl + C - 1) / C;
+    return 2 * (((R + 1) * 2 + 15) / 16 * 16) + std::max<int64_t>(0, 32 * mine - kTmRows * kNT) * 64;
+}
+
+template <class T, int C>
+cudaError_t launch_c(const BresP &P, int units, size_t smem, cudaStream_t s)
+{
+    auto kern = P.allpos ? k_batch_res<T, C, false> : k_batch_res<T, C, true>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(units * C));
+    cfg.blockDim = dim3(kNT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, P);
+}
+
+template <class T>
+cudaError_t launch_t(const BresP &P, int C, int units, size_t smem, cudaStream_t s)
+{
+    switch (C) {
+    case 1: return launch_c<T, 1>(P, units, smem, s);
+    case 2: return launch_c<T, 2>(P, units, smem, s);
+    case 4: return launch_c<T, 4>(P, units, smem, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace
+
+int64_t batch_res_rows(int C)
+{
+    const int64_t budget = (int64_t)dev_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024;
+    int64_t lo = 0, hi = 32767;   // most rows whose shared memory fits (15-bit slots)
+    while (lo < hi) {
+        const int64_t mid = (lo + hi + 1) / 2;
+        if (smem_bytes(mid, C) <= budget) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, int32_t agents, Work &w,
+                             cudaStream_t s, cudaStream_t *side, cudaEvent_t fork, cudaEvent_t *join, int *launches)
+{
+    BresP P;
+    P.slot0 = B.slot0;
+    P.slice0 = B.slice0;
+    P.rows = B.rows;
+    P.off = B.off;
+    P.col = (const uint2 *)B.col;
+    P.cb = (const float2 *)B.cb;
+    P.perm = B.perm;
+    P.coef = (const float4 *)w.coef32;
+    P.x = w.x;
+    P.y = w.y;
+    P.Wp = w.Wp;
+    P.ctl = w.ctl;
+    P.Ap = d.Ap;
+    P.W = d.W;
+    P.groups = (agents + 15) / 16;   // groups of padded agents alone stay as they began
+    P.nsteps = d.steps_run;
+    P.allpos = allpos ? 1 : 0;
+    // the cluster sizes on streams of their own, largest first: the smaller
+    // ones' CTAs fill the SMs that whole clusters leave
+    cudaError_t e = cudaEventRecord(fork, s);
+    int nside = 0;
+    for (int c = 2; c >= 0 && e == cudaSuccess; c--) {
+        if (!B.nbins[c]) continue;
+        P.bins = B.bins + B.bin0[c];
+        cudaStream_t t = side[nside];
+        e = cudaStreamWaitEvent(t, fork, 0);
+        if (e != cudaSuccess) break;
+        const int C = 1 << c, units = B.nbins[c] * P.groups;
+        const size_t smem = (size_t)smem_bytes(B.max_rows[c], C);
+        e = d.prec == P_BF16 ? launch_t<__nv_bfloat16>(P, C, units, smem, t) : launch_t<__half>(P, C, units, smem, t);
+        if (e == cudaSuccess) e = cudaEventRecord(join[nside], t);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join[nside], 0);
+        nside++;
+        (*launches)++;
+    }
+    return e;
+}
+
+}  // namespace sbx
