@@ -69,8 +69,8 @@ struct sbx_ctx {
     Work w;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evp[4] = {};
     int32_t *pinned = nullptr;   // stop-flag ring for the update-window poll
-    cudaStream_t side[3] = {};   // the on-chip batch kernel's cluster sizes, made on first use
-    cudaEvent_t fork = nullptr, join[3] = {};
+    cudaStream_t side[4] = {};   // the on-chip batch kernel's kinds of bins, made on first use
+    cudaEvent_t fork = nullptr, join[4] = {};
     // graph cache for the streaming chunk
     cudaGraphExec_t gexec = nullptr;
     std::string gkey;
@@ -1130,6 +1130,46 @@ int build_class(sbx_ctx *ctx, BatchClass &c)
     return SBX_OK;
 }
 
+// Entries of a slice's rows (row l's left[l] entries at ent + l pos) to their
+// positions in the sliced form: position j of row l at out[(j / 4) 128 + 4 l +
+// j % 4], positions not written keep the padding there.  The kernels gather the
+// 32 entries that the rows hold at one position with one shared load, and
+// random rows meet in a bank 2.7 deep (the gather's wavefronts bounded er800).
+// Neighbour counts of +-1 weights do not depend on the order, so each position
+// takes, row by row, an entry whose bank is still free there, or padding
+// while the row has positions to spare.  mask: the entry's bits of the byte
+// offset of its word.
+void place_entries(uint16_t *ent, int64_t pos, int rows, int32_t *left, uint32_t mask, uint16_t *out)
+{
+    for (int64_t j = 0; j < pos; j++) {
+        int32_t word[32];   // the shared word each bank serves at this position
+        std::fill(word, word + 32, -1);
+        for (int t = 0; t < rows; t++) {
+            const int l = (int)((t + j) % rows);
+            uint16_t *v = ent + l * pos;
+            const int32_t m = left[l];
+            if (!m) continue;
+            int32_t pick = m;
+            for (int32_t c = m - 1; c >= 0 && m - c <= 24; c--) {
+                const int32_t w = (int32_t)((v[c] & mask) >> 2);
+                if (word[w & 31] == -1 || word[w & 31] == w) {
+                    pick = c;
+                    break;
+                }
+            }
+            if (pick == m) {
+                if (m < pos - j) continue;   // padding here, the entry later
+                pick = m - 1;
+            }
+            const int32_t w = (int32_t)((v[pick] & mask) >> 2);
+            word[w & 31] = w;
+            out[(j / 4) * 128 + 4 * l + (j & 3)] = v[pick];
+            v[pick] = v[m - 1];
+            left[l] = m - 1;
+        }
+    }
+}
+
 // The sliced form of the matrix (engine.h, DevSell) with entries scaled by
 // scale; real weights' entries in the original order within each row (their
 // FP32 sums keep it).
@@ -1157,17 +1197,12 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
     int32_t *ho = (int32_t *)(buf.data() + bcol + bval), *hd = (int32_t *)(buf.data() + bcol + bval + boff);
     std::fill(col, col + blocks * 128, (uint16_t)(n * scale));
     for (int64_t k = 0; k <= nsl; k++) ho[k] = (int32_t)off[(size_t)k];
-    // The kernels gather the 32 entries that a slice's rows hold at one
-    // position with one shared load, and random rows meet in a bank 2.7 deep
-    // (the gather's wavefronts bounded er800).  Neighbour counts of +-1
-    // weights do not depend on the order, so each position takes, row by row,
-    // an entry whose bank is still free there, or padding while the row has
-    // positions to spare.
     auto place = [&](int64_t k, std::vector<uint16_t> &ent) {
-        const int64_t s0 = 32 * k, rows = std::min<int64_t>(32, n - s0), pos = 4 * (off[(size_t)k + 1] - off[(size_t)k]);
+        const int64_t s0 = 32 * k, pos = 4 * (off[(size_t)k + 1] - off[(size_t)k]);
+        const int rows = (int)std::min<int64_t>(32, n - s0);
         ent.resize((size_t)(32 * pos));
-        int64_t left[32];
-        for (int64_t l = 0; l < rows; l++) {
+        int32_t left[32];
+        for (int l = 0; l < rows; l++) {
             const size_t r = (size_t)J.hperm[(size_t)(s0 + l)];
             uint16_t *v = &ent[(size_t)(l * pos)];
             left[l] = J.hrowptr[r + 1] - J.hrowptr[r];
@@ -1175,33 +1210,7 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
                 *v++ = (uint16_t)((uint32_t)(inv[(size_t)J.hcol[(size_t)e]] * scale) |
                                   (J.hval[(size_t)e] < 0 ? 0x8000u : 0u));
         }
-        for (int64_t j = 0; j < pos; j++) {
-            int32_t word[32];   // the shared word each bank serves at this position
-            std::fill(word, word + 32, -1);
-            for (int64_t t = 0; t < rows; t++) {
-                const int64_t l = t + j % rows < rows ? t + j % rows : t + j % rows - rows;
-                uint16_t *v = &ent[(size_t)(l * pos)];
-                const int64_t m = left[l];
-                if (!m) continue;
-                int64_t pick = m;
-                for (int64_t c = m - 1; c >= 0 && m - c <= 24; c--) {
-                    const int32_t w = (v[c] & 0x7fff) >> 2;
-                    if (word[w & 31] == -1 || word[w & 31] == w) {
-                        pick = c;
-                        break;
-                    }
-                }
-                if (pick == m) {
-                    if (m < pos - j) continue;   // padding here, the entry later
-                    pick = m - 1;
-                }
-                const int32_t w = (v[pick] & 0x7fff) >> 2;
-                word[w & 31] = w;
-                col[(((size_t)off[(size_t)k] + (size_t)(j / 4)) * 32 + (size_t)l) * 4 + (size_t)(j & 3)] = v[pick];
-                v[pick] = v[m - 1];
-                left[l] = m - 1;
-            }
-        }
+        place_entries(ent.data(), pos, rows, left, 0x7fffu, col + off[(size_t)k] * 128);
     };
     for (int64_t s = 0; s < n; s++) hd[s] = degree(s);
     if (J.unit) {
@@ -1281,7 +1290,7 @@ void free_bres(DevBres &B)
 }
 
 // Pack a class for the on-chip batch kernel; leaves bres.rows null when an
-// instance does not fit.  A bin's cluster is the smallest that holds it and,
+// instance does not fit or stepping launch by launch is faster.  A bin's cluster is the smallest that holds it and,
 // when the class alone cannot fill the GPU, splits it down to an SM's share.
 int build_bres(sbx_ctx *ctx, BatchClass &c)
 {
@@ -1290,8 +1299,8 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
     B.tried = true;
     const DevCsr &J = c.J;
     const size_t ni = c.probs.size();
-    int64_t cap[3];
-    for (int k = 0; k < 3; k++) cap[k] = batch_res_rows(1 << k);
+    int64_t cap[4];
+    for (int k = 0; k < 4; k++) cap[k] = batch_res_rows(k);
     const int nsm = std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
     const int64_t share = std::max<int64_t>(512, J.n * (c.Ap / 16) / nsm);   // rows a CTA would hold in one even wave
     std::vector<size_t> ord(ni);
@@ -1299,34 +1308,50 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
     std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return c.probs[a]->J.n > c.probs[b]->J.n; });
     struct Bin {
         std::vector<int32_t> inst;
-        int64_t rows = 0;
-        int k = 0;   // cluster of 2^k CTAs
+        int64_t rows = 0, target = 0;
+        int k = 0;   // kind: clusters of 1, 2, 4 CTAs, and of 4 for the largest
     };
     std::vector<Bin> bins;
-    const int64_t room = std::min(cap[0], std::max<int64_t>(1024, share / 2));   // small instances share bins up to this
-    size_t open = (size_t)-1;   // first one-CTA bin with room (instances come in decreasing size)
+    // A CTA's warps take 32 slices a round, so a bin is filled to whole rounds:
+    // the large instances' bins with small ones, one-CTA bins of small ones up
+    // to a quarter of an SM's share (four waves: the last is seldom full).
+    const int64_t room = std::max<int64_t>(1024, std::min(cap[0], share / 4) / 1024 * 1024);
     for (size_t i : ord) {
         const int64_t n = c.probs[i]->J.n;
         int k = 0;
-        while (k < 3 && (n > cap[k] || (k < 2 && n / (1 << k) > share))) k++;
-        if (k == 3) return SBX_OK;   // too large for a cluster
+        while (k < 4 && (n > cap[k] || (k < 2 && n / batch_res_ctas(k) > share))) k++;
+        if (k == 4) return SBX_OK;   // too large for a cluster
         size_t at = bins.size();
-        if (k == 0) {
-            if (open == (size_t)-1) open = at;
-            while (open < bins.size() && bins[open].rows >= room - 32) open++;
-            for (size_t b = open; b < bins.size() && b < open + 64; b++)
-                if (bins[b].rows + n <= room) {
-                    at = b;
-                    break;
-                }
-        }
+        for (size_t b = 0; b < bins.size(); b++)   // the fullest bin that takes it
+            if (bins[b].rows + n <= bins[b].target && (at == bins.size() || bins[b].target - bins[b].rows < bins[at].target - bins[at].rows))
+                at = b;
         if (at == bins.size()) {
             bins.emplace_back();
-            bins.back().k = k;
+            Bin &b = bins.back();
+            const int64_t round = 1024 * batch_res_ctas(k);
+            b.k = k;
+            b.target = std::min(cap[k], std::max(k == 0 ? room : 0, (n + round - 1) / round * round));
         }
         bins[at].inst.push_back((int32_t)i);
         bins[at].rows += n;
     }
+    // Taken where its step is the shorter one (microseconds, both sides fitted
+    // on GB300 on 1 to 512 instances of 100 to 20,000 rows at 32, 64 and 128
+    // agents): a cluster's step is about 2 + 0.085 per slice of its CTAs at
+    // degree 24, and the step per launch about 6 + 0.06 per thousand rows and
+    // 32 agents.  One instance of 19,909 rows at 64 agents: 15.5 against 7.5;
+    // 32 instances, 154,000 rows: 16.6 against 22.7.
+    double sum = 0, longest = 0;
+    for (const Bin &b : bins) {
+        const int C = batch_res_ctas(b.k);
+        int64_t nnz = 0;
+        for (int32_t i : b.inst) nnz += c.probs[(size_t)i]->J.nnz;
+        const double deg = (double)nnz / (double)b.rows;
+        const double t = 2.0 + 0.085 * (double)(((b.rows + 31) / 32 + C - 1) / C) * (0.4 + 0.6 * deg / 24);
+        sum += t * C * (c.Ap / 16) / nsm;
+        longest = std::max(longest, t);
+    }
+    if (std::max(longest, 1.1 * sum) > 6.0 + 0.06e-3 * (double)J.n * (c.Ap / 32)) return SBX_OK;
     std::stable_sort(bins.begin(), bins.end(),
                      [](const Bin &a, const Bin &b) { return a.k != b.k ? a.k < b.k : a.rows > b.rows; });
     const size_t nb = bins.size();
@@ -1341,7 +1366,6 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
         rows[b] = (int32_t)bins[b].rows;
         if (!B.nbins[bins[b].k]) B.bin0[bins[b].k] = (int32_t)b;
         B.nbins[bins[b].k]++;
-        B.max_rows[bins[b].k] = std::max(B.max_rows[bins[b].k], bins[b].rows);
         slots += bins[b].rows;
         slices += (bins[b].rows + 31) / 32 + 1;
     }
@@ -1385,14 +1409,22 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
         for (size_t b = (size_t)t; b < nb; b += (size_t)TT) {
             for (int64_t s = 0; s < rows[b]; s++) inv[(size_t)perm[(size_t)(slot0[b] + s)]] = (int32_t)s;
             std::fill(col.begin() + (long)(first[b] * 128), col.begin() + (long)((first[b] + blocks[b]) * 128),
-                      (uint16_t)(2 * rows[b]));
+                      (uint16_t)batch_res_entry(bins[b].k, J.allpos, (uint32_t)rows[b], false));
             int32_t *o = &off[(size_t)slice0[b]];
-            for (int64_t s = 0; s < rows[b]; s++) {
-                const size_t r = (size_t)perm[(size_t)(slot0[b] + s)];
-                uint16_t *row = &col[((size_t)(first[b] + o[s / 32]) * 32 + (size_t)(s & 31)) * 4];
-                for (int32_t e = J.hrowptr[r], j = 0; e < J.hrowptr[r + 1]; e++, j++)
-                    row[(size_t)(j / 4) * 128 + (size_t)(j & 3)] =
-                        (uint16_t)(2 * inv[(size_t)J.hcol[(size_t)e]] + (J.hval[(size_t)e] < 0 ? 1 : 0));
+            uint16_t ent[32 * 128];   // degree <= 127: at most 128 positions
+            int32_t left[32];
+            for (int64_t k = 0; 32 * k < rows[b]; k++) {
+                const int64_t pos = 4 * (o[k + 1] - o[k]);
+                const int m = (int)std::min<int64_t>(32, rows[b] - 32 * k);
+                for (int l = 0; l < m; l++) {
+                    const size_t r = (size_t)perm[(size_t)(slot0[b] + 32 * k + l)];
+                    left[l] = J.hrowptr[r + 1] - J.hrowptr[r];
+                    uint16_t *v = ent + l * pos;
+                    for (int32_t e = J.hrowptr[r]; e < J.hrowptr[r + 1]; e++)
+                        *v++ = (uint16_t)batch_res_entry(bins[b].k, J.allpos, (uint32_t)inv[(size_t)J.hcol[(size_t)e]],
+                                                         J.hval[(size_t)e] < 0);
+                }
+                place_entries(ent, pos, m, left, 0xffffu, &col[(size_t)(first[b] + o[k]) * 128]);
             }
             for (int64_t k = 0; k <= (rows[b] + 31) / 32; k++) o[k] += (int32_t)first[b];
         }
@@ -1412,8 +1444,7 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
     return SBX_OK;
 }
 
-// dt * xi0 of each slot's instance, and the bias that turns a byte counter's
-// float into the force.
+// dt * xi0 of each slot's instance, and minus its degree.
 int upload_bres_cb(sbx_ctx *ctx, BatchClass &c, double dt)
 {
     DevBres &B = c.bres;
@@ -1421,7 +1452,7 @@ int upload_bres_cb(sbx_ctx *ctx, BatchClass &c, double dt)
     std::vector<float> cb(2 * B.hinst.size());
     for (size_t s = 0; s < B.hinst.size(); s++) {
         cb[2 * s] = (float)(dt * c.xi0[(size_t)B.hinst[s]]);
-        cb[2 * s + 1] = -(8388608.0f + (float)B.hdeg[s]);
+        cb[2 * s + 1] = -(float)B.hdeg[s];
     }
     CK(cudaMemcpy(B.cb, cb.data(), sizeof(float) * cb.size(), cudaMemcpyHostToDevice));
     B.dt = dt;
@@ -1790,7 +1821,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         c.J.bsm = nullptr;
         if (use_res) {
             if ((rc = upload_bres_cb(ctx, c, pr->dt))) return rc;
-            for (int k = 0; k < 3; k++) {
+            for (int k = 0; k < 4; k++) {
                 if (!ctx->side[k]) CK(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
                 if (!ctx->join[k]) CK(cudaEventCreateWithFlags(&ctx->join[k], cudaEventDisableTiming));
             }
@@ -2099,7 +2130,7 @@ int sbx_destroy(sbx_ctx *ctx)
     if (!ctx) return SBX_ERR_ARG;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (int k = 0; k < 3; k++) {
+    for (int k = 0; k < 4; k++) {
         if (ctx->side[k]) cudaStreamDestroy(ctx->side[k]);
         if (ctx->join[k]) cudaEventDestroy(ctx->join[k]);
     }

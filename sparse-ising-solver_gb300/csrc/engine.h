@@ -189,15 +189,15 @@ struct DevBsm {
 
 // A batch class packed for the on-chip batch kernel (k_batch_res.cu): whole
 // instances in bins, a bin's rows by decreasing degree ("slots") in slices of
-// 32 (as DevSell); the bins listed by cluster size 1, 2, 4, largest first.
+// 32 (as DevSell); the bins listed by kind -- clusters of 1, 2 and 4 CTAs, and
+// of 4 for bins past 16,383 rows -- each largest first.
 struct DevBres {
     bool tried = false;          // planned (rows is null when the class does not fit)
     int32_t *bins = nullptr, *slot0 = nullptr, *slice0 = nullptr, *rows = nullptr, *off = nullptr;
-    void *col = nullptr;         // [blocks][32] of four entries 2 slot + sign
-    void *cb = nullptr;          // per slot: dt * xi0, -(2^23 + degree)
+    void *col = nullptr;         // [blocks][32] of four entries (batch_res_entry)
+    void *cb = nullptr;          // per slot: dt * xi0, -degree
     int32_t *perm = nullptr;     // slot -> class row
-    int32_t bin0[3] = {0, 0, 0}, nbins[3] = {0, 0, 0};
-    int64_t max_rows[3] = {0, 0, 0};
+    int32_t bin0[4] = {}, nbins[4] = {};
     std::vector<int32_t> hinst, hdeg;   // per slot: instance, degree
     double dt = -1;              // dt of the uploaded cb
 };
@@ -282,10 +282,13 @@ cudaError_t launch_resident(const SolveDims &d, const DevCsr &J, Work &w, int ka
 int64_t resident_batch_max_rows();
 cudaError_t launch_resident_batch(const SolveDims &d, const DevRb &B, Work &w, cudaStream_t s);
 
-// On-chip batch kernel (k_batch_res.cu): most rows of a bin on a cluster of C
-// CTAs; all d.steps_run fused steps of every bin, the cluster sizes on the
-// side streams between fork and join.  agents: the class's largest count.
-int64_t batch_res_rows(int C);
+// On-chip batch kernel (k_batch_res.cu), kinds 0..3 of bins (DevBres): the
+// CTAs of a bin's cluster, its most rows, the entry of a neighbour.  The
+// launch runs all d.steps_run fused steps of every bin, the kinds on the side
+// streams between fork and join.  agents: the class's largest count.
+int batch_res_ctas(int kind);
+int64_t batch_res_rows(int kind);
+uint32_t batch_res_entry(int kind, bool allpos, uint32_t slot, bool neg);
 cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, int32_t agents, Work &w,
                              cudaStream_t s, cudaStream_t *side, cudaEvent_t fork, cudaEvent_t *join,
                              int *launches);

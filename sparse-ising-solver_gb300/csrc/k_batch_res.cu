@@ -13,8 +13,8 @@
 // columns (L2) and shared and tensor memory.
 //
 // Rows.  A bin's rows are in decreasing degree ("slots"), in slices of 32;
-// CTA r of the cluster takes slices r, r + C, ...  A thread's rows are one of
-// each 1,024; x and y of 16 agents are 64 bytes: the first 4 rows of a thread
+// CTA r of the cluster takes slices r, r + C, ..., its warps a round of 32 of
+// them at a time, forwards and backwards in turn (equal work to the barrier); x and y of 16 agents are 64 bytes: the first 4 rows of a thread
 // in tensor memory (16 columns each of its own lane), the rest in shared
 // memory.  Every CTA holds the signs of all the bin's rows, a 16-bit word a
 // row, double-buffered; a new word is stored to all CTAs of the cluster
@@ -46,14 +46,24 @@ struct BresP {
     const int32_t *__restrict__ rows;    // per bin: rows
     const int32_t *__restrict__ off;     // per slice: first block, and the end after a bin's last slice
     const uint2 *__restrict__ col;       // [blocks][32]
-    const float2 *__restrict__ cb;       // per slot: dt * xi0 of its instance, -(2^23 + degree)
+    const float2 *__restrict__ cb;       // per slot: dt * xi0 of its instance, -degree
     const int32_t *__restrict__ perm;    // slot -> state row
     const float4 *__restrict__ coef;
     void *x, *y;                         // global [rows][Ap]
     uint32_t *Wp;                        // global plane [rows][W]: signs of the last step
     int32_t *ctl;
-    int32_t Ap, W, groups, nsteps, allpos;
+    int32_t Ap, W, groups, nsteps;
+    uint32_t smem;                       // bytes of dynamic shared memory
 };
+
+// Shared memory: the sign planes at kPlane and 2 kPlane of the CTA's shared
+// window, the rows past tensor memory's in chunks of 32 (a warp's, [4 pieces of
+// 16 bytes][32]) before (from kFirst), between and after them.
+constexpr uint32_t kPlane = 0x10000, kChunk = 2048, kFirst = 0x800;
+// Sign planes of all +1 or +-1 weights as 16-bit words (the sign in bit 0 of
+// an entry), or words with their complement.
+enum { BR_POS = 0, BR_BIT = 1, BR_DUAL = 2 };
+template <int MODE> constexpr uint32_t kRowB = MODE == BR_DUAL ? 4 : 2;   // bytes of a row's signs
 
 struct Row16 {
     uint32_t x[8], y[8];   // packed pairs of 16 agents
@@ -62,7 +72,7 @@ struct Row16 {
 __device__ __forceinline__ uint32_t lds16(uint32_t a)
 {
     uint32_t v;
-    asm volatile("{\n\t.reg .u16 h;\n\tld.shared.u16 h, [%1];\n\tcvt.u32.u16 %0, h;\n\t}" : "=r"(v) : "r"(a) : "memory");
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ void tm_ld16(uint32_t ta, Row16 &v)
@@ -85,18 +95,20 @@ __device__ __forceinline__ void tm_st16(uint32_t ta, const Row16 &v)
                  "r"(v.y[6]), "r"(v.y[7])
                  : "memory");
 }
-// Address of the same shared location in CTA `rank` of the cluster, and a
-// 16-bit store there.
+// Address of the same shared location in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t peer(uint32_t a, uint32_t rank)
 {
     uint32_t d;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(rank));
     return d;
 }
-__device__ __forceinline__ void st_peer16(uint32_t a, uint32_t v)
+// A row's signs, 2 or 4 bytes, into this CTA's shared memory or a peer's.
+template <int BYTES, bool PEER> __device__ __forceinline__ void st_sign(uint32_t a, uint32_t v)
 {
-    asm volatile("{\n\t.reg .u16 h;\n\tcvt.u16.u32 h, %1;\n\tst.shared::cluster.u16 [%0], h;\n\t}" ::"r"(a), "r"(v)
-                 : "memory");
+    if (BYTES == 4 && PEER) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else if (BYTES == 4) asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else if (PEER) asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+    else asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
 }
 // All threads of the cluster's CTAs; orders their shared stores.
 template <int C> __device__ __forceinline__ void step_barrier()
@@ -108,34 +120,40 @@ template <int C> __device__ __forceinline__ void step_barrier()
     }
 }
 
-// A block's four neighbour words as two 32-bit words of two, the weights'
-// signs (bit 0 of an entry) applied.
-template <bool NEG> __device__ __forceinline__ void block_words(const uint2 &c, uint32_t S, uint32_t &w0, uint32_t &w1)
+// A block's four neighbour words as two 32-bit words of two.  S: the plane's
+// shared address, a multiple of 64 KB.
+template <int MODE> __device__ __forceinline__ void block_words(const uint2 &c, uint32_t S, uint32_t &w0, uint32_t &w1)
 {
-    const uint32_t u0 = NEG ? c.x & 0xfffefffeu : c.x, u1 = NEG ? c.y & 0xfffefffeu : c.y;
-    w0 = __byte_perm(lds16(S + (u0 & 0xffffu)), lds16(S + (u0 >> 16)), 0x5410);
-    w1 = __byte_perm(lds16(S + (u1 & 0xffffu)), lds16(S + (u1 >> 16)), 0x5410);
-    if (NEG) {   // 0 or 0xffff per half
+    const uint32_t u0 = MODE == BR_BIT ? c.x & 0xfffefffeu : c.x, u1 = MODE == BR_BIT ? c.y & 0xfffefffeu : c.y;
+    w0 = __byte_perm(lds16(__byte_perm(u0, S, 0x7610)), lds16(__byte_perm(u0, S, 0x7632)), 0x5410);
+    w1 = __byte_perm(lds16(__byte_perm(u1, S, 0x7610)), lds16(__byte_perm(u1, S, 0x7632)), 0x5410);
+    if (MODE == BR_BIT) {   // 0 or 0xffff per half
         w0 ^= (c.x & 0x00010001u) * 0xffffu;
         w1 ^= (c.y & 0x00010001u) * 0xffffu;
     }
 }
 
-// Byte counters of 2 * count over nb blocks: agents 8 h .. 8 h + 3 in
-// cnt[2 h], 8 h + 4 .. 8 h + 7 in cnt[2 h + 1].  PL planes hold the 2 nb
-// entries of a half word (2 nb < 2^PL).
-template <int PL, bool NEG>
-__device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32_t S, uint32_t (&cnt)[4])
+// Counts of the neighbours whose term is -1 over nb blocks as bit planes: bit
+// j of p[k] is bit k of agent j's count.  PL planes hold the 2 nb entries of
+// a half word (2 nb < 2^PL); one plane more comes out, seven at most (degree
+// <= 127).
+template <int PL, int MODE>
+__device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32_t S, uint32_t (&p)[7])
 {
-    uint32_t p[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 7; k++) p[k] = 0;
+    // the next two blocks' columns (L2) in flight while two are counted
+    uint2 n0 = make_uint2(0, 0), n1 = n0;
+    if (nb > 0) n0 = __ldg(cp);
+    if (nb > 1) n1 = __ldg(cp + 32);
     for (int32_t b = 0; b < nb; b += 2) {
-        const uint2 c0 = __ldg(cp + b * 32);
+        const uint2 c0 = n0, c1 = n1;
         const bool two = b + 1 < nb;   // warp-uniform
-        uint2 c1;
-        if (two) c1 = __ldg(cp + (b + 1) * 32);
+        if (b + 2 < nb) n0 = __ldg(cp + (b + 2) * 32);
+        if (b + 3 < nb) n1 = __ldg(cp + (b + 3) * 32);
         uint32_t w0, w1, w2 = 0u, w3 = 0u;
-        block_words<NEG>(c0, S, w0, w1);
-        if (two) block_words<NEG>(c1, S, w2, w3);
+        block_words<MODE>(c0, S, w0, w1);
+        if (two) block_words<MODE>(c1, S, w2, w3);
         const uint32_t a = fadd(p[0], w0, w1), d = fadd(p[0], w2, w3);
         uint32_t c = fadd(p[1], a, d);
 #pragma unroll
@@ -157,30 +175,39 @@ __device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32
             c = fadd(p[k], b, c);
         }
     }
-    if (PL < 7) p[PL] = c;   // counts are at most 127: seven planes
+    if (PL < 7) p[PL] = c;
+}
+
+// The force 2 count - degree of agents 8 h .. 8 h + 7 from the planes.  Byte h
+// of planes 0 to 3 in one word, of 4 to 6 in another; agent q's bits of both
+// (2^q each) times twice their planes' weights, added to the bits of 2^23 by
+// byte dot products, are the float 2^23 + 2^q 2 count, and one FMA scales that
+// by 2^-q and takes 2^(23 - q) + degree off: every step is exact.  (An 8x8 bit
+// transpose and a PRMT per agent took 70 ALU instructions for 16 agents, this
+// takes 42; dot products run on the FMA pipe.)
+__device__ __forceinline__ void force8(const uint32_t (&p)[7], int h, float negdeg, float (&tv)[8])
+{
+    const uint32_t s01 = (uint32_t)h | (((uint32_t)h + 4) << 4);
+    const uint32_t lo = __byte_perm(__byte_perm(p[0], p[1], s01), __byte_perm(p[2], p[3], s01), 0x5410);
+    const uint32_t hi = __byte_perm(__byte_perm(p[4], p[5], s01), p[6] >> (8 * h), 0x5410);
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        // byte h of each plane, shifted up a byte (which doubles the counts),
-        // then an 8x8 bit transpose
-        const uint32_t s01 = (uint32_t)h | (((uint32_t)h + 4) << 4);
-        uint32_t lo = __byte_perm(__byte_perm(0u, p[0], s01), __byte_perm(p[1], p[2], s01), 0x5410);
-        uint32_t hi = __byte_perm(__byte_perm(p[3], p[4], s01), __byte_perm(p[5], p[6], s01), 0x5410);
-        uint32_t t;
-        t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
-        lo ^= t ^ (t << 7);
-        t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
-        hi ^= t ^ (t << 7);
-        t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
-        lo ^= t ^ (t << 14);
-        t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
-        hi ^= t ^ (t << 14);
-        t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
-        cnt[2 * h] = lo ^ t;
-        cnt[2 * h + 1] = hi ^ (t >> 4);
+    for (int q = 0; q < 8; q += 2) {
+        float f[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const uint32_t m = 0x01010101u << (q + e);
+            const uint32_t v = __dp4a(lo & m, 0x10080402u, 0x4b000000u);
+            f[e] = __uint_as_float(__dp4a(hi & m, 0x00804020u, v));
+        }
+        const float a = 1.0f / (1 << q), b = 8388608.0f / (1 << q);
+        const float2 t = __ffma2_rn(make_float2(f[0], f[1]), make_float2(a, 0.5f * a),
+                                    __fadd2_rn(make_float2(negdeg, negdeg), make_float2(-b, -0.5f * b)));
+        tv[q] = t.x;
+        tv[q + 1] = t.y;
     }
 }
 
-template <class T, int C, bool NEG>
+template <class T, int C, int MODE>
 __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
 {
     static_assert(sizeof(T) == 2, "16-bit state: 16 agents in 32 bytes");
@@ -193,10 +220,32 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
     const int a0 = (unit % P.groups) * 16;
     const int R = __ldg(&P.rows[bin]), sl0 = __ldg(&P.slice0[bin]), s0 = __ldg(&P.slot0[bin]);
     const int nsl = (R + 31) / 32, mine = (nsl - rank + C - 1) / C;   // the bin's slices, this CTA's
-    const int ns = max(0, 32 * mine - kTmRows * kNT);                 // rows kept in shared memory
-    const uint32_t pb = ((uint32_t)(R + 1) * 2 + 15) & ~15u;          // bytes of a sign plane
-    const uint32_t sb = smem_u32(smem);
-    uint4 *st = (uint4 *)(smem + 2 * pb);                             // [4 pieces][ns]
+    // A CTA's window of the shared address space starts at a multiple of 16 MB
+    // (its rank in the cluster); below, offsets in the window.
+    const uint32_t sb = smem_u32(smem), win = sb & 0xff000000u, so = sb - win;
+    const uint32_t pb = ((uint32_t)(R + 1) * kRowB<MODE> + 15) & ~15u;   // bytes of a sign plane
+    // chunks before, between and after the planes
+    const uint32_t q0 = (kPlane - kFirst) / kChunk, q1 = (kPlane - pb) / kChunk, q2 = (P.smem - 2 * kPlane - pb) / kChunk;
+    // Never expected, the host leaves room: the layout does not fit.  The
+    // CTAs of a cluster agree before any of them leaves.
+    __shared__ uint32_t s_bad;
+    if (tid == 0)
+        s_bad = so > kFirst || pb > kPlane || 2 * kPlane + pb > P.smem || mine - kTmRows * (kNT / 32) > (int)(q0 + q1 + q2);
+    step_barrier<C>();
+    uint32_t bad = 0;
+    if (C == 1) bad = s_bad;
+#pragma unroll
+    for (int c = 0; c < C; c++)
+        if (C > 1) {
+            uint32_t v;
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer(smem_u32(&s_bad), (uint32_t)c)) : "memory");
+            bad |= v;
+        }
+    if (bad) {
+        if (tid == 0) atomicExch(&P.ctl[CTL_ERR], 1);
+        step_barrier<C>();
+        return;
+    }
     T *xg = (T *)P.x, *yg = (T *)P.y;
 
     // All of the SM's tensor memory: 1,024 threads of 64 registers leave room
@@ -207,8 +256,8 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {   // the zero row that padded entries read
-        ((uint16_t *)smem)[R] = 0;
-        ((uint16_t *)(smem + pb))[R] = 0;
+        st_sign<kRowB<MODE>, false>(win + kPlane + kRowB<MODE> * (uint32_t)R, 0xffff0000u);
+        st_sign<kRowB<MODE>, false>(win + 2 * kPlane + kRowB<MODE> * (uint32_t)R, 0xffff0000u);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     step_barrier<C>();   // the cluster's CTAs are running: their shared memory may be written
@@ -216,14 +265,24 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
     const uint32_t tmem = s_tmem;
     const uint32_t tw = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(16 * kTmRows * (warp >> 2));
 
+    // the CTA's slice that this warp takes in round i
+    auto slice = [&](int i) { return 32 * i + ((i & 1) ? 31 - warp : warp); };
+    // this lane's piece 0 of the chunk of round i (past tensor memory's)
+    auto chunk = [&](int i) {
+        const uint32_t q = (uint32_t)(slice(i) - kTmRows * (kNT / 32));
+        const uint32_t a = q < q0 ? kFirst + q * kChunk
+                                  : q < q0 + q1 ? kPlane + pb + (q - q0) * kChunk
+                                                : 2 * kPlane + pb + (q - q0 - q1) * kChunk;
+        return (uint4 *)(smem + (a - so)) + lane;
+    };
     auto get_row = [&](int i, Row16 &v) {
         if (i < kTmRows) {
             tm_ld16(tw + 16u * (uint32_t)i, v);
         } else {
-            const int r = (i - kTmRows) * kNT + tid;
+            const uint4 *c = chunk(i);
 #pragma unroll
             for (int p = 0; p < 4; p++) {
-                const uint4 u = st[p * ns + r];
+                const uint4 u = c[32 * p];
                 memcpy((unsigned char *)&v + 16 * p, &u, 16);
             }
         }
@@ -232,26 +291,22 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
         if (i < kTmRows) {
             tm_st16(tw + 16u * (uint32_t)i, v);
         } else {
-            const int r = (i - kTmRows) * kNT + tid;
+            uint4 *c = chunk(i);
 #pragma unroll
             for (int p = 0; p < 4; p++) {
                 uint4 u;
                 memcpy(&u, (const unsigned char *)&v + 16 * p, 16);
-                st[p * ns + r] = u;
+                c[32 * p] = u;
             }
         }
     };
-    uint32_t pk[C];   // the planes' base in every CTA of the cluster
+    uint32_t pk[C];   // the window of every CTA of the cluster
 #pragma unroll
-    for (int c = 0; c < C; c++) pk[c] = C == 1 ? sb : peer(sb, (uint32_t)c);
-    auto put_sign = [&](uint32_t o, uint32_t w) {
-        if (C == 1) {
-            asm volatile("{\n\t.reg .u16 h;\n\tcvt.u16.u32 h, %1;\n\tst.shared.u16 [%0], h;\n\t}" ::"r"(sb + o), "r"(w)
-                         : "memory");
-        } else {
+    for (int c = 0; c < C; c++) pk[c] = C == 1 ? win : peer(sb, (uint32_t)c) - so;
+    auto put_sign = [&](uint32_t plane, int s, uint32_t w) {
+        const uint32_t v = MODE == BR_DUAL ? w | (~w << 16) : w, a = plane + kRowB<MODE> * (uint32_t)s;
 #pragma unroll
-            for (int c = 0; c < C; c++) st_peer16(pk[c] + o, w);
-        }
+        for (int c = 0; c < C; c++) st_sign<kRowB<MODE>, (C > 1)>(pk[c] + a, v);
     };
     // signs of a row's 16 agents, agent j in bit j
     auto sign_word = [&](const Row16 &v) {
@@ -265,8 +320,8 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
     // The state after the pre-step Update_XY of step 0 (src/ising.cu:188),
     // computed and rounded as the streaming pre-step does.
     const float4 c00 = P.coef[0];
-    for (int i = 0; 32 * i + warp < mine; i++) {
-        const int s = 32 * ((32 * i + warp) * C + rank) + lane;   // slot of the bin
+    for (int i = 0; slice(i) < mine; i++) {
+        const int s = 32 * (slice(i) * C + rank) + lane;   // slot of the bin
         Row16 v = {};
         if (s < R) {
             const int64_t g = (int64_t)__ldg(&P.perm[s0 + s]) * P.Ap + a0;
@@ -288,7 +343,7 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
                 memcpy(&v.x[4 * h], &xr.u, 16);
                 memcpy(&v.y[4 * h], &yr.u, 16);
             }
-            put_sign(2u * (uint32_t)s, sign_word(v));   // step 0 reads plane 0
+            put_sign(kPlane, s, sign_word(v));   // step 0 reads the first plane
         }
         put_row(i, v);
     }
@@ -297,32 +352,22 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
 
     for (int32_t k = 0; k < P.nsteps; k++) {
         const float4 ck = __ldg(&P.coef[k]);
-        const uint32_t Sin = sb + ((k & 1) ? pb : 0u), onx = (k & 1) ? 0u : pb;
-        for (int i = 0; 32 * i + warp < mine; i++) {
-            const int sl = (32 * i + warp) * C + rank, s = 32 * sl + lane;
+        const uint32_t Sin = win + ((k & 1) ? 2 * kPlane : kPlane), Snx = (k & 1) ? kPlane : 2 * kPlane;
+        for (int i = 0; slice(i) < mine; i++) {
+            const int sl = slice(i) * C + rank, s = 32 * sl + lane;
             const bool live = s < R;
             const int32_t b0 = __ldg(&P.off[sl0 + sl]), nb = __ldg(&P.off[sl0 + sl + 1]) - b0;   // warp-uniform
             const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
             const float2 cb = __ldg(&P.cb[s0 + min(s, R - 1)]);
-            uint32_t cnt[4];
-            if (nb < 8) count_blocks<4, NEG>(cp, nb, Sin, cnt);
-            else count_blocks<7, NEG>(cp, nb, Sin, cnt);   // degree <= 127: at most 32 blocks
+            uint32_t p[7];
+            if (nb < 8) count_blocks<4, MODE>(cp, nb, Sin, p);
+            else count_blocks<7, MODE>(cp, nb, Sin, p);   // degree <= 127: at most 32 blocks
             Row16 v;
             get_row(i, v);
-            const float2 bias = make_float2(cb.y, cb.y);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 float tv[8];
-#pragma unroll
-                for (int q = 0; q < 8; q += 2) {
-                    const uint32_t w = cnt[2 * h + (q >> 2)];
-                    const float2 t =
-                        __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + (q & 3))),
-                                               __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7441u + (q & 3)))),
-                                   bias);
-                    tv[q] = t.x;
-                    tv[q + 1] = t.y;
-                }
+                force8(p, h, cb.y, tv);
                 uint32_t x[4], y[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -337,15 +382,15 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
                 }
             }
             put_row(i, v);
-            if (live) put_sign(onx + 2u * (uint32_t)s, sign_word(v));
+            if (live) put_sign(Snx, s, sign_word(v));
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         step_barrier<C>();
     }
 
     // the state and the signs of the last step back to global memory
-    for (int i = 0; 32 * i + warp < mine; i++) {
-        const int s = 32 * ((32 * i + warp) * C + rank) + lane;
+    for (int i = 0; slice(i) < mine; i++) {
+        const int s = 32 * (slice(i) * C + rank) + lane;
         Row16 v;
         get_row(i, v);
         if (s < R) {
@@ -368,23 +413,28 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
-// Dynamic shared memory of a bin of R rows on C CTAs.
-int64_t smem_bytes(int64_t R, int C)
+// Dynamic shared memory of a launch, and whether a bin of R rows fits C CTAs
+// with it (the kernel's layout).
+uint32_t smem_bytes() { return (uint32_t)std::max(0, dev_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024); }
+bool fits(int64_t R, int C, uint32_t row_bytes, uint32_t smem)
 {
-    const int64_t nsl = (R + 31) / 32, mine = (nsl + C - 1) / C;
-    return 2 * (((R + 1) * 2 + 15) / 16 * 16) + std::max<int64_t>(0, 32 * mine - kTmRows * kNT) * 64;
+    const int64_t pb = ((R + 1) * row_bytes + 15) / 16 * 16;
+    if (pb > kPlane || 2 * (int64_t)kPlane + pb > (int64_t)smem) return false;
+    const int64_t chunks = (kPlane - kFirst) / kChunk + (kPlane - pb) / kChunk + (smem - 2 * (int64_t)kPlane - pb) / kChunk;
+    const int64_t mine = ((R + 31) / 32 + C - 1) / C;
+    return mine - kTmRows * (kNT / 32) <= chunks;
 }
 
-template <class T, int C>
-cudaError_t launch_c(const BresP &P, int units, size_t smem, cudaStream_t s)
+template <class T, int C, int MODE>
+cudaError_t launch_m(const BresP &P, int units, cudaStream_t s)
 {
-    auto kern = P.allpos ? k_batch_res<T, C, false> : k_batch_res<T, C, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto kern = k_batch_res<T, C, MODE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(units * C));
     cfg.blockDim = dim3(kNT);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = P.smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -397,28 +447,36 @@ cudaError_t launch_c(const BresP &P, int units, size_t smem, cudaStream_t s)
 }
 
 template <class T>
-cudaError_t launch_t(const BresP &P, int C, int units, size_t smem, cudaStream_t s)
+cudaError_t launch_t(const BresP &P, int c, bool allpos, int units, cudaStream_t s)
 {
-    switch (C) {
-    case 1: return launch_c<T, 1>(P, units, smem, s);
-    case 2: return launch_c<T, 2>(P, units, smem, s);
-    case 4: return launch_c<T, 4>(P, units, smem, s);
-    default: return cudaErrorInvalidValue;
+    switch (c) {
+    case 0: return allpos ? launch_m<T, 1, BR_POS>(P, units, s) : launch_m<T, 1, BR_DUAL>(P, units, s);
+    case 1: return allpos ? launch_m<T, 2, BR_POS>(P, units, s) : launch_m<T, 2, BR_DUAL>(P, units, s);
+    case 2: return allpos ? launch_m<T, 4, BR_POS>(P, units, s) : launch_m<T, 4, BR_DUAL>(P, units, s);
+    default: return allpos ? launch_m<T, 4, BR_POS>(P, units, s) : launch_m<T, 4, BR_BIT>(P, units, s);
     }
 }
 
 }  // namespace
 
-int64_t batch_res_rows(int C)
+int batch_res_ctas(int c) { return c == 3 ? 4 : 1 << c; }
+
+int64_t batch_res_rows(int c)
 {
-    const int64_t budget = (int64_t)dev_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024;
-    int64_t lo = 0, hi = 32767;   // most rows whose shared memory fits (15-bit slots)
+    const uint32_t smem = smem_bytes();
+    const int C = batch_res_ctas(c);
+    int64_t lo = 0, hi = c == 3 ? 32767 : 16383;   // offsets of 16 bits
     while (lo < hi) {
         const int64_t mid = (lo + hi + 1) / 2;
-        if (smem_bytes(mid, C) <= budget) lo = mid;
+        if (fits(mid, C, c == 3 ? 2 : 4, smem)) lo = mid;
         else hi = mid - 1;
     }
     return lo;
+}
+
+uint32_t batch_res_entry(int c, bool allpos, uint32_t slot, bool neg)
+{
+    return allpos || c == 3 ? 2 * slot + neg : 4 * slot + 2 * neg;
 }
 
 cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, int32_t agents, Work &w,
@@ -441,20 +499,19 @@ cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, 
     P.W = d.W;
     P.groups = (agents + 15) / 16;   // groups of padded agents alone stay as they began
     P.nsteps = d.steps_run;
-    P.allpos = allpos ? 1 : 0;
+    P.smem = smem_bytes();
     // the cluster sizes on streams of their own, largest first: the smaller
     // ones' CTAs fill the SMs that whole clusters leave
     cudaError_t e = cudaEventRecord(fork, s);
     int nside = 0;
-    for (int c = 2; c >= 0 && e == cudaSuccess; c--) {
+    for (int c = 3; c >= 0 && e == cudaSuccess; c--) {
         if (!B.nbins[c]) continue;
         P.bins = B.bins + B.bin0[c];
         cudaStream_t t = side[nside];
         e = cudaStreamWaitEvent(t, fork, 0);
         if (e != cudaSuccess) break;
-        const int C = 1 << c, units = B.nbins[c] * P.groups;
-        const size_t smem = (size_t)smem_bytes(B.max_rows[c], C);
-        e = d.prec == P_BF16 ? launch_t<__nv_bfloat16>(P, C, units, smem, t) : launch_t<__half>(P, C, units, smem, t);
+        const int units = B.nbins[c] * P.groups;
+        e = d.prec == P_BF16 ? launch_t<__nv_bfloat16>(P, c, allpos, units, t) : launch_t<__half>(P, c, allpos, units, t);
         if (e == cudaSuccess) e = cudaEventRecord(join[nside], t);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join[nside], 0);
         nside++;
