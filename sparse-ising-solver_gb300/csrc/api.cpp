@@ -1788,7 +1788,8 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
                            (!c.J.unit || c.J.max_deg <= kHeavy) && c.J.n < (int64_t)1 << 30 && nchunks > 0;
         // Each 4-agent CTA re-reads its bin's rows every step and gathers
         // neighbour signs from shared memory, so by itself the resident batch
-        // is taken only for low-degree classes (mean degree <= 8); measured on
+        // is taken only for low-degree classes (mean degree <= 8) that neither
+        // the on-chip kernel nor the plane kernel takes (below); measured on
         // GB300 it trails the streaming kernel at degree ~20.
         const bool low_degree = c.J.nnz <= 8 * c.J.n;
         const bool want_rb = (pr->kernel == SBX_KERNEL_AUTO && low_degree) || pr->kernel == SBX_KERNEL_RESIDENT ||
@@ -1796,7 +1797,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         if (pr->kernel != SBX_KERNEL_AUTO && pr->kernel != SBX_KERNEL_STREAM && !rb_ok)
             return fail(ctx, SBX_ERR_UNSUPPORTED,
                         "batched resident kernel: fused 16-bit state, degree <= 127, instances that fit on chip");
-        const bool use_rb = want_rb && rb_ok;
+        bool use_rb = want_rb && rb_ok;
         // the shared-memory-plane step kernel, unless a streaming tile or
         // another count mode is asked for (count_mode 4 insists on it)
         const bool bsm_threads = pr->block_threads == 512 || pr->block_threads == 640 || pr->block_threads == 1024;
@@ -1811,13 +1812,20 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
                              pr->kernel != SBX_KERNEL_RESIDENT_SPLIT;
         // the on-chip batch kernel: +-1 fused 16-bit classes whose instances
         // fit a cluster, unless a tile, a count mode or a kernel is asked for
-        bool use_res = !use_rb && !tile_pinned && !bsm_threads && !pr->count_mode && pr->kernel == SBX_KERNEL_AUTO &&
+        // (256 tori of 947,961 rows in all at 64 agents: 52 us a step, the
+        // resident batch 94, the plane kernel 97)
+        const bool by_itself = pr->kernel == SBX_KERNEL_AUTO;
+        bool use_res = (!use_rb || by_itself) && !tile_pinned && !bsm_threads && !pr->count_mode && pr->kernel == SBX_KERNEL_AUTO &&
                        (d.prec == P_BF16 || d.prec == P_F16) && d.fused && !d.trace && nchunks > 0 && c.J.unit &&
                        c.J.max_deg <= kHeavy;
         if (use_res) {
             if (!c.bres.tried && (rc = build_bres(ctx, c))) return rc;
             use_res = c.bres.rows != nullptr;
+            if (use_res) use_rb = false;
         }
+        // ... else the plane kernel before the resident batch, which it also
+        // outruns at low degree (8 tori, 25,369 rows: 7.7 us a step against 18.7)
+        if (use_rb && by_itself && !tile_pinned && bsm_ok(c, d)) use_rb = false;
         c.J.bsm = nullptr;
         if (use_res) {
             if ((rc = upload_bres_cb(ctx, c, pr->dt))) return rc;
@@ -1932,7 +1940,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             r->xi0 = c.xi0[i];
             r->steps_run = total;
             r->windows_run = nchunks;
-            r->kernel_used = use_rb ? SBX_KERNEL_RESIDENT : SBX_KERNEL_STREAM;
+            r->kernel_used = use_rb || (use_res && low_degree) ? SBX_KERNEL_RESIDENT : SBX_KERNEL_STREAM;
             r->agents_per_block = use_rb ? 4 : use_res ? 16 : 0;
             r->kernel_launches = launches;
             r->kernel_ms = use_rb || use_res ? (profile ? ms : 0.0) : kms;
