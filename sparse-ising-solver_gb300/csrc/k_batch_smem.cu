@@ -218,17 +218,17 @@ __global__ void __launch_bounds__(NT, 1) k_bsm(const StepP P, const BsmP B, cons
                 // the counts of chunk k: cnt[2k], cnt[2k + 1] (word order), or
                 // in the interleaved order cnt[4 (k % 2) + 2 (k / 2)] ...
                 const int ci = IL ? 4 * (k % 2) + 2 * (k / 2) : 2 * k;
-                float tv[8], x[8], y[8];
+                float tv[8];
 #pragma unroll
                 for (int v = 0; v < 8; v++)
                     tv[v] = __uint_as_float(__byte_perm(cnt[ci + v / 4], 0x4b000000u, 0x7440u + (v & 3))) - bias;
-                to_vals<T, 8>(xr[k], x);
-                to_vals<T, 8>(yr[k], y);
-                sb_update<KIND, WIN, 8>(x, y, tv, c0, c, cn);
-#pragma unroll
-                for (int v = 0; v < 8; v++) b |= sbit(x[v]) << (8 * k + v);
-                xr[k] = from_vals<T, 8>(x);
-                yr[k] = from_vals<T, 8>(y);
+                uint32_t x[4], y[4];
+                memcpy(x, &xr[k].u, 16);
+                memcpy(y, &yr[k].u, 16);
+                sb_update16<T, KIND, WIN, 8>(x, y, tv, c0, c, cn);
+                b |= sign_bits16<8>(x) << (8 * k);
+                memcpy(&xr[k].u, x, 16);
+                memcpy(&yr[k].u, y, 16);
             }
             if (IL) {
                 // byte k of b: the signs of chunk 2 k + q; word q is the

@@ -21,8 +21,8 @@
 // put together in a word and XORed with the four weights' signs (one PRMT
 // makes the mask); the words add up in bit planes, full adders over four
 // byte lanes at once, as many planes as the row's blocks can fill; the lanes
-// are then summed plane by plane and the planes transposed into byte
-// counters.  Bound: issue.
+// are then summed plane by plane and the planes turned into forces by byte dot
+// products.  Bound: issue and the ALU pipe.
 #include "k_step.cuh"
 
 #include <algorithm>
@@ -118,22 +118,25 @@ template <int N, int SH> __device__ __forceinline__ void fold(uint32_t (&p)[8])
     p[N] = c;
 }
 
-// Byte counters of 2 * count over nb blocks (fewer than 2^PL): agents 0..3 in lo,
-// 4..7 in hi.
-template <int PL>
-__device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32_t S, bool neg, uint32_t &lo,
-                                             uint32_t &hi)
+// The force 2 count - degree of KA agents over nb blocks (fewer than 2^PL).
+// The byte lanes' planes are summed; then a byte of each of planes 0 to 3 in
+// one word, of 4 to 6 in another, and agent q's bits (2^q each) times twice
+// their planes' weights, added to the bits of 2^23 by byte dot products (FMA
+// pipe), are the float 2^23 + 2^q 2 count; one FMA scales that by 2^-q and
+// takes 2^(23 - q) + degree off, exactly.
+template <int PL, int KA, bool NEG>
+__device__ __forceinline__ void count_force(const uint2 *cp, int32_t nb, uint32_t S, float negdeg, float (&tv)[8])
 {
     uint32_t p[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (PL == 1) {
-        p[0] = block_word(__ldg(cp), S, neg);
+        p[0] = nb ? block_word(__ldg(cp), S, NEG) : 0u;
     } else {
         for (int32_t b = 0; b < nb; b += 2) {
             const uint2 c0 = __ldg(cp + b * 32);
             uint2 c1;
             const bool two = b + 1 < nb;   // warp-uniform
             if (two) c1 = __ldg(cp + (b + 1) * 32);
-            const uint32_t w0 = block_word(c0, S, neg), w1 = two ? block_word(c1, S, neg) : 0u;
+            const uint32_t w0 = block_word(c0, S, NEG), w1 = two ? block_word(c1, S, NEG) : 0u;
             uint32_t c = fadd(p[0], w0, w1);
 #pragma unroll
             for (int k = 1; k < PL; k++) {
@@ -145,26 +148,24 @@ __device__ __forceinline__ void count_blocks(const uint2 *cp, int32_t nb, uint32
     }
     fold<PL, 16>(p);
     fold<PL + 1, 8>(p);   // the low byte of each plane: PL + 2 planes, counts of at most 127
-    // bytes shifted up one plane (which doubles the counts), then an 8x8 bit
-    // transpose of (lo, hi)
-    lo = __byte_perm(__byte_perm(0u, p[0], 0x0040), __byte_perm(p[1], p[2], 0x0040), 0x5410);
-    hi = PL == 1 ? 0u
-                 : PL == 2 ? p[3] & 0xffu
-                           : __byte_perm(__byte_perm(p[3], p[4], 0x0040), __byte_perm(p[5], p[6], 0x0040), 0x5410);
-    uint32_t t;
-    t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
-    lo ^= t ^ (t << 7);
-    t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
-    lo ^= t ^ (t << 14);
-    if (PL > 1) {
-        t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
-        hi ^= t ^ (t << 7);
-        t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
-        hi ^= t ^ (t << 14);
+    const uint32_t lo = __byte_perm(__byte_perm(p[0], p[1], 0x0040), __byte_perm(p[2], p[3], 0x0040), 0x5410);
+    const uint32_t hi = __byte_perm(__byte_perm(p[4], p[5], 0x0040), p[6], 0x5410);
+#pragma unroll
+    for (int q = 0; q < KA; q += 2) {
+        float f[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const uint32_t m = 0x01010101u << (q + e);
+            uint32_t v = __dp4a(lo & m, 0x10080402u, 0x4b000000u);
+            if (PL > 2) v = __dp4a(hi & m, 0x00804020u, v);
+            f[e] = __uint_as_float(v);
+        }
+        const float a = 1.0f / (1 << q), b = 8388608.0f / (1 << q);
+        const float2 t = __ffma2_rn(make_float2(f[0], f[1]), make_float2(a, 0.5f * a),
+                                    __fadd2_rn(make_float2(negdeg, negdeg), make_float2(-b, -0.5f * b)));
+        tv[q] = t.x;
+        tv[q + 1] = t.y;
     }
-    t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
-    lo ^= t;
-    hi ^= t >> 4;
 }
 
 // The update of a row's agents; the new signs as a byte.
@@ -203,24 +204,11 @@ __device__ __forceinline__ void row_force(const RsP &P, int s, uint32_t S, float
     const int32_t b0 = __ldg(&P.off[sl]), nb = __ldg(&P.off[sl + 1]) - b0;   // warp-uniform
     const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
     if (MODE != RS_REAL) {
-        uint32_t lo = 0, hi = 0;
         constexpr bool neg = MODE == RS_PM1;
-        if (nb == 1) count_blocks<1>(cp, nb, S, neg, lo, hi);
-        else if (nb < 8) count_blocks<3>(cp, nb, S, neg, lo, hi);
-        else count_blocks<6>(cp, nb, S, neg, lo, hi);   // degree <= 127: at most 32 blocks
-        // PRMT builds the float 2^23 + 2 count; minus 2^23 + degree it is the
-        // force 2 count - degree, exactly
-        const float b = -(8388608.0f + (float)__ldg(&P.deg[min(s, P.n - 1)]));
-        const float2 bias = make_float2(b, b);
-#pragma unroll
-        for (int v = 0; v < KA; v += 2) {
-            const uint32_t w = v < 4 ? lo : hi;
-            const float2 f = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + (v & 3))),
-                                                    __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7441u + (v & 3)))),
-                                        bias);
-            tv[v] = f.x;
-            tv[v + 1] = f.y;
-        }
+        const float nd = -(float)__ldg(&P.deg[min(s, P.n - 1)]);
+        if (nb < 2) count_force<1, KA, neg>(cp, nb, S, nd, tv);
+        else if (nb < 8) count_force<3, KA, neg>(cp, nb, S, nd, tv);
+        else count_force<6, KA, neg>(cp, nb, S, nd, tv);   // degree <= 127: at most 32 blocks
     } else {
 #pragma unroll
         for (int v = 0; v < KA; v++) tv[v] = 0.0f;

@@ -124,7 +124,7 @@ template <class T, int V> __device__ __forceinline__ void vstore(T *p, const T (
     *(decltype(r.u) *)p = r.u;
 }
 
-// The two BF16 values of a word as FP32, by the mixed-precision addition of
+// The two BF16 (FP16) values of a word as FP32, by the mixed-precision addition of
 // -0 (exact, sign of zero kept): it runs on the FMA pipe at full rate, where a
 // shift and a mask take the ALU pipe at half rate (GB300: 114 against 59
 // lanes a cycle and SM), which bounds the 16-bit updates.
@@ -133,6 +133,16 @@ __device__ __forceinline__ float2 bf16_pair(uint32_t w)
     float2 f;
     asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\t"
         "add.rn.f32.bf16 %0, l, %3;\n\tadd.rn.f32.bf16 %1, h, %3;\n\t}"
+        : "=f"(f.x), "=f"(f.y)
+        : "r"(w), "f"(-0.0f));
+    return f;
+}
+
+__device__ __forceinline__ float2 f16_pair(uint32_t w)
+{
+    float2 f;
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\t"
+        "add.rn.f32.f16 %0, l, %3;\n\tadd.rn.f32.f16 %1, h, %3;\n\t}"
         : "=f"(f.x), "=f"(f.y)
         : "r"(w), "f"(-0.0f));
     return f;
@@ -153,7 +163,7 @@ __device__ __forceinline__ void to_vals(const Raw<V * sizeof(T)> &r, A (&o)[V])
                 o[2 * i] = f.x;
                 o[2 * i + 1] = f.y;
             } else {
-                const float2 f = __half22float2(*(const __half2 *)&w[i]);
+                const float2 f = f16_pair(w[i]);
                 o[2 * i] = f.x;
                 o[2 * i + 1] = f.y;
             }
@@ -615,6 +625,20 @@ __device__ __forceinline__ uint32_t sign_byte(uint32_t m0, uint32_t m1)
     return (uint32_t)__dp4a((int)m1, (int)0x80c0e0f0u, __dp4a((int)m0, (int)0xf8fcfeffu, 0));
 }
 
+// Signs of V packed 16-bit values, bit v the sign of value v.
+template <int V> __device__ __forceinline__ uint32_t sign_bits16(const uint32_t (&xw)[V / 2])
+{
+    if constexpr (V == 8) {
+        uint32_t m0, m1;
+        sign_masks(xw, m0, m1);
+        return sign_byte(m0, m1);
+    } else if constexpr (V == 4) {
+        return (uint32_t)__dp4a((int)prmt<0xfdb9>(xw[0], xw[1]), (int)0xf8fcfeffu, 0);
+    } else {
+        return ((xw[0] >> 15) & 1u) | ((xw[0] >> 30) & 2u);
+    }
+}
+
 // One SB step over every (row, agent).  Work item = (group of 32/LR rows,
 // segment of LR*V agents); lane l of a row owns V consecutive agents (one
 // vector load of x and of y).  Per neighbour j the lane reads the sign word
@@ -680,6 +704,17 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
     // new sign word written (and compared with the previous window's).
     auto finish = [&](int64_t r, int q, int off, int64_t base, bool live, const RawT &xr, const RawT &yr,
                       const A (&tv)[V], A c0, uint32_t wp_old) {
+        uint32_t b = 0;
+        RawT xw, yw;
+        if constexpr (sizeof(T) == 2 && V >= 2 && KIND != K_XY) {
+            uint32_t px[V / 2], py[V / 2];
+            memcpy(px, &xr.u, sizeof px);
+            memcpy(py, &yr.u, sizeof py);
+            sb_update16<T, KIND, WIN, V>(px, py, tv, c0, c, cn);
+            b = sign_bits16<V>(px);
+            memcpy(&xw.u, px, sizeof px);
+            memcpy(&yw.u, py, sizeof py);
+        } else {
         A x[V], y[V];
         to_vals<T, V>(xr, x);
         to_vals<T, V>(yr, y);
@@ -694,11 +729,11 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             sb_update<KIND, WIN, V>(x, y, tv, c0, c, cn);
         }
         // signs of the new x (rounding to the storage type keeps the sign)
-        uint32_t b = 0;
 #pragma unroll
         for (int v = 0; v < V; v++) b |= sbit(x[v]) << v;
-        const auto xw = from_vals<T, V>(x);
-        const auto yw = from_vals<T, V>(y);
+        xw = from_vals<T, V>(x);
+        yw = from_vals<T, V>(y);
+        }
         if (live) {
             vstore_s(xp + base, xw.u, cs);
             vstore_s(yp + base, yw.u, cs);
@@ -1164,24 +1199,39 @@ __global__ void __launch_bounds__(NT) k_iso(const StepP P, const int nsteps)
         const int64_t r = __ldg(&P.order[P.n - P.niso + i]);
         const int a0 = seg * V, q = a0 >> 5, off = a0 & 31;
         const int64_t base = r * P.Ap + a0;
-        A x[V], y[V];
+        A x[V], y[V];                            // wider types
+        uint32_t px[V / 2 + 1], py[V / 2 + 1];   // 16-bit types, packed
         RawT xw = vload_s<T, V>(xp + base, cs), yw = vload_s<T, V>(yp + base, cs);
-        to_vals<T, V>(xw, x);
-        to_vals<T, V>(yw, y);
+        uint32_t(&qx)[V / 2] = *(uint32_t(*)[V / 2])px, (&qy)[V / 2] = *(uint32_t(*)[V / 2])py;
+        if constexpr (sizeof(T) == 2) {
+            memcpy(px, &xw.u, sizeof xw.u);
+            memcpy(py, &yw.u, sizeof yw.u);
+        } else {
+            to_vals<T, V>(xw, x);
+            to_vals<T, V>(yw, y);
+        }
         A c0 = (A)P.c0;
         if (P.c0r32) c0 = std::is_same<A, double>::value ? (A)__ldg(&P.c0r64[r]) : (A)__ldg(&P.c0r32[r]);
         auto one = [&](int k) {
             const auto c = Coef<A>::get(P, step0 + k);
-            sb_update<K_FUSED, false, V>(x, y, zero, c0, c, c);
-            xw = from_vals<T, V>(x);
-            yw = from_vals<T, V>(y);
-            to_vals<T, V>(xw, x);
-            to_vals<T, V>(yw, y);
+            if constexpr (sizeof(T) == 2) {
+                sb_update16<T, K_FUSED, false, V>(qx, qy, zero, c0, c, c);
+            } else {
+                sb_update<K_FUSED, false, V>(x, y, zero, c0, c, c);
+                xw = from_vals<T, V>(x);
+                yw = from_vals<T, V>(y);
+                to_vals<T, V>(xw, x);
+                to_vals<T, V>(yw, y);
+            }
         };
         auto signs = [&]() {
             uint32_t b = 0;
+            if constexpr (sizeof(T) == 2) {
+                b = sign_bits16<V>(qx);
+            } else {
 #pragma unroll
-            for (int v = 0; v < V; v++) b |= sbit(x[v]) << v;
+                for (int v = 0; v < V; v++) b |= sbit(x[v]) << v;
+            }
             return b << off;
         };
         const int body = nsteps > 2 ? nsteps - 2 : 0;
@@ -1192,6 +1242,10 @@ __global__ void __launch_bounds__(NT) k_iso(const StepP P, const int nsteps)
             one(k);
             bprev = b;
             b = signs();
+        }
+        if constexpr (sizeof(T) == 2) {
+            memcpy(&xw.u, px, sizeof xw.u);
+            memcpy(&yw.u, py, sizeof yw.u);
         }
         if (nsteps > 0 && live) {
             vstore_s(xp + base, xw.u, cs);
