@@ -191,19 +191,10 @@ __device__ __forceinline__ void force8(const uint32_t (&p)[7], int h, float negd
     const uint32_t lo = __byte_perm(__byte_perm(p[0], p[1], s01), __byte_perm(p[2], p[3], s01), 0x5410);
     const uint32_t hi = __byte_perm(__byte_perm(p[4], p[5], s01), p[6] >> (8 * h), 0x5410);
 #pragma unroll
-    for (int q = 0; q < 8; q += 2) {
-        float f[2];
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const uint32_t m = 0x01010101u << (q + e);
-            const uint32_t v = __dp4a(lo & m, 0x10080402u, 0x4b000000u);
-            f[e] = __uint_as_float(__dp4a(hi & m, 0x00804020u, v));
-        }
-        const float a = 1.0f / (1 << q), b = 8388608.0f / (1 << q);
-        const float2 t = __ffma2_rn(make_float2(f[0], f[1]), make_float2(a, 0.5f * a),
-                                    __fadd2_rn(make_float2(negdeg, negdeg), make_float2(-b, -0.5f * b)));
-        tv[q] = t.x;
-        tv[q + 1] = t.y;
+    for (int q = 0; q < 8; q++) {
+        const uint32_t m = 0x01010101u << q;
+        const uint32_t v = __dp4a(hi & m, 0x00804020u, __dp4a(lo & m, 0x10080402u, 0x4b000000u));
+        tv[q] = fmaf(__uint_as_float(v), 1.0f / (1 << q), negdeg - 8388608.0f / (1 << q));
     }
 }
 
