@@ -1190,13 +1190,17 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
     if (blocks * 32 > INT32_MAX) return fail(ctx, SBX_ERR_UNSUPPORTED, "resident kernel: matrix too large");
     // one buffer: blocks' columns, blocks' weights, slice offsets, degrees
     const size_t bcol = (size_t)blocks * 32 * 8, bval = J.unit ? 0 : (size_t)blocks * 32 * 16;
-    const size_t boff = ((size_t)(nsl + 1) * 4 + 15) / 16 * 16, bdeg = (size_t)n * 4;
+    const size_t boff = ((size_t)nsl * 8 + 15) / 16 * 16, bdeg = (size_t)n * 4;
     std::vector<unsigned char> buf(bcol + bval + boff + bdeg, 0);
     uint16_t *col = (uint16_t *)buf.data();
     float *val = (float *)(buf.data() + bcol);
-    int32_t *ho = (int32_t *)(buf.data() + bcol + bval), *hd = (int32_t *)(buf.data() + bcol + bval + boff);
+    int32_t *ho = (int32_t *)(buf.data() + bcol + bval);
+    float *hd = (float *)(buf.data() + bcol + bval + boff);
     std::fill(col, col + blocks * 128, (uint16_t)(n * scale));
-    for (int64_t k = 0; k <= nsl; k++) ho[k] = (int32_t)off[(size_t)k];
+    for (int64_t k = 0; k < nsl; k++) {
+        ho[2 * k] = (int32_t)off[(size_t)k];
+        ho[2 * k + 1] = (int32_t)(off[(size_t)k + 1] - off[(size_t)k]);
+    }
     auto place = [&](int64_t k, std::vector<uint16_t> &ent) {
         const int64_t s0 = 32 * k, pos = 4 * (off[(size_t)k + 1] - off[(size_t)k]);
         const int rows = (int)std::min<int64_t>(32, n - s0);
@@ -1212,7 +1216,7 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
         }
         place_entries(ent.data(), pos, rows, left, 0x7fffu, col + off[(size_t)k] * 128);
     };
-    for (int64_t s = 0; s < n; s++) hd[s] = degree(s);
+    for (int64_t s = 0; s < n; s++) hd[s] = (float)degree(s);
     if (J.unit) {
         parallel(J.nnz > (1 << 16) ? std::min(host_threads(), 8) : 1, [&](int t, int TT) {
             std::vector<uint16_t> ent;
@@ -1221,7 +1225,7 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
     } else {
         for (int64_t s = 0; s < n; s++) {
             const size_t r = (size_t)J.hperm[(size_t)s];
-            for (int32_t j = 0; j < hd[s]; j++) {
+            for (int32_t j = 0; j < degree(s); j++) {
                 const size_t e = (size_t)J.hrowptr[r] + (size_t)j;
                 const size_t at = ((size_t)(off[(size_t)(s / 32)] + j / 4) * 32 + (size_t)(s & 31)) * 4 + (size_t)(j & 3);
                 col[at] = (uint16_t)(inv[(size_t)J.hcol[e]] * scale);
@@ -1235,8 +1239,8 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
     CK(cudaMemcpy(dev, buf.data(), buf.size(), cudaMemcpyHostToDevice));
     L.col = (const uint2 *)dev;
     L.val = J.unit ? nullptr : (const float4 *)(dev + bcol);
-    L.off = (const int32_t *)(dev + bcol + bval);
-    L.deg = (const int32_t *)(dev + bcol + bval + boff);
+    L.off = (const int2 *)(dev + bcol + bval);
+    L.deg = (const float *)(dev + bcol + bval + boff);
     return SBX_OK;
 }
 

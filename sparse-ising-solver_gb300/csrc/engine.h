@@ -54,8 +54,8 @@ struct DevBsm;
 // of other matrices, zero past a row's end.
 struct DevSell {
     void *base = nullptr;              // one allocation holding the arrays below
-    const int32_t *off = nullptr;      // [slices + 1] first block of each slice
-    const int32_t *deg = nullptr;      // [n] entries of each slot
+    const int2 *off = nullptr;         // per slice: first block, blocks
+    const float *deg = nullptr;        // per slot: entries
     const uint2 *col = nullptr;        // [blocks][32]
     const float4 *val = nullptr;       // [blocks][32], null for +-1 weights
 };

@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(1024) k_resident(const ResP P)
 
 struct Res8P {
     ResP r;
-    const int32_t *__restrict__ off;   // sliced matrix (engine.h, DevSell)
-    const int32_t *__restrict__ deg;
+    const int2 *__restrict__ off;      // sliced matrix (engine.h, DevSell)
+    const float *__restrict__ deg;
     const uint2 *__restrict__ col;
     const float4 *__restrict__ val;
     int32_t allpos;
@@ -387,11 +387,11 @@ __device__ __forceinline__ void count8_blocks(const uint2 *cp, int32_t nb, uint3
 
 // Totals from byte counters of `m` entries (at most 120): PRMT builds the
 // float 2^23 + 2 * count; minus 2^23 + m it is 2 * count - m, exactly.
-__device__ __forceinline__ void totals8(uint32_t lo, uint32_t hi, int32_t m, float (&tv)[8])
+__device__ __forceinline__ void totals8(uint32_t lo, uint32_t hi, float m, float (&tv)[8])
 {
     lo += lo;
     hi += hi;
-    const float b = -(8388608.0f + (float)m);
+    const float b = -8388608.0f - m;
     const float2 bias = make_float2(b, b);
 #pragma unroll
     for (int q = 0; q < 8; q += 2) {
@@ -409,8 +409,9 @@ template <bool NEG>
 __device__ __forceinline__ void count8(const Res8P &P, int s, uint32_t S, float (&tv)[8])
 {
     const int sl = s >> 5, lane = s & 31;
-    const int32_t b0 = __ldg(&P.off[sl]), nb = __ldg(&P.off[sl + 1]) - b0;   // warp-uniform
-    const int32_t deg = __ldg(&P.deg[s]);
+    const int2 o = __ldg(&P.off[sl]);   // warp-uniform
+    const int32_t b0 = o.x, nb = o.y;
+    const float deg = __ldg(&P.deg[s]);
     const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
 #pragma unroll
     for (int q = 0; q < 8; q++) tv[q] = 0.f;
@@ -419,7 +420,7 @@ __device__ __forceinline__ void count8(const Res8P &P, int s, uint32_t S, float 
         float t[8];
         uint32_t lo = 0, hi = 0;
         count8_blocks<NEG>(cp + c0 * 32, min(nb - c0, 30), S, lo, hi);
-        totals8(lo, hi, max(0, min(deg - 4 * c0, 120)), t);
+        totals8(lo, hi, fmaxf(0.f, fminf(deg - (float)(4 * c0), 120.f)), t);
 #pragma unroll
         for (int q = 0; q < 8; q++) tv[q] += t[q];
     }
@@ -429,7 +430,8 @@ __device__ __forceinline__ void count8(const Res8P &P, int s, uint32_t S, float 
 __device__ __forceinline__ void sum8(const Res8P &P, int s, uint32_t S, float (&tv)[8])
 {
     const int sl = s >> 5, lane = s & 31;
-    const int32_t b0 = __ldg(&P.off[sl]), nb = __ldg(&P.off[sl + 1]) - b0;   // warp-uniform
+    const int2 o2 = __ldg(&P.off[sl]);   // warp-uniform
+    const int32_t b0 = o2.x, nb = o2.y;
     const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
     const float4 *vp = P.val + (int64_t)b0 * 32 + lane;
     float2 t[4];

@@ -32,8 +32,8 @@ namespace sbx {
 namespace {
 
 struct RsP {
-    const int32_t *__restrict__ off;    // sliced matrix (engine.h, DevSell)
-    const int32_t *__restrict__ deg;
+    const int2 *__restrict__ off;       // sliced matrix (engine.h, DevSell)
+    const float *__restrict__ deg;
     const uint2 *__restrict__ col;
     const float4 *__restrict__ val;
     const int32_t *__restrict__ perm;   // slot -> row
@@ -192,11 +192,12 @@ __device__ __forceinline__ void row_force(const RsP &P, int s, uint32_t S, float
 {
     constexpr int KA = kAgents<T>;
     const int sl = s >> 5, lane = s & 31;
-    const int32_t b0 = __ldg(&P.off[sl]), nb = __ldg(&P.off[sl + 1]) - b0;   // warp-uniform
+    const int2 o2 = __ldg(&P.off[sl]);   // warp-uniform
+    const int32_t b0 = o2.x, nb = o2.y;
     const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
     if (MODE != RS_REAL) {
         constexpr bool neg = MODE == RS_PM1;
-        const float nd = -(float)__ldg(&P.deg[min(s, P.n - 1)]);
+        const float nd = -__ldg(&P.deg[min(s, P.n - 1)]);
         if (nb < 2) count_force<1, KA, neg>(cp, nb, S, nd, tv);
         else if (nb < 8) count_force<3, KA, neg>(cp, nb, S, nd, tv);
         else count_force<6, KA, neg>(cp, nb, S, nd, tv);   // degree <= 127: at most 32 blocks
@@ -346,21 +347,35 @@ __global__ void __launch_bounds__(kNT, 1) k_resident_rs(const RsP P)
         const bool win = ((k + 1) % P.period) == 0;
         const float4 ck = P.coef[k];
         uint32_t chg = 0;
-        for (int i = 0; i * NT + w0 < n; i++) {
+        // the signs of row s, new and in window steps against the last window's
+        auto put_sign = [&](int s, uint32_t nb) {
+            Snx[s] = (uint8_t)nb;
+            if (win) {
+                chg |= nb ^ Wb[s];
+                Wb[s] = (uint8_t)nb;
+            }
+        };
+        // rows in tensor memory (whole warps: a lane past the rows steps what
+        // lies there and keeps nothing), then the others
+        const int nt = min(kTmRows, (n - w0 + NT - 1) / NT);
+        for (int i = 0; i < nt; i++) {
             const int s = i * NT + tid;
             float tv[8];
             row_force<T, MODE>(P, s, Sin, tv);
-            uint4 xv = make_uint4(0, 0, 0, 0), yv = xv;
-            get_row(i, s, xv, yv);
+            uint4 xv, yv;
+            tm_ld(tw + 8u * (uint32_t)i, xv, yv);
             const uint32_t nb = update_row<T>(xv, yv, tv, P.c0, ck);
-            put_row(i, s, xv, yv);
-            if (s < n) {
-                Snx[s] = (uint8_t)nb;
-                if (win) {
-                    chg |= nb ^ Wb[s];
-                    Wb[s] = (uint8_t)nb;
-                }
-            }
+            tm_st(tw + 8u * (uint32_t)i, xv, yv);
+            if (s < n) put_sign(s, nb);
+        }
+        for (int s = kTmRows * NT + tid; s < n; s += NT) {
+            float tv[8];
+            row_force<T, MODE>(P, s, Sin, tv);
+            uint4 xv = xs[s - kTmRows * NT], yv = ys[s - kTmRows * NT];
+            const uint32_t nb = update_row<T>(xv, yv, tv, P.c0, ck);
+            xs[s - kTmRows * NT] = xv;
+            ys[s - kTmRows * NT] = yv;
+            put_sign(s, nb);
         }
         tm_wait_st();
         if (win) {
