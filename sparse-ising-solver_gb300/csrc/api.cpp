@@ -54,7 +54,7 @@ struct BatchClass {
     DevRb rb;                             // packed for the resident batch kernel (on first use)
     int64_t rb_max = 0;                   // bin capacity the packing was made for
     DevBsm bsm;                           // plan of the shared-memory-plane step (on first use)
-    DevBres bres;                         // packed for the on-chip batch kernel (on first use)
+    DevBres bres[2];                      // packed for the on-chip batch kernel, 16-bit and FP32 state (on first use)
     std::vector<int32_t> agent_off;       // instance i's cuts at [agent_off[i], agent_off[i + 1])
     int32_t *daoff = nullptr;             // the same on the device
     // Each instance's rows are renumbered by decreasing degree inside its
@@ -1296,17 +1296,18 @@ void free_bres(DevBres &B)
 // Pack a class for the on-chip batch kernel; leaves bres.rows null when an
 // instance does not fit or stepping launch by launch is faster.  A bin's cluster is the smallest that holds it and,
 // when the class alone cannot fill the GPU, splits it down to an SM's share.
-int build_bres(sbx_ctx *ctx, BatchClass &c)
+int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32)
 {
-    DevBres &B = c.bres;
+    DevBres &B = c.bres[f32];
     free_bres(B);
     B.tried = true;
     const DevCsr &J = c.J;
     const size_t ni = c.probs.size();
     int64_t cap[4];
-    for (int k = 0; k < 4; k++) cap[k] = batch_res_rows(k);
+    for (int k = 0; k < 4; k++) cap[k] = batch_res_rows(k, f32);
     const int nsm = std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
-    const int64_t share = std::max<int64_t>(512, J.n * (c.Ap / 16) / nsm);   // rows a CTA would hold in one even wave
+    const int groups = c.Ap / (f32 ? 8 : 16);
+    const int64_t share = std::max<int64_t>(512, J.n * groups / nsm);   // rows a CTA would hold in one even wave
     std::vector<size_t> ord(ni);
     std::iota(ord.begin(), ord.end(), 0);
     std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return c.probs[a]->J.n > c.probs[b]->J.n; });
@@ -1342,20 +1343,22 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
     // Taken where its step is the shorter one (microseconds, both sides fitted
     // on GB300 on 1 to 512 instances of 100 to 20,000 rows at 32, 64 and 128
     // agents): a cluster's step is about 2 + 0.085 per slice of its CTAs at
-    // degree 24, and the step per launch about 6 + 0.06 per thousand rows and
-    // 32 agents.  One instance of 19,909 rows at 64 agents: 15.5 against 7.5;
-    // 32 instances, 154,000 rows: 16.6 against 22.7.
+    // degree 24 (FP32, half the agents: 0.06), and the step per launch about 6 +
+    // 0.06 per thousand rows and 32 agents (FP32: 4 + 0.11).  One instance of
+    // 19,909 rows at 64 agents, 16 bits: 15.5 against 7.5; 32 instances, 154,000
+    // rows: 16.6 against 22.7, FP32 22.5 against 40.2.
     double sum = 0, longest = 0;
     for (const Bin &b : bins) {
         const int C = batch_res_ctas(b.k);
         int64_t nnz = 0;
         for (int32_t i : b.inst) nnz += c.probs[(size_t)i]->J.nnz;
         const double deg = (double)nnz / (double)b.rows;
-        const double t = 2.0 + 0.085 * (double)(((b.rows + 31) / 32 + C - 1) / C) * (0.4 + 0.6 * deg / 24);
-        sum += t * C * (c.Ap / 16) / nsm;
+        const double t = 2.0 + (f32 ? 0.060 : 0.085) * (double)(((b.rows + 31) / 32 + C - 1) / C) * (0.4 + 0.6 * deg / 24);
+        sum += t * C * groups / nsm;
         longest = std::max(longest, t);
     }
-    if (std::max(longest, 1.1 * sum) > 6.0 + 0.06e-3 * (double)J.n * (c.Ap / 32)) return SBX_OK;
+    if (std::max(longest, 1.1 * sum) > (f32 ? 4.0 : 6.0) + (f32 ? 0.11e-3 : 0.06e-3) * (double)J.n * (c.Ap / 32))
+        return SBX_OK;
     std::stable_sort(bins.begin(), bins.end(),
                      [](const Bin &a, const Bin &b) { return a.k != b.k ? a.k < b.k : a.rows > b.rows; });
     const size_t nb = bins.size();
@@ -1413,7 +1416,7 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
         for (size_t b = (size_t)t; b < nb; b += (size_t)TT) {
             for (int64_t s = 0; s < rows[b]; s++) inv[(size_t)perm[(size_t)(slot0[b] + s)]] = (int32_t)s;
             std::fill(col.begin() + (long)(first[b] * 128), col.begin() + (long)((first[b] + blocks[b]) * 128),
-                      (uint16_t)batch_res_entry(bins[b].k, J.allpos, (uint32_t)rows[b], false));
+                      (uint16_t)batch_res_entry(bins[b].k, f32, J.allpos, (uint32_t)rows[b], false));
             int32_t *o = &off[(size_t)slice0[b]];
             uint16_t ent[32 * 128];   // degree <= 127: at most 128 positions
             int32_t left[32];
@@ -1425,7 +1428,7 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
                     left[l] = J.hrowptr[r + 1] - J.hrowptr[r];
                     uint16_t *v = ent + l * pos;
                     for (int32_t e = J.hrowptr[r]; e < J.hrowptr[r + 1]; e++)
-                        *v++ = (uint16_t)batch_res_entry(bins[b].k, J.allpos, (uint32_t)inv[(size_t)J.hcol[(size_t)e]],
+                        *v++ = (uint16_t)batch_res_entry(bins[b].k, f32, J.allpos, (uint32_t)inv[(size_t)J.hcol[(size_t)e]],
                                                          J.hval[(size_t)e] < 0);
                 }
                 place_entries(ent, pos, m, left, 0xffffu, &col[(size_t)(first[b] + o[k]) * 128]);
@@ -1449,9 +1452,8 @@ int build_bres(sbx_ctx *ctx, BatchClass &c)
 }
 
 // dt * xi0 of each slot's instance, and minus its degree.
-int upload_bres_cb(sbx_ctx *ctx, BatchClass &c, double dt)
+int upload_bres_cb(sbx_ctx *ctx, BatchClass &c, DevBres &B, double dt)
 {
-    DevBres &B = c.bres;
     if (B.dt == dt) return SBX_OK;
     std::vector<float> cb(2 * B.hinst.size());
     for (size_t s = 0; s < B.hinst.size(); s++) {
@@ -1683,7 +1685,7 @@ void free_batch(sbx_ctx *ctx)
         free_csr(c.J);
         free_rb(c.rb);
         free_bsm(c.bsm);
-        free_bres(c.bres);
+        for (DevBres &B : c.bres) free_bres(B);
         cudaFree(c.daoff);
         cudaFree(c.dslot);
     }
@@ -1814,17 +1816,18 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
                         "32/64/128 agents and instances whose plane fits in shared memory");
         const bool use_bsm = bsm_fit && !tile_pinned && pr->kernel != SBX_KERNEL_RESIDENT &&
                              pr->kernel != SBX_KERNEL_RESIDENT_SPLIT;
-        // the on-chip batch kernel: +-1 fused 16-bit classes whose instances
+        // the on-chip batch kernel: +-1 fused classes (not FP64) whose instances
         // fit a cluster, unless a tile, a count mode or a kernel is asked for
         // (256 tori of 947,961 rows in all at 64 agents: 52 us a step, the
         // resident batch 94, the plane kernel 97)
         const bool by_itself = pr->kernel == SBX_KERNEL_AUTO;
+        DevBres &bres = c.bres[d.prec == P_F32];
         bool use_res = (!use_rb || by_itself) && !tile_pinned && !bsm_threads && !pr->count_mode && pr->kernel == SBX_KERNEL_AUTO &&
-                       (d.prec == P_BF16 || d.prec == P_F16) && d.fused && !d.trace && nchunks > 0 && c.J.unit &&
+                       d.prec != P_F64 && d.fused && !d.trace && nchunks > 0 && c.J.unit &&
                        c.J.max_deg <= kHeavy;
         if (use_res) {
-            if (!c.bres.tried && (rc = build_bres(ctx, c))) return rc;
-            use_res = c.bres.rows != nullptr;
+            if (!bres.tried && (rc = build_bres(ctx, c, d.prec == P_F32))) return rc;
+            use_res = bres.rows != nullptr;
             if (use_res) use_rb = false;
         }
         // ... else the plane kernel before the resident batch, which it also
@@ -1832,7 +1835,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         if (use_rb && by_itself && !tile_pinned && bsm_ok(c, d)) use_rb = false;
         c.J.bsm = nullptr;
         if (use_res) {
-            if ((rc = upload_bres_cb(ctx, c, pr->dt))) return rc;
+            if ((rc = upload_bres_cb(ctx, c, bres, pr->dt))) return rc;
             for (int k = 0; k < 4; k++) {
                 if (!ctx->side[k]) CK(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
                 if (!ctx->join[k]) CK(cudaEventCreateWithFlags(&ctx->join[k], cudaEventDisableTiming));
@@ -1859,7 +1862,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         CK(cudaEventRecord(ctx->ev0, s));
         if (use_res) {
             d.steps_run = (int32_t)total;
-            const cudaError_t e = launch_batch_res(d, c.bres, c.J.allpos, *std::max_element(c.agents.begin(), c.agents.end()),
+            const cudaError_t e = launch_batch_res(d, bres, c.J.allpos, *std::max_element(c.agents.begin(), c.agents.end()),
                                                    ctx->w, s, ctx->side, ctx->fork, ctx->join, &launches);
             if (e != cudaSuccess)   // what was launched ends before the buffers are used again
                 for (cudaStream_t t : ctx->side) cudaStreamSynchronize(t);
@@ -1914,7 +1917,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             r->time_to_target_us = -1;
             r->steps_to_target = -1;
             if (use_res) {
-                r->lane_agents = 16;
+                r->lane_agents = d.prec == P_F32 ? 8 : 16;
                 r->row_lanes = 1;
                 r->block_threads = 1024;
                 r->count_mode = 4;
@@ -1945,7 +1948,7 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             r->steps_run = total;
             r->windows_run = nchunks;
             r->kernel_used = use_rb || (use_res && low_degree) ? SBX_KERNEL_RESIDENT : SBX_KERNEL_STREAM;
-            r->agents_per_block = use_rb ? 4 : use_res ? 16 : 0;
+            r->agents_per_block = use_rb ? 4 : use_res ? (d.prec == P_F32 ? 8 : 16) : 0;
             r->kernel_launches = launches;
             r->kernel_ms = use_rb || use_res ? (profile ? ms : 0.0) : kms;
             r->gpu_launches = launches + 4;

@@ -187,7 +187,8 @@ struct DevBsm {
     int64_t max_rows = 0;         // largest instance: the shared-memory plane's rows
 };
 
-// A batch class packed for the on-chip batch kernel (k_batch_res.cu): whole
+// A batch class packed for the on-chip batch kernel (k_batch_res.cu), 16-bit or
+// FP32 state: whole
 // instances in bins, a bin's rows by decreasing degree ("slots") in slices of
 // 32 (as DevSell); the bins listed by kind -- clusters of 1, 2 and 4 CTAs, and
 // of 4 for bins past 16,383 rows -- each largest first.
@@ -287,8 +288,8 @@ cudaError_t launch_resident_batch(const SolveDims &d, const DevRb &B, Work &w, c
 // launch runs all d.steps_run fused steps of every bin, the kinds on the side
 // streams between fork and join.  agents: the class's largest count.
 int batch_res_ctas(int kind);
-int64_t batch_res_rows(int kind);
-uint32_t batch_res_entry(int kind, bool allpos, uint32_t slot, bool neg);
+int64_t batch_res_rows(int kind, bool f32);
+uint32_t batch_res_entry(int kind, bool f32, bool allpos, uint32_t slot, bool neg);
 cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, int32_t agents, Work &w,
                              cudaStream_t s, cudaStream_t *side, cudaEvent_t fork, cudaEvent_t *join,
                              int *launches);

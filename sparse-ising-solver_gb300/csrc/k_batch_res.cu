@@ -3,7 +3,8 @@
 // its own), and a cluster of C = 1, 2 or 4 CTAs owns 16 agents of every row of
 // one bin from the first step to the last.  Instances never interact and
 // neither do agents, so a cluster needs no other.  +-1 weights, degree <= 127,
-// 16-bit state, fused steps; the arithmetic is the streaming kernel's (exact
+// fused steps, 16-bit or FP32 state (FP32: 8 agents for 16 in all of this, a
+// row's signs in a byte, four neighbours to a word); the arithmetic is the streaming kernel's (exact
 // force, sb_update's roundings), so the results are identical.
 //
 // A step launched per kernel (k_bsm) reads and writes the whole state each
@@ -56,19 +57,29 @@ struct BresP {
     uint32_t smem;                       // bytes of dynamic shared memory
 };
 
+// agents of a cluster: 64 bytes of x and y a row
+template <class T> constexpr int kAgents = sizeof(T) == 4 ? 8 : 16;
+
 // Shared memory: the sign planes at kPlane and 2 kPlane of the CTA's shared
 // window, the rows past tensor memory's in chunks of 32 (a warp's, [4 pieces of
 // 16 bytes][32]) before (from kFirst), between and after them.
 constexpr uint32_t kPlane = 0x10000, kChunk = 2048, kFirst = 0x800;
-// Sign planes of all +1 or +-1 weights as 16-bit words (the sign in bit 0 of
-// an entry), or words with their complement.
+// Sign planes of all +1 or +-1 weights as words (the sign in bit 0 of an
+// entry), or words with their complement (the only ones of FP32 state).
 enum { BR_POS = 0, BR_BIT = 1, BR_DUAL = 2 };
-template <int MODE> constexpr uint32_t kRowB = MODE == BR_DUAL ? 4 : 2;   // bytes of a row's signs
+// bytes of a row's signs
+template <class T, int MODE> constexpr uint32_t kRowB = kAgents<T> / 8 * (MODE == BR_DUAL ? 2 : 1);
 
 struct Row16 {
-    uint32_t x[8], y[8];   // packed pairs of 16 agents
+    uint32_t x[8], y[8];   // packed pairs of 16 agents, or FP32 of 8
 };
 
+__device__ __forceinline__ uint32_t lds8(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
 __device__ __forceinline__ uint32_t lds16(uint32_t a)
 {
     uint32_t v;
@@ -131,6 +142,58 @@ template <int MODE> __device__ __forceinline__ void block_words(const uint2 &c, 
         w0 ^= (c.x & 0x00010001u) * 0xffffu;
         w1 ^= (c.y & 0x00010001u) * 0xffffu;
     }
+}
+
+// FP32 state: a block's four neighbour bytes as one word.
+__device__ __forceinline__ uint32_t block_word8(const uint2 &c, uint32_t S)
+{
+    const uint32_t b0 = lds8(__byte_perm(c.x, S, 0x7610)), b1 = lds8(__byte_perm(c.x, S, 0x7632));
+    const uint32_t b2 = lds8(__byte_perm(c.y, S, 0x7610)), b3 = lds8(__byte_perm(c.y, S, 0x7632));
+    return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
+}
+
+// The same counts for it: the nb entries of a byte lane in PL planes (nb <
+// 2^PL), the lanes summed; the low byte of each plane counts.
+template <int PL>
+__device__ __forceinline__ void count_blocks8(const uint2 *cp, int32_t nb, uint32_t S, uint32_t (&p)[7])
+{
+    uint32_t q[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) q[k] = 0;
+    uint2 n0 = make_uint2(0, 0), n1 = n0;
+    if (nb > 0) n0 = __ldg(cp);
+    if (nb > 1) n1 = __ldg(cp + 32);
+    for (int32_t b = 0; b < nb; b += 2) {
+        const uint2 c0 = n0, c1 = n1;
+        const bool two = b + 1 < nb;   // warp-uniform
+        if (b + 2 < nb) n0 = __ldg(cp + (b + 2) * 32);
+        if (b + 3 < nb) n1 = __ldg(cp + (b + 3) * 32);
+        const uint32_t w0 = block_word8(c0, S), w1 = two ? block_word8(c1, S) : 0u;
+        uint32_t c = fadd(q[0], w0, w1);
+#pragma unroll
+        for (int k = 1; k < PL; k++) {
+            const uint32_t t = q[k] & c;
+            q[k] ^= c;
+            c = t;
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < 2; f++) {   // 32 -> 16 -> 8 bits, a plane more each
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < PL + f; k++) {
+            const uint32_t b = q[k] >> (16 >> f);
+            if (k == 0) {
+                c = q[0] & b;
+                q[0] ^= b;
+            } else {
+                c = fadd(q[k], b, c);
+            }
+        }
+        q[PL + f] = c;
+    }
+#pragma unroll
+    for (int k = 0; k < 7; k++) p[k] = q[k];   // degree <= 127: seven planes
 }
 
 // Counts of the neighbours whose term is -1 over nb blocks as bit planes: bit
@@ -201,20 +264,22 @@ __device__ __forceinline__ void force8(const uint32_t (&p)[7], int h, float negd
 template <class T, int C, int MODE>
 __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
 {
-    static_assert(sizeof(T) == 2, "16-bit state: 16 agents in 32 bytes");
+    constexpr int KA = kAgents<T>;
+    constexpr uint32_t RB = kRowB<T, MODE>;
+    static_assert(sizeof(T) == 2 || MODE == BR_DUAL, "FP32 state: words with their complement");
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = C == 1 ? 0 : (int)(blockIdx.x % C);
     const int unit = blockIdx.x / C;
     const int bin = __ldg(&P.bins[unit / P.groups]);
-    const int a0 = (unit % P.groups) * 16;
+    const int a0 = (unit % P.groups) * KA;
     const int R = __ldg(&P.rows[bin]), sl0 = __ldg(&P.slice0[bin]), s0 = __ldg(&P.slot0[bin]);
     const int nsl = (R + 31) / 32, mine = (nsl - rank + C - 1) / C;   // the bin's slices, this CTA's
     // A CTA's window of the shared address space starts at a multiple of 16 MB
     // (its rank in the cluster); below, offsets in the window.
     const uint32_t sb = smem_u32(smem), win = sb & 0xff000000u, so = sb - win;
-    const uint32_t pb = ((uint32_t)(R + 1) * kRowB<MODE> + 15) & ~15u;   // bytes of a sign plane
+    const uint32_t pb = ((uint32_t)(R + 1) * RB + 15) & ~15u;   // bytes of a sign plane
     // chunks before, between and after the planes
     const uint32_t q0 = (kPlane - kFirst) / kChunk, q1 = (kPlane - pb) / kChunk, q2 = (P.smem - 2 * kPlane - pb) / kChunk;
     // Never expected, the host leaves room: the layout does not fit.  The
@@ -247,8 +312,9 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {   // the zero row that padded entries read
-        st_sign<kRowB<MODE>, false>(win + kPlane + kRowB<MODE> * (uint32_t)R, 0xffff0000u);
-        st_sign<kRowB<MODE>, false>(win + 2 * kPlane + kRowB<MODE> * (uint32_t)R, 0xffff0000u);
+        const uint32_t z = MODE == BR_DUAL ? ~0u << KA : 0u;
+        st_sign<RB, false>(win + kPlane + RB * (uint32_t)R, z);
+        st_sign<RB, false>(win + 2 * kPlane + RB * (uint32_t)R, z);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     step_barrier<C>();   // the cluster's CTAs are running: their shared memory may be written
@@ -295,17 +361,25 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
 #pragma unroll
     for (int c = 0; c < C; c++) pk[c] = C == 1 ? win : peer(sb, (uint32_t)c) - so;
     auto put_sign = [&](uint32_t plane, int s, uint32_t w) {
-        const uint32_t v = MODE == BR_DUAL ? w | (~w << 16) : w, a = plane + kRowB<MODE> * (uint32_t)s;
+        const uint32_t v = MODE == BR_DUAL ? w | (~w << KA) : w, a = plane + RB * (uint32_t)s;
 #pragma unroll
-        for (int c = 0; c < C; c++) st_sign<kRowB<MODE>, (C > 1)>(pk[c] + a, v);
+        for (int c = 0; c < C; c++) st_sign<RB, (C > 1)>(pk[c] + a, v);
     };
-    // signs of a row's 16 agents, agent j in bit j
+    // signs of a row's agents, agent j in bit j
     auto sign_word = [&](const Row16 &v) {
+        if constexpr (sizeof(T) == 4) {
+            float x[8];
+            memcpy(x, v.x, 32);
+            uint32_t m0, m1;
+            sign_masks(x, m0, m1);
+            return sign_byte(m0, m1);
+        } else {
         const uint32_t h0[4] = {v.x[0], v.x[1], v.x[2], v.x[3]}, h1[4] = {v.x[4], v.x[5], v.x[6], v.x[7]};
         uint32_t m0, m1, m2, m3;
         sign_masks(h0, m0, m1);
         sign_masks(h1, m2, m3);
         return sign_byte(m0, m1) | (sign_byte(m2, m3) << 8);
+        }
     };
 
     // The state after the pre-step Update_XY of step 0 (src/ising.cu:188),
@@ -316,24 +390,25 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
         Row16 v = {};
         if (s < R) {
             const int64_t g = (int64_t)__ldg(&P.perm[s0 + s]) * P.Ap + a0;
+            const uint4 xl = ((const uint4 *)(xg + g))[0], xh = ((const uint4 *)(xg + g))[1];
+            const uint4 yl = ((const uint4 *)(yg + g))[0], yh = ((const uint4 *)(yg + g))[1];
+            memcpy(v.x, &xl, 16);
+            memcpy(v.x + 4, &xh, 16);
+            memcpy(v.y, &yl, 16);
+            memcpy(v.y + 4, &yh, 16);
+            T x[KA], y[KA];
+            memcpy(x, v.x, 32);
+            memcpy(y, v.y, 32);
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                Raw<16> xr, yr;
-                float x[8], y[8];
-                xr.u = *(const uint4 *)(xg + g + 8 * h);
-                yr.u = *(const uint4 *)(yg + g + 8 * h);
-                to_vals<T, 8>(xr, x);
-                to_vals<T, 8>(yr, y);
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    y[q] = fmaf(c00.w, x[q], y[q]);
-                    x[q] = fmaf(c00.z, y[q], x[q]);
-                }
-                xr = from_vals<T, 8>(x);
-                yr = from_vals<T, 8>(y);
-                memcpy(&v.x[4 * h], &xr.u, 16);
-                memcpy(&v.y[4 * h], &yr.u, 16);
+            for (int q = 0; q < KA; q++) {
+                float a = St<T>::ld(x[q]), b = St<T>::ld(y[q]);
+                b = fmaf(c00.w, a, b);
+                a = fmaf(c00.z, b, a);
+                x[q] = St<T>::st(a);
+                y[q] = St<T>::st(b);
             }
+            memcpy(v.x, x, 32);
+            memcpy(v.y, y, 32);
             put_sign(kPlane, s, sign_word(v));   // step 0 reads the first plane
         }
         put_row(i, v);
@@ -351,9 +426,21 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
             const uint2 *cp = P.col + (int64_t)b0 * 32 + lane;
             const float2 cb = __ldg(&P.cb[s0 + min(s, R - 1)]);
             uint32_t p[7];
-            if (nb < 8) count_blocks<4, MODE>(cp, nb, Sin, p);
-            else count_blocks<7, MODE>(cp, nb, Sin, p);   // degree <= 127: at most 32 blocks
             Row16 v;
+            if constexpr (sizeof(T) == 4) {
+                if (nb < 8) count_blocks8<3>(cp, nb, Sin, p);
+                else count_blocks8<6>(cp, nb, Sin, p);   // degree <= 127: at most 32 blocks
+                get_row(i, v);
+                float tv[8], x[8], y[8];
+                force8(p, 0, cb.y, tv);
+                memcpy(x, v.x, 32);
+                memcpy(y, v.y, 32);
+                sb_update<K_FUSED, false, 8>(x, y, tv, cb.x, ck, ck);
+                memcpy(v.x, x, 32);
+                memcpy(v.y, y, 32);
+            } else {
+            if (nb < 8) count_blocks<4, MODE>(cp, nb, Sin, p);
+            else count_blocks<7, MODE>(cp, nb, Sin, p);
             get_row(i, v);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -372,6 +459,7 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
                     v.y[4 * h + q] = y[q];
                 }
             }
+            }
             put_row(i, v);
             if (live) put_sign(Snx, s, sign_word(v));
         }
@@ -388,10 +476,11 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
             const int64_t r = __ldg(&P.perm[s0 + s]), g = r * P.Ap + a0;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                *(uint4 *)(xg + g + 8 * h) = make_uint4(v.x[4 * h], v.x[4 * h + 1], v.x[4 * h + 2], v.x[4 * h + 3]);
-                *(uint4 *)(yg + g + 8 * h) = make_uint4(v.y[4 * h], v.y[4 * h + 1], v.y[4 * h + 2], v.y[4 * h + 3]);
+                ((uint4 *)(xg + g))[h] = make_uint4(v.x[4 * h], v.x[4 * h + 1], v.x[4 * h + 2], v.x[4 * h + 3]);
+                ((uint4 *)(yg + g))[h] = make_uint4(v.y[4 * h], v.y[4 * h + 1], v.y[4 * h + 2], v.y[4 * h + 3]);
             }
-            ((uint16_t *)P.Wp)[r * P.W * 2 + a0 / 16] = (uint16_t)sign_word(v);
+            if (KA == 16) ((uint16_t *)P.Wp)[r * P.W * 2 + a0 / 16] = (uint16_t)sign_word(v);
+            else ((uint8_t *)P.Wp)[r * P.W * 4 + a0 / 8] = (uint8_t)sign_word(v);
         }
     }
     if (blockIdx.x == 0 && tid == 0) {
@@ -440,6 +529,13 @@ cudaError_t launch_m(const BresP &P, int units, cudaStream_t s)
 template <class T>
 cudaError_t launch_t(const BresP &P, int c, bool allpos, int units, cudaStream_t s)
 {
+    if constexpr (sizeof(T) == 4) {
+        switch (c) {
+        case 0: return launch_m<T, 1, BR_DUAL>(P, units, s);
+        case 1: return launch_m<T, 2, BR_DUAL>(P, units, s);
+        default: return launch_m<T, 4, BR_DUAL>(P, units, s);
+        }
+    } else
     switch (c) {
     case 0: return allpos ? launch_m<T, 1, BR_POS>(P, units, s) : launch_m<T, 1, BR_DUAL>(P, units, s);
     case 1: return allpos ? launch_m<T, 2, BR_POS>(P, units, s) : launch_m<T, 2, BR_DUAL>(P, units, s);
@@ -452,22 +548,23 @@ cudaError_t launch_t(const BresP &P, int c, bool allpos, int units, cudaStream_t
 
 int batch_res_ctas(int c) { return c == 3 ? 4 : 1 << c; }
 
-int64_t batch_res_rows(int c)
+int64_t batch_res_rows(int c, bool f32)
 {
     const uint32_t smem = smem_bytes();
     const int C = batch_res_ctas(c);
-    int64_t lo = 0, hi = c == 3 ? 32767 : 16383;   // offsets of 16 bits
+    const bool two = f32 || c == 3;                // bytes of a row's signs: two, or four
+    int64_t lo = 0, hi = two ? 32767 : 16383;      // offsets of 16 bits
     while (lo < hi) {
         const int64_t mid = (lo + hi + 1) / 2;
-        if (fits(mid, C, c == 3 ? 2 : 4, smem)) lo = mid;
+        if (fits(mid, C, two ? 2 : 4, smem)) lo = mid;
         else hi = mid - 1;
     }
     return lo;
 }
 
-uint32_t batch_res_entry(int c, bool allpos, uint32_t slot, bool neg)
+uint32_t batch_res_entry(int c, bool f32, bool allpos, uint32_t slot, bool neg)
 {
-    return allpos || c == 3 ? 2 * slot + neg : 4 * slot + 2 * neg;
+    return f32 || allpos || c == 3 ? 2 * slot + neg : 4 * slot + 2 * neg;
 }
 
 cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, int32_t agents, Work &w,
@@ -488,7 +585,8 @@ cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, 
     P.ctl = w.ctl;
     P.Ap = d.Ap;
     P.W = d.W;
-    P.groups = (agents + 15) / 16;   // groups of padded agents alone stay as they began
+    const int ka = d.prec == P_F32 ? kAgents<float> : kAgents<__half>;
+    P.groups = (agents + ka - 1) / ka;   // groups of padded agents alone stay as they began
     P.nsteps = d.steps_run;
     P.smem = smem_bytes();
     // the cluster sizes on streams of their own, largest first: the smaller
@@ -502,7 +600,9 @@ cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, 
         e = cudaStreamWaitEvent(t, fork, 0);
         if (e != cudaSuccess) break;
         const int units = B.nbins[c] * P.groups;
-        e = d.prec == P_BF16 ? launch_t<__nv_bfloat16>(P, c, allpos, units, t) : launch_t<__half>(P, c, allpos, units, t);
+        e = d.prec == P_F32    ? launch_t<float>(P, c, allpos, units, t)
+            : d.prec == P_BF16 ? launch_t<__nv_bfloat16>(P, c, allpos, units, t)
+                               : launch_t<__half>(P, c, allpos, units, t);
         if (e == cudaSuccess) e = cudaEventRecord(join[nside], t);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join[nside], 0);
         nside++;
