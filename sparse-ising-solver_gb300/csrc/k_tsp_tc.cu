@@ -23,8 +23,7 @@
 //
 // The MMA completion is a bounded mbarrier wait: a wait that runs out flags
 // CTL_ERR, waits (bounded) for the MMAs in flight, frees TMEM and returns.
-#include "common.cuh"
-#include "engine.h"
+#include "k_step.cuh"
 
 namespace sbx {
 
@@ -37,6 +36,7 @@ constexpr int SBO = 8 * ROWB;         // bytes between 8-row core-matrix groups
 constexpr int LBO = 128;              // bytes between 16-byte K chunks of a group
 constexpr int XROWS = 256 + 2 * KA;   // two tiles of rows and the halo
 constexpr int DPART = NP * ROWB;      // one 32 x 32 part of D
+constexpr int CSP = NP + 4;           // floats of an agent's column sums
 constexpr uint32_t kTcLimit = 1u << 22;
 
 struct TcP {
@@ -124,11 +124,11 @@ __device__ __forceinline__ bool mbar_wait_n(uint32_t bar, uint32_t parity, uint3
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// C FP32 columns of this thread's TMEM lane (C = 32, 16 or 8)
-template <int C> __device__ __forceinline__ void tmem_ld(uint32_t ta, float *v);
-template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t ta, float *v)
+// C FP32 columns of this thread's TMEM lane (C = 32, 16 or 8); tmem_wait before
+// the values are used
+template <int C> __device__ __forceinline__ void tmem_ld(uint32_t ta, uint32_t (&r)[C]);
+template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t ta, uint32_t (&r)[32])
 {
-    uint32_t r[32];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                  "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
                  "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -139,44 +139,66 @@ template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t ta, float *v)
                    "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
                    "=r"(r[31])
                  : "r"(ta));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = __uint_as_float(r[k]);
 }
-template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t ta, float *v)
+template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t ta, uint32_t (&r)[16])
 {
-    uint32_t r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
                  "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
                    "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
                    "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(ta));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
-template <> __device__ __forceinline__ void tmem_ld<8>(uint32_t ta, float *v)
+template <> __device__ __forceinline__ void tmem_ld<8>(uint32_t ta, uint32_t (&r)[8])
 {
-    uint32_t r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
                    "=r"(r[7])
                  : "r"(ta));
+}
+
+// Wait for the thread's loads; the values pass through so that no use of them
+// is moved ahead of it.
+template <int C> __device__ __forceinline__ void tmem_wait(uint32_t (&a)[C], uint32_t (&b)[C], uint32_t (&c)[C])
+{
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = __uint_as_float(r[k]);
+    for (int k = 0; k < C; k++) asm volatile("" : "+r"(a[k]), "+r"(b[k]), "+r"(c[k]));
 }
 
 template <class T> __device__ __forceinline__ float rnd(float v) { return St<T>::ld(St<T>::st(v)); }
 
-// two values rounded to the storage type and back (one packed conversion)
-template <class T> __device__ __forceinline__ float2 rnd2(float2 v);
-template <> __device__ __forceinline__ float2 rnd2<__nv_bfloat16>(float2 v)
+// Packed 16-bit pairs: rounding, and 0xffff per half where x is outside [-1, 1]
+// with x clamped (the reference's sign(x)).
+template <class T> __device__ __forceinline__ uint32_t pack2(float2 v)
 {
-    return __bfloat1622float2(__float22bfloat162_rn(v));
+    const float o[2] = {v.x, v.y};
+    return from_vals<T, 2>(o).u;
 }
-template <> __device__ __forceinline__ float2 rnd2<__half>(float2 v) { return __half22float2(__float22half2_rn(v)); }
+template <class T> __device__ __forceinline__ float2 unpack2(uint32_t w)
+{
+    float o[2];
+    Raw<4> r;
+    r.u = w;
+    to_vals<T, 2>(r, o);
+    return make_float2(o[0], o[1]);
+}
+__device__ __forceinline__ uint32_t outside2(uint32_t &x, __nv_bfloat16)
+{
+    uint32_t c;
+    asm("max.NaN.bf16x2 %0, %1, %2;\n\tmin.NaN.bf16x2 %0, %0, %3;" : "=&r"(c) : "r"(x), "r"(0xbf80bf80u), "r"(0x3f803f80u));
+    const uint32_t m = __hne2_mask(*(const __nv_bfloat162 *)&c, *(const __nv_bfloat162 *)&x);
+    x = c;
+    return m;
+}
+__device__ __forceinline__ uint32_t outside2(uint32_t &x, __half)
+{
+    uint32_t c;
+    asm("max.NaN.f16x2 %0, %1, %2;\n\tmin.NaN.f16x2 %0, %0, %3;" : "=&r"(c) : "r"(x), "r"(0xbc00bc00u), "r"(0x3c003c00u));
+    const uint32_t m = __hne2_mask(*(const __half2 *)&c, *(const __half2 *)&x);
+    x = c;
+    return m;
+}
 
 // H threads share a row m = (i, a): thread part hh owns the cities
 // [32 hh / H, 32 (hh + 1) / H).  Warp w reads TMEM lanes 32 (w mod 4) of
@@ -188,7 +210,8 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
     constexpr int CPT = NP / H;                     // cities of a thread
     __shared__ __align__(1024) unsigned char xs[XROWS * ROWB];   // X with halo, operand layout
     __shared__ __align__(1024) unsigned char ds[3 * DPART];      // D = hi + mid + lo
-    __shared__ float colsum[NP * KA], rsum[NP * KA];
+    __shared__ __align__(16) float colsum[KA * CSP];   // [agent][city], rows padded
+    __shared__ float rsum[NP * KA];
     __shared__ uint32_t rowbits[NP * KA], prevbits[NP * KA];
     __shared__ int aflag[2 * KA];
     __shared__ float s_I2[NP];
@@ -223,6 +246,7 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
         *(unsigned short *)(ds + 2 * DPART + o) = lo;
     }
     for (int t = tid; t < NP; t += blockDim.x) s_I2[t] = t < N ? P.I2[t] : 0.f;
+    for (int t = tid; t < KA * CSP; t += blockDim.x) colsum[t] = 0.f;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -241,7 +265,7 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
 
     // Initial state (x = 0, y from the init stream) and the pre-step
     // Update_XY at step 0 (src/ising_tsp.cu:155).
-    float yr[CPT], xo[CPT];
+    float yi[CPT], xi[CPT];
 #pragma unroll
     for (int j = 0; j < CPT; j++) {
         const int k = k0 + j;
@@ -253,16 +277,20 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
             y = rnd<T>(y + P.k2u * x);
             x = rnd<T>(x + P.k1u * y);
         }
-        yr[j] = y;
-        xo[j] = x;
+        yi[j] = y;
+        xi[j] = x;
+    }
+    // the state in pairs, and 0xffff for each city past N (which stays zero)
+    uint32_t xw[CPT / 2], yw[CPT / 2], pad[CPT / 2];
+#pragma unroll
+    for (int c = 0; c < CPT / 2; c++) {
+        xw[c] = pack2<T>(make_float2(xi[2 * c], xi[2 * c + 1]));
+        yw[c] = pack2<T>(make_float2(yi[2 * c], yi[2 * c + 1]));
+        pad[c] = (k0 + 2 * c < N ? 0u : 0xffffu) | (k0 + 2 * c + 1 < N ? 0u : 0xffff0000u);
     }
     // this thread's part of its row of X (and the halo copies of positions
     // 0 and N-1)
     auto put_row = [&]() {
-        uint32_t w[CPT / 2];
-#pragma unroll
-        for (int c = 0; c < CPT / 2; c++)
-            w[c] = (uint32_t)TT::bits(xo[2 * c]) | ((uint32_t)TT::bits(xo[2 * c + 1]) << 16);
         const int rows[3] = {(i + 1) * KA + a, i == 0 ? (N + 1) * KA + a : -1, i == N - 1 ? a : -1};
 #pragma unroll
         for (int h = 0; h < 3; h++) {
@@ -270,7 +298,7 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
 #pragma unroll
             for (int c = 0; c < CPT / 8; c++)
                 *(uint4 *)(xs + opoff(rows[h], k0 + 8 * c)) =
-                    make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                    make_uint4(xw[4 * c], xw[4 * c + 1], xw[4 * c + 2], xw[4 * c + 3]);
         }
     };
     if (active) {
@@ -333,10 +361,14 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
 #pragma unroll
                     for (int p = 0; p < NP; p++)
                         if (p < N) cs += TT::val(*(const unsigned short *)(xs + opoff((p + 1) * KA + a, i)));
-                    colsum[m] = cs;
+                    colsum[a * CSP + i] = cs;
                     if (H == 1) {
 #pragma unroll
-                        for (int l = 0; l < NP; l++) rs += xo[l];
+                        for (int c = 0; c < CPT / 2; c++) {
+                            const float2 x = unpack2<T>(xw[c]);
+                            rs += x.x;
+                            rs += x.y;
+                        }
                     }
                 } else if (hh == 1) {
                     const int r = (i + 1) * KA + a;
@@ -346,8 +378,9 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
                         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
-                            rs += TT::val((unsigned short)(u[e] & 0xffffu));
-                            rs += TT::val((unsigned short)(u[e] >> 16));
+                            const float2 x = unpack2<T>(u[e]);
+                            rs += x.x;
+                            rs += x.y;
                         }
                     }
                     rsum[m] = rs;
@@ -367,46 +400,48 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
             phase ^= 1u;
             tc_after();
             // the products with hi, mid and lo, summed (hi + mid) + lo
-            float dk[CPT], dm[CPT], dl[CPT];
+            uint32_t dk[CPT], dm[CPT], dl[CPT];
             tmem_ld<CPT>(tlane, dk);
             tmem_ld<CPT>(tlane + NP, dm);
             tmem_ld<CPT>(tlane + 2 * NP, dl);
-#pragma unroll
-            for (int j = 0; j < CPT; j++) dk[j] = (dk[j] + dm[j]) + dl[j];
+            tmem_wait(dk, dm, dl);
             if (active) {
                 if (H > 1) rs = rsum[m];
-                // two cities at a time in packed FP32 (per component the
-                // roundings of fmaf / __fmul_rn), both clamp branches
-                // computed and selected; cities past N stay zero
+                // two cities at a time, FP32 arithmetic in packed pairs (per
+                // component the roundings of fmaf / __fmul_rn) on the packed
+                // 16-bit state, both clamp branches computed and selected
                 const float2 qc = make_float2(P.qc4, P.qc4), qb = make_float2(P.qb4, P.qb4);
                 const float2 rs2 = make_float2(rs, rs);
-                const float2 qa = make_float2(qa8u, qa8u), m1005 = make_float2(-1.005f, -1.005f);
-                const float2 two = make_float2(2.f, 2.f), bt = make_float2(sc.x, sc.x);
+                // twice -1.005 times the force: the doubling is exact
+                const float2 qa = make_float2(qa8u, qa8u), m201 = make_float2(2.f * -1.005f, 2.f * -1.005f);
+                const float2 bt = make_float2(sc.x, sc.x);
                 const float2 cxi = make_float2(P.dtxi0, P.dtxi0), cdt = make_float2(P.dt, P.dt);
                 const float2 cy = make_float2(sc.y, sc.y);
 #pragma unroll
-                for (int j = 0; j < CPT; j += 2) {
-                    const int k = k0 + j;
-                    const float2 cs2 = make_float2(colsum[k * KA + a], colsum[(k + 1) * KA + a]);
-                    // jx = (qc4 colsum + qb4 rs) + qa8u dk as the CUDA-core
-                    // kernel contracts it; qa8u = A/8 times the FP16 operand
-                    // scale 2^s (exact), so qa8u dk is A/8 (2^s dk) bit for bit
-                    const float2 jx = __ffma2_rn(qa, make_float2(dk[j], dk[j + 1]),
-                                                 __ffma2_rn(qb, rs2, __fmul2_rn(qc, cs2)));
-                    const float2 i1 = __fmul2_rn(m1005, jx);
-                    const float2 x0 = make_float2(xo[j], xo[j + 1]), y0 = make_float2(yr[j], yr[j + 1]);
-                    float2 y = rnd2<T>(__ffma2_rn(cxi, __ffma2_rn(bt, make_float2(i2r[j], i2r[j + 1]),
-                                                                   __fmul2_rn(two, i1)), y0));
-                    const float2 x = rnd2<T>(__ffma2_rn(cdt, y, x0));
-                    y = rnd2<T>(__ffma2_rn(cy, x, y));
-                    const bool c0 = fabsf(x0.x) > 1.f, c1 = fabsf(x0.y) > 1.f;
-                    if (k < N) {
-                        xo[j] = c0 ? spin_of(x0.x) : x.x;
-                        yr[j] = c0 ? 0.f : y.x;
-                    }
-                    if (k + 1 < N) {
-                        xo[j + 1] = c1 ? spin_of(x0.y) : x.y;
-                        yr[j + 1] = c1 ? 0.f : y.y;
+                for (int j = 0; j < CPT; j += 4) {
+                    const float4 c4 = *(const float4 *)&colsum[a * CSP + k0 + j];
+#pragma unroll
+                    for (int e = 0; e < 4; e += 2) {
+                        const int k = j + e, c = k / 2;
+                        const float2 cs2 = e ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+                        const float2 d = __fadd2_rn(
+                            __fadd2_rn(make_float2(__uint_as_float(dk[k]), __uint_as_float(dk[k + 1])),
+                                       make_float2(__uint_as_float(dm[k]), __uint_as_float(dm[k + 1]))),
+                            make_float2(__uint_as_float(dl[k]), __uint_as_float(dl[k + 1])));
+                        // jx = (qc4 colsum + qb4 rs) + qa8u d; qa8u = A/8 times
+                        // the FP16 operand scale 2^s (exact), so qa8u d is
+                        // A/8 (2^s d) bit for bit
+                        const float2 jx = __ffma2_rn(qa, d, __ffma2_rn(qb, rs2, __fmul2_rn(qc, cs2)));
+                        const float2 x0 = unpack2<T>(xw[c]), y0 = unpack2<T>(yw[c]);
+                        float2 y = __ffma2_rn(cxi, __ffma2_rn(bt, make_float2(i2r[k], i2r[k + 1]),
+                                                              __fmul2_rn(m201, jx)), y0);
+                        y = unpack2<T>(pack2<T>(y));
+                        const uint32_t nx = pack2<T>(__ffma2_rn(cdt, y, x0));
+                        const uint32_t ny = pack2<T>(__ffma2_rn(cy, unpack2<T>(nx), y));
+                        uint32_t cl = xw[c];
+                        const uint32_t out = outside2(cl, T()) | pad[c];
+                        xw[c] = (cl & out) | (nx & ~out);
+                        yw[c] = ny & ~out;
                     }
                 }
                 put_row();
@@ -424,7 +459,7 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
         if (active) {
 #pragma unroll
             for (int j = 0; j < CPT; j++)
-                if (k0 + j < N) part |= sbit(xo[j]) << j;
+                part |= ((xw[j / 2] >> (15 + 16 * (j & 1))) & 1u) << j;   // cities past N are +0
             if (H == 1) rowbits[m] = part;
             else if (H == 2) ((unsigned short *)rowbits)[2 * m + hh] = (unsigned short)part;
             else ((unsigned char *)rowbits)[4 * m + hh] = (unsigned char)part;
@@ -466,8 +501,10 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
             const int k = k0 + j;
             if (k < N) {
                 const int64_t gi = (int64_t)(i * N + k) * P.Ap + ag;
-                xg[gi] = St<T>::st(xo[j]);
-                yg[gi] = St<T>::st(yr[j]);
+                const unsigned short xb = (unsigned short)(xw[j / 2] >> (16 * (j & 1)));
+                const unsigned short yb = (unsigned short)(yw[j / 2] >> (16 * (j & 1)));
+                memcpy(&xg[gi], &xb, 2);
+                memcpy(&yg[gi], &yb, 2);
             }
         }
         const uint32_t bits = prevbits[m];
