@@ -795,6 +795,9 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     if ((pr->kernel == SBX_KERNEL_AUTO || pr->kernel == SBX_KERNEL_RESIDENT_SPLIT) && !d.trace && !ka &&
         !pr->agents_per_block)
         rs = resident_rs_pick(d, p->J, pr->kernel == SBX_KERNEL_RESIDENT_SPLIT);
+    // FP64: by itself, unless a streaming tile or a profile is asked for
+    const bool r64 = pr->kernel == SBX_KERNEL_AUTO && !d.trace && !profile && !pr->agents_per_block && !pr->lane_agents &&
+                     !pr->row_lanes && !pr->block_threads && !pr->count_mode && !pr->staging && resident64_pick(d, p->J);
     if (pr->kernel == SBX_KERNEL_RESIDENT && !ka)
         return fail(ctx, SBX_ERR_UNSUPPORTED, "resident kernel: shape does not fit on chip (or FP64)");
     if (pr->kernel == SBX_KERNEL_RESIDENT_SPLIT && !rs)
@@ -802,8 +805,8 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
                     "split resident kernel: 16-bit fused state, degree <= 127 and fitting on chip only");
     DevCsr &Jm = const_cast<DevCsr &>(p->J);
     if (ka == 8 && (rc = ensure_sell(ctx, Jm, Jm.sell[0], 4))) return rc;
-    if (rs && (rc = ensure_sell(ctx, Jm, Jm.sell[1], 1))) return rc;
-    if (!ka && !rs) {
+    if ((rs || r64) && (rc = ensure_sell(ctx, Jm, Jm.sell[1], 1))) return rc;
+    if (!ka && !rs && !r64) {
         bool timed = false;
         if ((rc = pick_tile(ctx, d, p->J, pr, &timed))) return rc;
         if (timed && (rc = init_state(ctx, d, pr->seed, false))) return rc;
@@ -811,8 +814,9 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     int launches = 0, hot = 0;
     CK(cudaEventRecord(ctx->ev0, s));
     auto resident = [&](int32_t step0, int32_t nsteps, bool first) {
-        return ka ? launch_resident(d, p->J, ctx->w, ka, step0, nsteps, first, s)
-                  : launch_resident_rs(d, p->J, ctx->w, rs, step0, nsteps, first, false, s);
+        return ka    ? launch_resident(d, p->J, ctx->w, ka, step0, nsteps, first, s)
+               : r64 ? launch_resident64(d, p->J, ctx->w, step0, nsteps, first, s)
+                     : launch_resident_rs(d, p->J, ctx->w, rs, step0, nsteps, first, false, s);
     };
     bool coop_done = false;
     if (rs && d.uw && nchunks > 0) {
@@ -831,7 +835,7 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
         }
     }
     if (coop_done) {
-    } else if (ka || rs) {
+    } else if (ka || rs || r64) {
         if (d.uw) {
             for (int64_t c = 0; c < std::max<int64_t>(nchunks, 1); c++) {
                 CK(resident((int32_t)(c * d.period), nchunks ? d.period : 0, c == 0));
@@ -875,9 +879,9 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     res->steps_run = ctl[CTL_STEP];
     res->windows_run = ctl[CTL_WINDOWS];
     for (uint8_t b : bif) res->bifurcated += b;
-    res->kernel_used = ka ? SBX_KERNEL_RESIDENT : rs ? SBX_KERNEL_RESIDENT_SPLIT : SBX_KERNEL_STREAM;
-    res->agents_per_block = ka ? ka : rs;
-    if (!ka && !rs) {
+    res->kernel_used = ka || r64 ? SBX_KERNEL_RESIDENT : rs ? SBX_KERNEL_RESIDENT_SPLIT : SBX_KERNEL_STREAM;
+    res->agents_per_block = ka ? ka : r64 ? 1 : rs;
+    if (!ka && !rs && !r64) {
         res->lane_agents = d.tv ? d.tv : default_v(d);
         res->row_lanes = d.tlr;
         res->block_threads = d.tbt;
@@ -885,7 +889,7 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
         res->staging = d.tst + 1;
     }
     if ((rc = read_trace(ctx, d, ctl[CTL_TRACED], pr->target, res))) return rc;
-    if (ka || rs) {
+    if (ka || rs || r64) {
         res->kernel_launches = hot;
         res->kernel_ms = profile ? ms : 0;
     } else {

@@ -283,6 +283,12 @@ cudaError_t launch_resident(const SolveDims &d, const DevCsr &J, Work &w, int ka
 int64_t resident_batch_max_rows();
 cudaError_t launch_resident_batch(const SolveDims &d, const DevRb &B, Work &w, cudaStream_t s);
 
+// Resident FP64 kernel for small graphs, +-1 weights (k_resident_f64.cu), one
+// agent per CTA: whether it is the faster one, and nsteps steps of it.
+bool resident64_pick(const SolveDims &d, const DevCsr &J);
+cudaError_t launch_resident64(const SolveDims &d, const DevCsr &J, Work &w, int32_t step0, int32_t nsteps, bool first,
+                              cudaStream_t s);
+
 // On-chip batch kernel (k_batch_res.cu), kinds 0..3 of bins (DevBres): the
 // CTAs of a bin's cluster, its most rows, the entry of a neighbour.  The
 // launch runs all d.steps_run fused steps of every bin, the kinds on the side
