@@ -336,14 +336,19 @@ __device__ __forceinline__ void count_bits_s(const StepP &P, const uint32_t *Sq,
     constexpr int T = 32 / LR;     // column words per lane per block
     constexpr int KPL = LR / G;    // neighbours per lane per column word
     const uint32_t *cwp = P.colw + e0 + sl;   // this lane's column words, from one base
+    // past a row's end: the zero row (word 0, weight sign clear), so those
+    // terms vanish without a test per word.  The next block's column words are
+    // on their way while this one's sign words are gathered.
+    uint32_t nextcw[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) nextcw[t] = t * LR + sl < dw ? __ldg(cwp + t * LR) : P.zrow;
     for (int32_t cb = 0; cb < dmax; cb += 32) {
-        // past a row's end: the zero row (word 0, weight sign clear), so
-        // those terms vanish without a test per word
         uint32_t mycw[T];
 #pragma unroll
         for (int t = 0; t < T; t++) {
-            const int32_t idx = cb + t * LR + sl;
-            mycw[t] = idx < dw ? __ldg(cwp + cb + t * LR) : P.zrow;
+            mycw[t] = nextcw[t];
+            const int32_t idx = cb + 32 + t * LR + sl;
+            nextcw[t] = idx < dw ? __ldg(cwp + cb + 32 + t * LR) : P.zrow;
         }
         uint32_t w[T * KPL];
 #pragma unroll
@@ -1155,6 +1160,53 @@ cudaError_t step_kw(const SolveDims &d, const DevCsr &J, const StepP &P, int off
     return cudaErrorInvalidValue;
 }
 
+// Two 16-bit values at a time: x clamped to [-1, 1], 0xffff for each that the
+// clamp moved.
+template <class T> __device__ __forceinline__ uint32_t outside2(uint32_t &x);
+template <> __device__ __forceinline__ uint32_t outside2<__nv_bfloat16>(uint32_t &x)
+{
+    uint32_t c;
+    asm("max.NaN.bf16x2 %0, %1, %2;\n\tmin.NaN.bf16x2 %0, %0, %3;" : "=&r"(c) : "r"(x), "r"(0xbf80bf80u), "r"(0x3f803f80u));
+    const uint32_t m = __hne2_mask(*(const __nv_bfloat162 *)&c, *(const __nv_bfloat162 *)&x);
+    x = c;
+    return m;
+}
+template <> __device__ __forceinline__ uint32_t outside2<__half>(uint32_t &x)
+{
+    uint32_t c;
+    asm("max.NaN.f16x2 %0, %1, %2;\n\tmin.NaN.f16x2 %0, %0, %3;" : "=&r"(c) : "r"(x), "r"(0xbc00bc00u), "r"(0x3c003c00u));
+    const uint32_t m = __hne2_mask(*(const __half2 *)&c, *(const __half2 *)&x);
+    x = c;
+    return m;
+}
+
+// sb_update16 of a fused step with a zero force: a clamped y is zeroed before
+// it is unpacked (one instruction for two), the zero force's addition only
+// turns -0 into +0.
+template <class T, int V>
+__device__ __forceinline__ void iso_update16(uint32_t (&xw)[V / 2], uint32_t (&yw)[V / 2], float c0, const float4 &c)
+{
+    const float2 c02 = make_float2(c0, c0), zero = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < V / 2; i++) {
+        Raw<4> r;
+        float x[2], y[2];
+        r.u = yw[i] & ~outside2<T>(xw[i]);
+        to_vals<T, 2>(r, y);
+        float2 Y = __ffma2_rn(c02, zero, make_float2(y[0], y[1]));
+        r.u = xw[i];
+        to_vals<T, 2>(r, x);
+        const float2 X = __ffma2_rn(make_float2(c.x, c.x), Y, make_float2(x[0], x[1]));
+        Y = __ffma2_rn(make_float2(c.y, c.y), X, Y);
+        x[0] = X.x;
+        x[1] = X.y;
+        y[0] = Y.x;
+        y[1] = Y.y;
+        xw[i] = from_vals<T, 2>(x).u;
+        yw[i] = from_vals<T, 2>(y).u;
+    }
+}
+
 // Isolated rows (degree 0, the last P.niso entries of P.order) have no
 // neighbour and are no row's neighbour: the force on them is zero at every
 // step and no step reads their signs.  One launch advances them through a
@@ -1215,7 +1267,7 @@ __global__ void __launch_bounds__(NT) k_iso(const StepP P, const int nsteps)
         auto one = [&](int k) {
             const auto c = Coef<A>::get(P, step0 + k);
             if constexpr (sizeof(T) == 2) {
-                sb_update16<T, K_FUSED, false, V>(qx, qy, zero, c0, c, c);
+                iso_update16<T, V>(qx, qy, c0, c);
             } else {
                 sb_update<K_FUSED, false, V>(x, y, zero, c0, c, c);
                 xw = from_vals<T, V>(x);

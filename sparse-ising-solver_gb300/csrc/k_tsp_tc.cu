@@ -168,8 +168,7 @@ template <int C> __device__ __forceinline__ void tmem_wait(uint32_t (&a)[C], uin
 
 template <class T> __device__ __forceinline__ float rnd(float v) { return St<T>::ld(St<T>::st(v)); }
 
-// Packed 16-bit pairs: rounding, and 0xffff per half where x is outside [-1, 1]
-// with x clamped (the reference's sign(x)).
+// Packed 16-bit pairs.
 template <class T> __device__ __forceinline__ uint32_t pack2(float2 v)
 {
     const float o[2] = {v.x, v.y};
@@ -183,23 +182,6 @@ template <class T> __device__ __forceinline__ float2 unpack2(uint32_t w)
     to_vals<T, 2>(r, o);
     return make_float2(o[0], o[1]);
 }
-__device__ __forceinline__ uint32_t outside2(uint32_t &x, __nv_bfloat16)
-{
-    uint32_t c;
-    asm("max.NaN.bf16x2 %0, %1, %2;\n\tmin.NaN.bf16x2 %0, %0, %3;" : "=&r"(c) : "r"(x), "r"(0xbf80bf80u), "r"(0x3f803f80u));
-    const uint32_t m = __hne2_mask(*(const __nv_bfloat162 *)&c, *(const __nv_bfloat162 *)&x);
-    x = c;
-    return m;
-}
-__device__ __forceinline__ uint32_t outside2(uint32_t &x, __half)
-{
-    uint32_t c;
-    asm("max.NaN.f16x2 %0, %1, %2;\n\tmin.NaN.f16x2 %0, %0, %3;" : "=&r"(c) : "r"(x), "r"(0xbc00bc00u), "r"(0x3c003c00u));
-    const uint32_t m = __hne2_mask(*(const __half2 *)&c, *(const __half2 *)&x);
-    x = c;
-    return m;
-}
-
 // H threads share a row m = (i, a): thread part hh owns the cities
 // [32 hh / H, 32 (hh + 1) / H).  Warp w reads TMEM lanes 32 (w mod 4) of
 // tile (w / 4) mod T, part (w / 4) / T; 128 T H threads.
@@ -439,7 +421,7 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
                         const uint32_t nx = pack2<T>(__ffma2_rn(cdt, y, x0));
                         const uint32_t ny = pack2<T>(__ffma2_rn(cy, unpack2<T>(nx), y));
                         uint32_t cl = xw[c];
-                        const uint32_t out = outside2(cl, T()) | pad[c];
+                        const uint32_t out = outside2<T>(cl) | pad[c];
                         xw[c] = (cl & out) | (nx & ~out);
                         yw[c] = ny & ~out;
                     }
