@@ -150,6 +150,9 @@ void free_csr(DevCsr &J)
     cudaFree(J.valf);
     cudaFree(J.perm);
     cudaFree(J.hchunk);
+    cudaFree(J.light);
+    J.light = nullptr;
+    J.nlight = 0;
     cudaFree(J.chunk_row);
     cudaFree(J.c0r32);
     cudaFree(J.c0r64);
@@ -328,6 +331,28 @@ int upload_device(sbx_ctx *ctx, DevCsr &J)
         }
     }
     CK(cudaMemcpy(J.perm, J.hperm.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
+    if (J.unit && (J.skewed || J.niso)) {   // visited in degree order
+        int64_t first = n - J.niso;
+        while (first > 0) {
+            const size_t r = (size_t)J.hperm[(size_t)first - 1];
+            if (rowptr[r + 1] - rowptr[r] > kLight) break;
+            first--;
+        }
+        J.nlight = (int32_t)(n - J.niso - first);
+        std::vector<uint32_t> rec((size_t)J.nlight * 8, (uint32_t)n);   // past a row's end: the zero row
+        parallel(J.nlight > (1 << 16) ? host_threads() : 1, [&](int t, int TT) {
+            for (int64_t i = (int64_t)J.nlight * t / TT; i < (int64_t)J.nlight * (t + 1) / TT; i++) {
+                const size_t r = (size_t)J.hperm[(size_t)(first + i)];
+                rec[(size_t)i * 8] = (uint32_t)r;
+                rec[(size_t)i * 8 + 1] = (uint32_t)(rowptr[r + 1] - rowptr[r]);
+                for (int32_t e = rowptr[r]; e < rowptr[r + 1]; e++) rec[(size_t)i * 8 + 2 + (size_t)(e - rowptr[r])] = colw[(size_t)e];
+            }
+        });
+        if (J.nlight) {
+            CK(cudaMalloc(&J.light, sizeof(uint32_t) * rec.size()));
+            CK(cudaMemcpy(J.light, rec.data(), sizeof(uint32_t) * rec.size(), cudaMemcpyHostToDevice));
+        }
+    }
     if (J.nchunks) {
         std::vector<int32_t> hchunk((size_t)n, -1), crow;
         crow.reserve((size_t)J.nchunks);

@@ -30,6 +30,10 @@ constexpr int kHeavy = 127;
 // (R-MAT scale 20 on GB300: 8, 12 and 20 timed within 1%).
 constexpr int kBitsMin = 12;
 
+// Rows of 1 to kLight neighbours of a +-1 matrix whose rows are visited in
+// degree order have a record of eight words: row, degree, column words.
+constexpr int kLight = 6;
+
 inline size_t prec_bytes(int p) { return p == P_F64 ? 8 : p == P_F32 ? 4 : 2; }
 
 // An attribute of the calling thread's current device (0 when the query
@@ -73,6 +77,8 @@ struct DevCsr {
     bool skewed = false;     // max degree > 8x mean: the step kernel visits rows in perm order
     int64_t nheavy = 0;      // heavy rows: the first nheavy entries of perm
     int64_t niso = 0;        // isolated rows (degree 0): the last niso entries of perm
+    uint32_t *light = nullptr;   // records of the nlight rows before those (kLight)
+    int32_t nlight = 0;
     // Heavy rows (unit weights, degree > kHeavy) are split into chunks of
     // kHeavy neighbours, each counted by its own work item of the step kernel.
     int32_t *hchunk = nullptr;    // per row: first chunk of a heavy row, else -1

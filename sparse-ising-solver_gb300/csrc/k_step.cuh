@@ -55,6 +55,8 @@ struct StepP {
                                           // are counted in bit planes (INT32_MAX: none)
     int64_t niso;                         // isolated rows left to k_iso: the last niso entries of
                                           // order, which the row items then skip
+    const uint32_t *__restrict__ light;   // records of the light rows, the nlight entries of order
+    int32_t nlight;                       // before those (0: none), which the row items skip too
     double c0;
     int32_t giveup;                       // test only: the staged-row wait gives up at once
 };
@@ -805,9 +807,69 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
         }
     }
 
+    // The totals from byte counters of 2 * count.
+    auto unit_totals = [&](uint32_t lo, uint32_t hi, int32_t deg, A (&tv)[V]) {
+        if constexpr (std::is_same<A, float>::value) {
+            // PRMT builds the float 2^23 + 2*count from a byte
+            // counter; minus (2^23 + deg) it is 2*count - deg exactly
+            const float bias = 8388608.0f + (float)deg;
+#pragma unroll
+            for (int v = 0; v < V; v++)
+                tv[v] = __uint_as_float(__byte_perm(v < 4 ? lo : hi, 0x4b000000u, 0x7440u + (v & 3))) - bias;
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; v++)
+                tv[v] = (A)((int)(((v < 4 ? lo : hi) >> (8 * (v & 3))) & 0xffu) - deg);
+        }
+    };
+
+    // Light rows (at most kLight neighbours): one record of eight words a row
+    // -- row, degree, columns -- loaded an item ahead, so that a row's x, y and
+    // all its sign words are requested at once.  Through the order, the row
+    // pointers and the columns it is four dependent loads, and rows of two
+    // neighbours (most of R-MAT's) took three times their bytes' time.
+    if constexpr (WM == W_UNIT && LR == 32 && !ST && KIND != K_XY) {
+        // from the last warp down: the row items' remainder is the first warps'
+        int32_t g = (int32_t)(nw - 1 - w0);
+        const int32_t nw32 = (int32_t)nw;
+        uint32_t rec = g < P.nlight ? __ldg(&P.light[(int64_t)g * 8 + (lane & 7)]) : 0u;
+        while (g < P.nlight) {
+            const uint32_t cur = rec;
+            g += nw32;
+            if (g < P.nlight) rec = __ldg(&P.light[(int64_t)g * 8 + (lane & 7)]);
+            const int32_t r = (int32_t)__shfl_sync(FULL, cur, 0), deg = (int32_t)__shfl_sync(FULL, cur, 1);
+            for (int it = 0; it < nit; it++) {
+                const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
+                const int q = a0 >> 5, off = a0 & 31;
+                const int64_t base = (int64_t)r * P.Ap + a0;
+                uint32_t wp_old = 0;
+                if (WIN && (lane & (G - 1)) == 0) wp_old = P.Wp[(int64_t)r * P.W + q];
+                const RawT xr = vload_s<T, V>(xp + base, cs);
+                const RawT yr = vload_s<T, V>(yp + base, cs);
+                uint32_t w[kLight], lo = 0, hi = 0;
+#pragma unroll
+                for (int k = 0; k < kLight; k++) {
+                    const uint32_t cw = __shfl_sync(FULL, cur, 2 + k);   // past the row's end: the zero row
+                    w[k] = 0u;
+                    if (k < deg) w[k] = plane_ld(Scur + q, cw & 0x7fffffffu, P.W) ^ (uint32_t)((int32_t)cw >> 31);
+                }
+#pragma unroll
+                for (int k = 0; k < kLight; k++) {
+                    if (k >= deg) break;   // warp-uniform
+                    const uint32_t bits = w[k] >> off;
+                    lo += spread2x(bits & 0xfu);
+                    if (V == 8) hi += spread2x((bits >> 4) & 0xfu);
+                }
+                A tv[V];
+                unit_totals(lo, hi, deg, tv);
+                finish(r, q, off, base, !RAG || a1 == a0, xr, yr, tv, row_c0(r), wp_old);
+            }
+        }
+    }
+
     // Row items (group g, segment it) in steps of the warp count, advanced
     // without divisions: g += nw / nit, it += nw % nit with carry.
-    const int64_t nrows = P.n - P.row0 - P.niso;
+    const int64_t nrows = P.n - P.row0 - P.niso - P.nlight;
     const int64_t ng = (nrows + RW - 1) / RW;
     const int64_t dr = nw / nit;
     const int dit = (int)(nw - dr * nit);
@@ -827,18 +889,7 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
                 } else {
                     count_unit<V, LR>(P, Scur + q, off, e0, deg, sl, lo, hi);
                 }
-                if constexpr (std::is_same<A, float>::value) {
-                    // PRMT builds the float 2^23 + 2*count from a byte
-                    // counter; minus (2^23 + deg) it is 2*count - deg exactly
-                    const float bias = 8388608.0f + (float)deg;
-#pragma unroll
-                    for (int v = 0; v < V; v++)
-                        tv[v] = __uint_as_float(__byte_perm(v < 4 ? lo : hi, 0x4b000000u, 0x7440u + (v & 3))) - bias;
-                } else {
-#pragma unroll
-                    for (int v = 0; v < V; v++)
-                        tv[v] = (A)((int)(((v < 4 ? lo : hi) >> (8 * (v & 3))) & 0xffu) - deg);
-                }
+                unit_totals(lo, hi, deg, tv);
             } else {
                 R tot[V];
 #pragma unroll
@@ -1046,7 +1097,13 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
     }
     // isolated rows (P.niso, left to k_iso) are the end of the degree order
     if (P.niso && !Q.order) return cudaErrorInvalidValue;
-    const int64_t items = ((d.n - Q.row0 - P.niso + RW - 1) / RW + (big ? J.nchunks : 0)) * nit;
+    // light rows by their records, where they end the row items
+    const bool stage = LR == 32 && !WIN && KIND != K_XY && !RAG && d.tst != 0 && J.unit;
+    if (LR == 32 && KIND != K_XY && J.unit && J.light && Q.order && P.niso == J.niso && !stage) {
+        Q.light = J.light;
+        Q.nlight = J.nlight;
+    }
+    const int64_t items = ((d.n - Q.row0 - P.niso - Q.nlight + RW - 1) / RW + Q.nlight + (big ? J.nchunks : 0)) * nit;
     // count mode of the +-1 rows: byte counters per lane (0), bit planes (1),
     // or mixed (2: the byte-counter kernel with P.bits_min set, heavy rows
     // only); staged rows (x, y copied ahead into shared memory) for

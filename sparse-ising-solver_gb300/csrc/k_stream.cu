@@ -170,6 +170,8 @@ StepP make_step(const SolveDims &d, const DevCsr &J, Work &w)
     P.allpos = J.allpos ? 1 : 0;
     P.bits_min = d.tcm == 2 ? kBitsMin : INT32_MAX;
     P.niso = 0;
+    P.light = nullptr;   // set per kernel (step_vl)
+    P.nlight = 0;
     P.nchunks = J.nchunks;
     P.order = nullptr;   // set per kernel (step_vl)
     P.row0 = 0;
@@ -288,6 +290,10 @@ cudaError_t launch_chunk(const SolveDims &d, const DevCsr &J, Work &w, cudaStrea
 cudaError_t launch_plain_steps(const SolveDims &d, const DevCsr &J, Work &w, int count, cudaStream_t s)
 {
     StepP P = make_step(d, J, w);
+    if (d.fused && J.niso && !d.tbsm) {   // as launch_chunk: the step kernels of a window skip them
+        P.niso = J.niso;
+        P.order = J.perm;
+    }
     for (int i = 0; i < count; i++) {
         const cudaError_t e = step(d, J, P, d.fused ? K_FUSED : K_FC, false, 0, s);
         if (e != cudaSuccess) return e;
