@@ -830,39 +830,57 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
     // neighbours (most of R-MAT's) took three times their bytes' time.
     if constexpr (WM == W_UNIT && LR == 32 && !ST && KIND != K_XY) {
         // from the last warp down: the row items' remainder is the first warps'
-        int32_t g = (int32_t)(nw - 1 - w0);
-        const int32_t nw32 = (int32_t)nw;
-        uint32_t rec = g < P.nlight ? __ldg(&P.light[(int64_t)g * 8 + (lane & 7)]) : 0u;
-        while (g < P.nlight) {
-            const uint32_t cur = rec;
-            g += nw32;
-            if (g < P.nlight) rec = __ldg(&P.light[(int64_t)g * 8 + (lane & 7)]);
-            const int32_t r = (int32_t)__shfl_sync(FULL, cur, 0), deg = (int32_t)__shfl_sync(FULL, cur, 1);
-            for (int it = 0; it < nit; it++) {
-                const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
-                const int q = a0 >> 5, off = a0 & 31;
-                const int64_t base = (int64_t)r * P.Ap + a0;
-                uint32_t wp_old = 0;
-                if (WIN && (lane & (G - 1)) == 0) wp_old = P.Wp[(int64_t)r * P.W + q];
-                const RawT xr = vload_s<T, V>(xp + base, cs);
-                const RawT yr = vload_s<T, V>(yp + base, cs);
-                uint32_t w[kLight], lo = 0, hi = 0;
+        int32_t g = (int32_t)(nw - 1 - w0), it = 0;
+        const int32_t nw32 = (int32_t)nw, nl = P.nlight;
+        auto record = [&](int32_t i) { return i < nl ? __ldg(&P.light[(int64_t)i * 8 + (lane & 7)]) : 0u; };
+        // x, y of segment i of a record's row, one item ahead of their use
+        auto state = [&](uint32_t rec, int i, RawT &xr, RawT &yr) {
+            const int a1 = i * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
+            const int64_t base = (int64_t)__shfl_sync(FULL, rec, 0) * P.Ap + a0;
+            xr = vload_s<T, V>(xp + base, cs);
+            yr = vload_s<T, V>(yp + base, cs);
+        };
+        uint32_t rec = record(g), rec1 = record(g + nw32), rec2;
+        RawT xr, yr;
+        if (g < nl) state(rec, 0, xr, yr);
+        while (g < nl) {
+            const bool end = it + 1 == nit;   // warp-uniform
+            const bool more = !end || g + nw32 < nl;
+            if (end) rec2 = record(g + 2 * nw32);
+            RawT xn = xr, yn = yr;
+            if (more) state(end ? rec1 : rec, end ? 0 : it + 1, xn, yn);
+            const int32_t r = (int32_t)__shfl_sync(FULL, rec, 0), deg = (int32_t)__shfl_sync(FULL, rec, 1);
+            const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
+            const int q = a0 >> 5, off = a0 & 31;
+            const int64_t base = (int64_t)r * P.Ap + a0;
+            uint32_t wp_old = 0;
+            if (WIN && (lane & (G - 1)) == 0) wp_old = P.Wp[(int64_t)r * P.W + q];
+            uint32_t w[kLight], lo = 0, hi = 0;
 #pragma unroll
-                for (int k = 0; k < kLight; k++) {
-                    const uint32_t cw = __shfl_sync(FULL, cur, 2 + k);   // past the row's end: the zero row
-                    w[k] = 0u;
-                    if (k < deg) w[k] = plane_ld(Scur + q, cw & 0x7fffffffu, P.W) ^ (uint32_t)((int32_t)cw >> 31);
-                }
+            for (int k = 0; k < kLight; k++) {
+                const uint32_t cw = __shfl_sync(FULL, rec, 2 + k);   // past the row's end: the zero row
+                w[k] = 0u;
+                if (k < deg) w[k] = plane_ld(Scur + q, cw & 0x7fffffffu, P.W) ^ (uint32_t)((int32_t)cw >> 31);
+            }
 #pragma unroll
-                for (int k = 0; k < kLight; k++) {
-                    if (k >= deg) break;   // warp-uniform
-                    const uint32_t bits = w[k] >> off;
-                    lo += spread2x(bits & 0xfu);
-                    if (V == 8) hi += spread2x((bits >> 4) & 0xfu);
-                }
-                A tv[V];
-                unit_totals(lo, hi, deg, tv);
-                finish(r, q, off, base, !RAG || a1 == a0, xr, yr, tv, row_c0(r), wp_old);
+            for (int k = 0; k < kLight; k++) {
+                if (k >= deg) break;   // warp-uniform
+                const uint32_t bits = w[k] >> off;
+                lo += spread2x(bits & 0xfu);
+                if (V == 8) hi += spread2x((bits >> 4) & 0xfu);
+            }
+            A tv[V];
+            unit_totals(lo, hi, deg, tv);
+            finish(r, q, off, base, !RAG || a1 == a0, xr, yr, tv, row_c0(r), wp_old);
+            xr = xn;
+            yr = yn;
+            if (end) {
+                g += nw32;
+                rec = rec1;
+                rec1 = rec2;
+                it = 0;
+            } else {
+                it++;
             }
         }
     }
