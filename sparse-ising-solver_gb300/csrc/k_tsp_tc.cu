@@ -317,7 +317,9 @@ __global__ void __launch_bounds__(128 * 2 * H, 1) k_tsp_tc(const TcP P)
             // the distance product of the current X: 4 MMAs per tile (both
             // neighbour positions, two K halves), N = 96 covering the three
             // parts of D at once
-            if (tid == 0) {
+            // (issued by the last warp, which with H = 4 has no sum to add:
+            // behind the first warp's issue its column sums waited too)
+            if (tid == (int)blockDim.x - 32) {
                 for (int t = 0; t < T2; t++) {
                     uint32_t acc = 0;
 #pragma unroll
