@@ -814,15 +814,16 @@ int solve_maxcut(sbx_ctx *ctx, const sbx_problem *p, const sbx_params *pr, sbx_r
     if ((rc = init_state(ctx, d, pr->seed, false))) return rc;
 
     // on-chip kernels first: shared-memory resident, then tensor memory + shared
+    const bool tile_asked = pr->lane_agents || pr->row_lanes || pr->block_threads || pr->count_mode || pr->staging;
     int ka = 0, rs = 0;
     if ((pr->kernel == SBX_KERNEL_AUTO || pr->kernel == SBX_KERNEL_RESIDENT) && !d.trace)
         ka = resident_pick_ka(d, p->J, pr->agents_per_block);
     if ((pr->kernel == SBX_KERNEL_AUTO || pr->kernel == SBX_KERNEL_RESIDENT_SPLIT) && !d.trace && !ka &&
         !pr->agents_per_block)
-        rs = resident_rs_pick(d, p->J, pr->kernel == SBX_KERNEL_RESIDENT_SPLIT);
+        rs = resident_rs_pick(d, p->J, pr->kernel == SBX_KERNEL_RESIDENT_SPLIT, tile_asked);
     // FP64: by itself, unless a streaming tile or a profile is asked for
-    const bool r64 = pr->kernel == SBX_KERNEL_AUTO && !d.trace && !profile && !pr->agents_per_block && !pr->lane_agents &&
-                     !pr->row_lanes && !pr->block_threads && !pr->count_mode && !pr->staging && resident64_pick(d, p->J);
+    const bool r64 = pr->kernel == SBX_KERNEL_AUTO && !d.trace && !profile && !pr->agents_per_block && !tile_asked &&
+                     resident64_pick(d, p->J);
     if (pr->kernel == SBX_KERNEL_RESIDENT && !ka)
         return fail(ctx, SBX_ERR_UNSUPPORTED, "resident kernel: shape does not fit on chip (or FP64)");
     if (pr->kernel == SBX_KERNEL_RESIDENT_SPLIT && !rs)
@@ -1843,8 +1844,8 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             return fail(ctx, SBX_ERR_UNSUPPORTED,
                         "count_mode 4 (shared-memory planes): 16-bit state, +-1 weights, degree <= 127, "
                         "32/64/128 agents and instances whose plane fits in shared memory");
-        const bool use_bsm = bsm_fit && !tile_pinned && pr->kernel != SBX_KERNEL_RESIDENT &&
-                             pr->kernel != SBX_KERNEL_RESIDENT_SPLIT;
+        bool use_bsm = bsm_fit && !tile_pinned && pr->kernel != SBX_KERNEL_RESIDENT &&
+                       pr->kernel != SBX_KERNEL_RESIDENT_SPLIT;
         // the on-chip batch kernel: +-1 fused classes (not FP64) whose instances
         // fit a cluster, unless a tile, a count mode or a kernel is asked for
         // (256 tori of 947,961 rows in all at 64 agents: 52 us a step, the
@@ -1859,9 +1860,14 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             use_res = bres.rows != nullptr;
             if (use_res) use_rb = false;
         }
-        // ... else the plane kernel before the resident batch, which it also
-        // outruns at low degree (8 tori, 25,369 rows: 7.7 us a step against 18.7)
-        if (use_rb && by_itself && !tile_pinned && bsm_ok(c, d)) use_rb = false;
+        // ... else a step kernel before the resident batch, which they outrun
+        // at low degree (8 tori, 20,434 rows at 64 agents: 17.7 us a step, the
+        // plane kernel 6.3, the streaming step 4.3): the streaming step, unless
+        // a CTA size of the plane kernel is asked for
+        if (use_rb && by_itself && !tile_pinned && bsm_ok(c, d)) {
+            use_rb = false;
+            use_bsm = bsm_threads;
+        }
         c.J.bsm = nullptr;
         if (use_res) {
             if ((rc = upload_bres_cb(ctx, c, bres, pr->dt))) return rc;

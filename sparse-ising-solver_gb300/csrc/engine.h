@@ -308,7 +308,7 @@ cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, 
 
 // Tensor-memory + shared-memory resident kernel (k_resident_rs.cu), fused
 // steps: its agents per CTA (8 of 16-bit state, 4 of FP32) when it is to run.
-int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced);
+int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced, bool tile);
 // coop: the update-window mode's windows in one co-resident launch (a
 // bounded barrier per window); cudaErrorCooperativeLaunchTooLarge when the
 // CTAs cannot all be resident.

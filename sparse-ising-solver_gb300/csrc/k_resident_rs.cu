@@ -527,7 +527,7 @@ cudaError_t launch_rs_t(const DevCsr &J, const RsP &P, size_t smem, cudaStream_t
 
 }  // namespace
 
-int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced)
+int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced, bool tile)
 {
     const bool half = d.prec == P_BF16 || d.prec == P_F16;
     if (!half && (forced || d.prec != P_F32)) return 0;
@@ -537,7 +537,11 @@ int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced)
     const int64_t budget = (int64_t)dev_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024;
     // asked for: the rows that four a thread in registers and shared memory
     // hold (what the entry point has always taken)
-    if (forced) return std::max<int64_t>(0, d.n - 4096) * 32 + d.n * 3 <= budget ? 8 : 0;
+    const int held = std::max<int64_t>(0, d.n - 4096) * 32 + d.n * 3 <= budget ? 8 : 0;
+    if (forced) return held;
+    // a streaming tile asked for without a kernel: 16-bit state whose agents
+    // fill half the SMs has always stayed on chip, the rest streamed with it
+    if (tile) return half && (d.A + 7) / 8 >= nsm / 2 ? held : 0;
     const int ka = half ? 8 : 4;
     if ((int64_t)rs_smem(d.n) > budget) return 0;
     // Chosen by itself where its step (microseconds) is the shorter one.  Both

@@ -56,3 +56,28 @@ def test_edges_of_slices_rounds_and_clusters(ctx, prec, agents, pm1):
 def test_rows_past_the_complemented_planes(ctx, prec):
     gs = past_16383()
     check(ctx, gs, [64] * len(gs), prec, [0, 7])
+
+
+@pytest.mark.parametrize("threads", [0, 512, 640, 1024])
+def test_low_degree_with_a_cta_size(ctx, threads):
+    # a CTA size of the plane kernel is taken, also by a low-degree class
+    gs = [sbx.gen_torus(20 + i, 30, seed=i + 1) for i in range(6)]
+    probs = [ctx.problem(g) for g in gs]
+    base = dict(dt=0.5, steps=1000, run_steps=100, seed=3, precision=sbx.BF16)
+    _, want, _ = ctx.solve_batch(probs, [64] * 6, sbx.params(kernel=sbx.KERNEL_STREAM, **base))
+    _, got, _ = ctx.solve_batch(probs, [64] * 6, sbx.params(block_threads=threads, **base))
+    np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("prec", [sbx.F32, sbx.BF16])
+def test_streaming_tile_without_a_kernel(ctx, prec):
+    # agents that fill few SMs: a tile asked for is run, one that no kernel has is refused
+    g = sbx.gen_torus(80, 90, seed=2)
+    p = ctx.problem(g)
+    base = dict(dt=0.5, steps=1000, run_steps=100, agents=256, seed=3, precision=prec)
+    res, got = ctx.solve(p, sbx.params(lane_agents=2, **base))
+    assert res["lane_agents"] == 2
+    _, want = ctx.solve(p, sbx.params(**base))
+    np.testing.assert_array_equal(got, want)
+    with pytest.raises(sbx.SbxError):
+        ctx.solve(p, sbx.params(lane_agents=3, **base))
