@@ -962,7 +962,9 @@ def run_batch(args, wl, rank, world, local):
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": tr[0] if tr else None,
                 "traffic_source": tr[1] if tr else None, "peak_kind": peak_kind,
-                "kernel": "step kernel, one launch per SB step over all instances",
+                "kernel": ("k_batch_res (the whole solve in up to four launches; state on chip, "
+                           "effective bytes of one SB step)") if rp[0]["staging"] == 3 else
+                          "step kernel, one launch per SB step over all instances",
                 "bytes_per_launch": b_step, "launch_us": per_launch_s * 1e6,
                 "launches": rp[0]["kernel_launches"]}
     # the same instances in FP16 state, and in FP32 from other seeds (the

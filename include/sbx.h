@@ -45,8 +45,10 @@ extern "C" {
 enum { SBX_F32 = 0, SBX_BF16 = 1, SBX_F16 = 2, SBX_F64 = 3 };
 /* kernel family: chosen by shape (AUTO) or forced.  RESIDENT keeps a CTA's
  * agents in shared memory; RESIDENT_SPLIT (MaxCut, fused, 16-bit state) keeps
- * 8 agents per CTA split between registers and shared memory, for graphs too
- * large for the former.  TENSOR (TSP, 16-bit state, 3 <= N <= 32) is the
+ * 8 agents per CTA split between tensor memory and shared memory, for graphs
+ * too large for the former (AUTO also takes it for FP32 state, 4 agents).  For
+ * batches, RESIDENT and RESIDENT_SPLIT ask for the resident batch kernel; AUTO
+ * may take the on-chip one, which a result shows as staging 3.  TENSOR (TSP, 16-bit state, 3 <= N <= 32) is the
  * resident TSP kernel with the distance product on the tensor cores
  * (tcgen05): AUTO's choice for BF16 and FP16 TSP states that fit it. */
 enum { SBX_KERNEL_AUTO = 0, SBX_KERNEL_STREAM = 1, SBX_KERNEL_RESIDENT = 2, SBX_KERNEL_RESIDENT_SPLIT = 3,
@@ -90,7 +92,8 @@ typedef struct sbx_params {
      * tile computes identical results. */
     int32_t lane_agents;    /* agents per lane: 1, 2, 4 or 8 (16-bit states) */
     int32_t row_lanes;      /* lanes per row: 32, or 16/8/4 (several rows per
-                               warp; then lane_agents * row_lanes = padded agents) */
+                               warp; then lane_agents * row_lanes = padded agents).
+                               With 32 the last lanes of a row may hold no agents */
     int32_t block_threads;  /* threads per CTA: 128 or 256 */
     int32_t count_mode;     /* +-1 weights: 1 byte counters per lane, 2 bit
                                planes per sign word (neighbours split across
@@ -102,7 +105,8 @@ typedef struct sbx_params {
                                shared memory, a lane per 32-agent word --
                                block_threads 512, 640 (default) or 1024
                                sets its CTA size;
-                               0: autotuned (batches that fit take 4) */
+                               0: autotuned (batches that fit run on chip, or
+                               take 4) */
     int32_t staging;        /* state larger than L2, whole-warp rows: 1 direct
                                loads, 2 rows copied ahead into shared memory
                                (bulk asynchronous copies); 0: autotuned */
@@ -120,13 +124,15 @@ typedef struct sbx_result {
     int64_t bifurcated;     /* agents whose bifurcated flag is set */
     int64_t valid;          /* TSP: agents holding a valid tour */
     int32_t best_agent;     /* first agent reaching max (MaxCut) / min (TSP) */
-    int32_t kernel_used;    /* SBX_KERNEL_STREAM or SBX_KERNEL_RESIDENT */
+    int32_t kernel_used;    /* the SBX_KERNEL_* that ran */
     int32_t agents_per_block;
-    int32_t lane_agents;    /* streaming tile used (0 for other kernels) */
+    int32_t lane_agents;    /* streaming tile used (0 for other kernels; the
+                               on-chip batch kernel: agents of a cluster) */
     int32_t row_lanes;
     int32_t block_threads;
-    int32_t count_mode;
-    int32_t staging;
+    int32_t count_mode;     /* as above; the batch kernels report 4 */
+    int32_t staging;        /* as above; 3: a batch's state stayed on chip for
+                               the whole solve */
     double kernel_ms;       /* SBX_FLAG_PROFILE: summed hot-kernel time */
     int64_t kernel_launches;/* hot-kernel launches issued by the solve */
     int64_t gpu_launches;   /* all kernel launches issued by the solve */

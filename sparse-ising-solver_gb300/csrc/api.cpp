@@ -628,9 +628,9 @@ int pick_tile(sbx_ctx *ctx, SolveDims &d, const DevCsr &J, const sbx_params *pr,
     Work &w = ctx->w;
     // Every candidate over an eighth of 2 ms of launches, then those within a
     // quarter of the fastest over 2 ms, best of two rounds: most of the up to
-    // 24 candidates are far off, and timing all of them three times as long
-    // was most of a first solve (R-MAT 2^16 x 256, 1,000 steps: 176 ms, now
-    // 46; 20,000 rows x 200 in FP32: 75, now 29; the same tiles chosen).
+    // 24 candidates are far off, and timing all of them at length was most of
+    // a first solve (R-MAT 2^16 x 256, 1,000 steps: 176 ms, now 46; 20,000
+    // rows x 200 in FP32: 75, now 29; the same tiles chosen).
     CK(launch_plain_steps(d, J, w, 1, s));
     CK(cudaEventRecord(ctx->ev0, s));
     CK(launch_plain_steps(d, J, w, 1, s));
