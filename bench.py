@@ -77,16 +77,17 @@ def restart_copies(rows_missed, rows_total):
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of
 # each workload's dominant kernel, from one ncu capture of the same kernel
-# and tile (the command is in the source string); the resident kernels'
-# launch covers the whole solve.
+# (the command is in the source string); the resident kernels' launch covers
+# the whole solve.
 TRAFFIC = {
-    "torus": (45.85e6, "ncu --set full -k regex:k_resident_rs -c 1: bench.py --workload torus "
-                       "--profile 20000 --kernel split (one 20,000-step launch)"),
+    "torus": (43.17e6, "ncu -k regex:k_resident_rs -c 1: bench.py --workload torus "
+                       "--profile 2000 --kernel split (one 2,000-step launch)"),
     # per SB step: the k_row launch plus 1/100 of the isolated rows' k_iso
-    "rmat20": (9.814e8, "ncu --set full -k regex:k_row|k_iso: bench.py --workload rmat20 "
+    "rmat20": (9.792e8, "ncu -k regex:k_row|k_iso: bench.py --workload rmat20 "
                         "--profile 100 (k_row launch + k_iso / 100)"),
-    "batch512": (1.0662e9, "ncu --set full -k regex:k_bsm -s 4 -c 1: bench.py --workload batch512 "
-                           "--profile 100 (one k_bsm launch)"),
+    # the state is read and written once a solve: per step of a solve of 100
+    "batch512": (8.80e6, "ncu -k regex:k_batch_res -c 4: bench.py --workload batch512 "
+                         "--profile 100 (the four launches / 100 steps)"),
     # the whole 2,000-step solve is one launch; per launch of the bench's
     # 20,000-step solve the state read once is the same
     "tsp30": (3.870e6, "ncu --set full -k regex:k_tsp_tc -c 1: bench.py --workload tsp30 "
