@@ -824,31 +824,44 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
     };
 
     // Light rows (at most kLight neighbours): one record of eight words a row
-    // -- row, degree, columns -- loaded an item ahead, so that a row's x, y and
-    // all its sign words are requested at once.  Through the order, the row
-    // pointers and the columns it is four dependent loads, and rows of two
-    // neighbours (most of R-MAT's) took three times their bytes' time.
+    // -- row, degree, columns -- loaded two items ahead and its x, y one ahead,
+    // so that a row's state and all its sign words are requested at once.
+    // Through the order, the row pointers and the columns it is four dependent
+    // loads, and rows of two neighbours (most of R-MAT's) took three times
+    // their bytes' time.  An item is a segment of a row, as below (whole rows a
+    // warp left a small graph's many segments to as few warps as it has light
+    // rows: a star of 300 rows at 1,024 agents, FP64, 22.6 us a step).
     if constexpr (WM == W_UNIT && LR == 32 && !ST && KIND != K_XY) {
         // from the last warp down: the row items' remainder is the first warps'
-        int32_t g = (int32_t)(nw - 1 - w0), it = 0;
-        const int32_t nw32 = (int32_t)nw, nl = P.nlight;
+        const int32_t nl = P.nlight, dg = (int32_t)(nw / nit), di = (int32_t)nw - dg * nit;
+        int32_t g = (int32_t)(nw - 1 - w0) / nit, it = (int32_t)(nw - 1 - w0) - g * nit;
+        auto advance = [&](int32_t &gg, int32_t &ii) {
+            gg += dg;
+            ii += di;
+            if (ii >= nit) {
+                ii -= nit;
+                gg++;
+            }
+        };
         auto record = [&](int32_t i) { return i < nl ? __ldg(&P.light[(int64_t)i * 8 + (lane & 7)]) : 0u; };
-        // x, y of segment i of a record's row, one item ahead of their use
+        // x, y of segment i of a record's row
         auto state = [&](uint32_t rec, int i, RawT &xr, RawT &yr) {
             const int a1 = i * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
             const int64_t base = (int64_t)__shfl_sync(FULL, rec, 0) * P.Ap + a0;
             xr = vload_s<T, V>(xp + base, cs);
             yr = vload_s<T, V>(yp + base, cs);
         };
-        uint32_t rec = record(g), rec1 = record(g + nw32), rec2;
+        int32_t g1 = g, it1 = it;
+        advance(g1, it1);
+        uint32_t rec = record(g), rec1 = record(g1);
         RawT xr, yr;
-        if (g < nl) state(rec, 0, xr, yr);
+        if (g < nl) state(rec, it, xr, yr);
         while (g < nl) {
-            const bool end = it + 1 == nit;   // warp-uniform
-            const bool more = !end || g + nw32 < nl;
-            if (end) rec2 = record(g + 2 * nw32);
+            int32_t g2 = g1, it2 = it1;
+            advance(g2, it2);
+            const uint32_t rec2 = record(g2);
             RawT xn = xr, yn = yr;
-            if (more) state(end ? rec1 : rec, end ? 0 : it + 1, xn, yn);
+            if (g1 < nl) state(rec1, it1, xn, yn);
             const int32_t r = (int32_t)__shfl_sync(FULL, rec, 0), deg = (int32_t)__shfl_sync(FULL, rec, 1);
             const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
             const int q = a0 >> 5, off = a0 & 31;
@@ -874,14 +887,12 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             finish(r, q, off, base, !RAG || a1 == a0, xr, yr, tv, row_c0(r), wp_old);
             xr = xn;
             yr = yn;
-            if (end) {
-                g += nw32;
-                rec = rec1;
-                rec1 = rec2;
-                it = 0;
-            } else {
-                it++;
-            }
+            rec = rec1;
+            rec1 = rec2;
+            g = g1;
+            it = it1;
+            g1 = g2;
+            it1 = it2;
         }
     }
 
