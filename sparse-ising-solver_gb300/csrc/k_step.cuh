@@ -316,7 +316,12 @@ __device__ __forceinline__ void count_unit(const StepP &P, const uint32_t *Sq, i
 // then summed across the group (butterfly of shuffles and bit-sliced adds)
 // and each lane takes out its V agents as byte counters holding 2 * count,
 // the form count_unit leaves.  Counts stay below 128 (kHeavy = 127).
-template <int V, int LR, bool NEG>
+// AHEAD: a block's column words are loaded before the block before it is
+// counted: the heavy-row kernels (R-MAT 2^20 x 256 agents 310 -> 302 us a step)
+// and rows sharing a warp (6,000 rows of degree 24 at 32 agents, FP32: 3.43 us a
+// step, 3.65 without); whole-warp rows without heavy ones lose a CTA's worth of
+// registers to it (the same rows at 256 agents: 7.3 us, 6.7 without).
+template <int V, int LR, bool NEG, bool AHEAD>
 __device__ __forceinline__ void count_bits_s(const StepP &P, const uint32_t *Sq, int off, int32_t e0,
                                              int32_t dw, int sl, uint32_t &lo, uint32_t &hi)
 {
@@ -339,18 +344,23 @@ __device__ __forceinline__ void count_bits_s(const StepP &P, const uint32_t *Sq,
     constexpr int KPL = LR / G;    // neighbours per lane per column word
     const uint32_t *cwp = P.colw + e0 + sl;   // this lane's column words, from one base
     // past a row's end: the zero row (word 0, weight sign clear), so those
-    // terms vanish without a test per word.  The next block's column words are
-    // on their way while this one's sign words are gathered.
-    uint32_t nextcw[T];
+    // terms vanish without a test per word
+    auto columns = [&](int32_t cb, uint32_t (&cw)[T]) {
 #pragma unroll
-    for (int t = 0; t < T; t++) nextcw[t] = t * LR + sl < dw ? __ldg(cwp + t * LR) : P.zrow;
+        for (int t = 0; t < T; t++) cw[t] = cb + t * LR + sl < dw ? __ldg(cwp + cb + t * LR) : P.zrow;
+    };
+    uint32_t nextcw[T];
+    if (AHEAD) columns(0, nextcw);
     for (int32_t cb = 0; cb < dmax; cb += 32) {
         uint32_t mycw[T];
+        if (AHEAD) {
+            // the next block's column words are on their way while this one's
+            // sign words are gathered
 #pragma unroll
-        for (int t = 0; t < T; t++) {
-            mycw[t] = nextcw[t];
-            const int32_t idx = cb + 32 + t * LR + sl;
-            nextcw[t] = idx < dw ? __ldg(cwp + cb + 32 + t * LR) : P.zrow;
+            for (int t = 0; t < T; t++) mycw[t] = nextcw[t];
+            columns(cb + 32, nextcw);
+        } else {
+            columns(cb, mycw);
         }
         uint32_t w[T * KPL];
 #pragma unroll
@@ -457,12 +467,12 @@ __device__ __forceinline__ void count_bits_s(const StepP &P, const uint32_t *Sq,
         }
     }
 }
-template <int V, int LR>
+template <int V, int LR, bool AHEAD>
 __device__ __forceinline__ void count_bits(const StepP &P, const uint32_t *Sq, int off, int32_t e0,
                                            int32_t dw, int sl, uint32_t &lo, uint32_t &hi)
 {
-    if (P.allpos) count_bits_s<V, LR, false>(P, Sq, off, e0, dw, sl, lo, hi);
-    else count_bits_s<V, LR, true>(P, Sq, off, e0, dw, sl, lo, hi);
+    if (P.allpos) count_bits_s<V, LR, false, AHEAD>(P, Sq, off, e0, dw, sl, lo, hi);
+    else count_bits_s<V, LR, true, AHEAD>(P, Sq, off, e0, dw, sl, lo, hi);
 }
 
 // The SB update of V agents from their totals (the force sum_j J_ij s_j):
@@ -666,13 +676,17 @@ template <int V> __device__ __forceinline__ uint32_t sign_bits16(const uint32_t 
 // registers), 5 otherwise (heavy-row kernels: 6 spilled more and ran 2%
 // slower on R-MAT 2^20, 7 ran 11% slower).
 // RAG: the lanes of a row's last segment hold more agents than the row has.
-template <class T, int V, int KIND, bool WIN, int WM, bool BIG, int LR, int CM, int ST, bool RAG>
+// LT: light rows are walked by their records; a variant of its own because
+// their loop costs the others registers (FP32, four agents a lane, bit planes:
+// 64 against 56, 5 to 10% of a step at degree 12 to 24).
+template <class T, int V, int KIND, bool WIN, int WM, bool BIG, int LR, int CM, int ST, bool RAG, bool LT>
 __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P, const int offset)
 {
     static_assert(LR == 32 || !BIG, "heavy rows are counted by whole warps");
     static_assert(!ST || (LR == 32 && !WIN && KIND != K_XY), "staged rows: whole-warp rows, plain steps");
     static_assert(LR * V >= 32, "a sign word belongs to one row's lanes");
     static_assert(!RAG || (!ST && KIND != K_XY), "left-over lanes: direct steps");
+    static_assert(!LT || (WM == W_UNIT && LR == 32 && !ST && KIND != K_XY), "light rows: whole-warp +-1 rows");
     using A = typename St<T>::A;
     using R = typename std::conditional<WM == W_F64, double, float>::type;
     using RawT = Raw<V * sizeof(T)>;
@@ -777,7 +791,7 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
             const int q = a0 >> 5, off = a0 & 31;
             uint32_t lo = 0, hi = 0;
-            count_bits<V, 32>(P, Scur + q, off, e0, min(re - e0, (int32_t)kHeavy), lane, lo, hi);
+            count_bits<V, 32, BIG>(P, Scur + q, off, e0, min(re - e0, (int32_t)kHeavy), lane, lo, hi);
             P.part[item * 32 + lane] = make_uint2(lo, hi);
             // publish the partial, then count the row's finished chunks
             __threadfence();
@@ -831,7 +845,7 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
     // their bytes' time.  An item is a segment of a row, as below (whole rows a
     // warp left a small graph's many segments to as few warps as it has light
     // rows: a star of 300 rows at 1,024 agents, FP64, 22.6 us a step).
-    if constexpr (WM == W_UNIT && LR == 32 && !ST && KIND != K_XY) {
+    if constexpr (LT) {
         // from the last warp down: the row items' remainder is the first warps'
         const int32_t nl = P.nlight, dg = (int32_t)(nw / nit), di = (int32_t)nw - dg * nit;
         int32_t g = (int32_t)(nw - 1 - w0) / nit, it = (int32_t)(nw - 1 - w0) - g * nit;
@@ -910,10 +924,10 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             if (WM == W_UNIT) {
                 uint32_t lo = 0, hi = 0;
                 if (CM) {
-                    count_bits<V, LR>(P, Scur + q, off, e0, deg, sl, lo, hi);
+                    count_bits<V, LR, BIG || LR < 32>(P, Scur + q, off, e0, deg, sl, lo, hi);
                 } else if constexpr (BIG) {
                     // one row per warp: the choice is warp-uniform
-                    if (deg >= P.bits_min) count_bits<V, LR>(P, Scur + q, off, e0, deg, sl, lo, hi);
+                    if (deg >= P.bits_min) count_bits<V, LR, BIG || LR < 32>(P, Scur + q, off, e0, deg, sl, lo, hi);
                     else count_unit<V, LR>(P, Scur + q, off, e0, deg, sl, lo, hi);
                 } else {
                     count_unit<V, LR>(P, Scur + q, off, e0, deg, sl, lo, hi);
@@ -1126,9 +1140,14 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
     }
     // isolated rows (P.niso, left to k_iso) are the end of the degree order
     if (P.niso && !Q.order) return cudaErrorInvalidValue;
-    // light rows by their records, where they end the row items
+    // light rows by their records, where they end the row items: in the
+    // heavy-row kernels, and in the others when they are at least half of the
+    // rows (20,000 rows of mean degree 8, 31% of them light, 128 agents: 10.5 us
+    // a step by records, 9.7 without; 30,000 of degree 3, nearly all light:
+    // 11.0 against 11.6)
     const bool stage = LR == 32 && !WIN && KIND != K_XY && !RAG && d.tst != 0 && J.unit;
-    if (LR == 32 && KIND != K_XY && J.unit && J.light && Q.order && P.niso == J.niso && !stage) {
+    if (LR == 32 && KIND != K_XY && J.unit && J.light && Q.order && P.niso == J.niso && !stage &&
+        (big || 2 * (int64_t)J.nlight >= d.n - J.niso)) {
         Q.light = J.light;
         Q.nlight = J.nlight;
     }
@@ -1145,33 +1164,38 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
         if (big) {
             if constexpr (can_st) {
                 if (st) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 1, false>, d, items, bt, smem_st, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1, false>, d, items, bt, smem_st, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
-            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG>, d, items, bt, smem, s, Q, offset);
-            return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
+            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG, KIND != K_XY>, d, items, bt, smem, s, Q, offset);
+            return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, RAG, KIND != K_XY>, d, items, bt, smem, s, Q, offset);
         }
     } else {
         if (big) return cudaErrorInvalidValue;
     }
-    if (KIND == K_XY) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
+    if (KIND == K_XY) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
     if (J.unit) {
         if constexpr (KIND != K_XY) {
             if constexpr (can_st) {
                 if (st) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 1, false>, d, items, bt, smem_st, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 1, false>, d, items, bt, smem_st, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
-            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 0, RAG>, d, items, bt, smem, s, Q, offset);
+            if constexpr (LR == 32)
+                if (Q.nlight) {
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, 32, 1, 0, RAG, true>, d, items, bt, smem, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, 32, 0, 0, RAG, true>, d, items, bt, smem, s, Q, offset);
+                }
+            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
         }
-        return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
     }
     if constexpr (sizeof(T) == 8)
-        return launch_grid(k_row<T, V, KIND, WIN, W_F64, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_F64, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
     else
-        return launch_grid(k_row<T, V, KIND, WIN, W_F32, false, LR, 0, 0, RAG>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_F32, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
 }
 
 template <class T, int V, int LR, int KIND, bool WIN>

@@ -40,6 +40,25 @@ def test_segments_of_light_rows(ctx, prec, lanes, n, segments):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("prec", [sbx.F64, sbx.F32, sbx.F16])
+@pytest.mark.parametrize("degree", [1.0, 3.0, 6.5, 9.0])
+@pytest.mark.parametrize("fused", [1, 0])
+@pytest.mark.parametrize("agents", [32, 256, 300])
+def test_records_by_the_share_of_light_rows(ctx, prec, degree, fused, agents):
+    # no heavy row: records where at least half of the rows are light (here up
+    # to a mean degree of about 6.5), the row pointers otherwise
+    g = sbx.gen_er(2500, degree / 2499, pm1=True, seed=int(10 * degree))
+    prob = ctx.problem(g)
+    base = dict(dt=0.5, steps=2000, run_steps=200, agents=agents, seed=5, precision=prec, fused=fused,
+                kernel=sbx.KERNEL_STREAM)
+    out = []
+    for tile in ({}, dict(lane_agents=1, row_lanes=32)):
+        _, cut = ctx.solve(prob, sbx.params(**tile, **base))
+        out.append((cut,) + ctx.state(g.n, agents))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_many_segments_fill_the_gpu(ctx):
     # 300 rows of 16 segments: 1.2 times the time of rows that have no records;
     # whole rows a warp took 2.9 times
