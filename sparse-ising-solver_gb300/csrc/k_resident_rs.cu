@@ -544,22 +544,37 @@ int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced, bool tile
     if (tile) return half && (d.A + 7) / 8 >= nsm / 2 ? held : 0;
     const int ka = half ? 8 : 4;
     if ((int64_t)rs_smem(d.n) > budget) return 0;
-    // Chosen by itself where its step (microseconds) is the shorter one.  Both
-    // sides fitted on GB300 over 5,900 to 9,900 rows, 200 to 1,024 agents and
-    // mean degrees 4 to 40: waves of one CTA an SM, each a cost per row that
-    // grows with the degree (FP32: 0.83 ns at degree 4, 1.65 at 16, 2.9 at
-    // 40), against the streaming step's cost per row and agent (FP32 2.1 to
-    // 3.2 ps, 16 bits 1.45 to 2.45) and its latency.  E.g. 6,000 rows, FP32,
-    // 1,024 agents: 9.8 us a step against 16.1 at degree 4, 24.8 against 21.1
-    // at degree 24.
+    // Chosen by itself where its step is clearly the shorter one (by 5%, the
+    // fits' error).  Both sides fitted on GB300 (mean error 3 to 10%) on 13
+    // graphs each of 3,136 to 14,000 rows (16 bits: 5,400 to 14,000) and mean
+    // degrees 2 to 85, +-1 and real weights apart, at 32 to 2,000 agents.  A
+    // wave of one CTA an SM has a fixed time and one per row and neighbour, and
+    // rows past tensor memory's cost more; the streaming step has a fixed time
+    // and one per row and agent, the agents as its tile holds them.  E.g. FP32
+    // (us a step, resident against streaming): 5,929 rows of degree 4 at 32
+    // agents 4.5 against 2.7, at 1,024 9.2 against 16.8; 3,136 of degree 8 at 32
+    // agents 4.1 against 2.9; 12,500 of degree 16, real weights, at 480 agents
+    // 25 against 43; at degree 85, 256 agents 105 against 83.
+    struct Fit {
+        double wave, row4, row, nbr, past;     // us; ns per row (up to degree 4), per row, per neighbour, past 8,192
+        double step, cell4, cell, cell_nbr;    // us; ps per row and agent (up to degree 4), ..., per neighbour
+    };
+    static const Fit kFit[2][2] = {
+        {{1.0, 0.61, 0.65, 0.043, 0.32, 2.65, 2.2, 2.65, 0.025}, {1.2, 0, 0.35, 0.094, 0.30, 3.9, 0, 1.75, 0.27}},
+        {{1.25, 0.77, 0.86, 0.041, 0.28, 2.9, 1.23, 1.5, 0.02}, {2.2, 0, 0.52, 0.122, 0.36, 4.7, 0, 0.73, 0.19}},
+    };
+    const Fit &f = kFit[half][!J.unit];
     const double n = (double)d.n, deg = (double)J.nnz / n;
+    const bool low = J.unit && deg <= 4;   // one block of four neighbours a row
     const double waves = (double)(((d.A + ka - 1) / ka + nsm - 1) / nsm);
-    const double per_row = half ? (deg <= 4 ? 1.0 : 1.1 + 0.047 * deg) : (deg <= 4 ? 0.83 : 0.86 + 0.051 * deg);
-    const double more = deg > 24 ? deg - 24 : 0;
-    const double per_cell = half ? (deg <= 4 ? 1.45 : 2.0 + 0.03 * more) : (deg <= 4 ? 2.1 : 2.65 + 0.035 * more);
-    const double res = waves * (n * per_row * 1e-3 + 0.3);
-    const double str = (half ? 3.0 : 4.0) + n * ((d.A + 127) / 128 * 128) * per_cell * 1e-6;
-    return res < str ? ka : 0;
+    const int most = half ? 256 : 128;     // agents of a whole-warp row's widest vectors
+    int held_agents = 32;
+    while (held_agents < most && held_agents < d.Ap) held_agents *= 2;
+    if (d.Ap > most) held_agents = (d.Ap + most - 1) / most * most;
+    const double res = waves * (f.wave + 1e-3 * (n * (low ? f.row4 : f.row + f.nbr * deg) +
+                                                 std::max(0.0, n - kTmRows * kNT) * f.past));
+    const double str = f.step + 1e-6 * n * held_agents * (low ? f.cell4 : f.cell + f.cell_nbr * deg);
+    return 1.05 * res < str ? ka : 0;
 }
 
 cudaError_t launch_resident_rs(const SolveDims &d, const DevCsr &J, Work &w, int ka, int32_t step0,
