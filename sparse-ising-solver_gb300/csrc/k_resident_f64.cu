@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(1024) k_res64(const R64P P)
 }
 
 size_t smem64(int64_t n) { return (size_t)n * 19 + 2; }
+int threads64(int64_t n) { return (int)std::min<int64_t>(1024, std::max<int64_t>(64, (n + 31) / 32 * 32)); }
 
 }  // namespace
 
@@ -184,13 +185,21 @@ bool resident64_pick(const SolveDims &d, const DevCsr &J)
 {
     if (d.prec != P_F64 || !J.unit || J.n > 32767) return false;
     if (smem64(d.n) + 1024 > (size_t)dev_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin)) return false;
-    // The shorter step (microseconds, both sides fitted on GB300 over 100 to
-    // 3,000 rows and 33 to 1,024 agents): an SM's agents one after another
-    // through its FP64 pipe against a launch and the whole GPU's.  300 rows: 1.7
-    // against 3.2 at 128 agents, 8.8 against 7.4 at 1,024.
+    // The shorter step (microseconds, both sides fitted on GB300, mean error 11%,
+    // over 50 to 6,000 rows, mean degrees 2 to 900, stars and R-MAT, and 1 to
+    // 1,024 agents): an SM's agents one after another through its FP64 pipe, and
+    // its CTAs' walks over the neighbours, where one thread walks the longest
+    // row, against a launch, the whole GPU's FP64 pipes and 32 agents a gathered
+    // word, heavy rows in chunks.  300 rows of degree 12: 1.8 against 3.3 at 128
+    // agents, 8.9 against 7.6 at 1,024; 128 agents and 1,000 rows of degree 900:
+    // 34.5 against 19.6; a star of 1,000: 10.2 against 7.7.
     const double nsm = std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
-    const double waves = std::ceil(d.A / nsm);
-    return 0.75 + 3.7e-3 * (double)d.n * waves < 2.4 + 17e-6 * (double)d.n * d.Ap;
+    const double n = (double)d.n, deg = (double)J.nnz / n, more = std::max(0.0, deg - 12);
+    const double waves = std::ceil(d.A / nsm), together = std::max(1, 1024 / threads64(d.n));   // CTAs of an SM
+    const double walk = more / 4 * std::max(0.04, 0.13e-3 * n) + 6e-3 * ((double)J.max_deg - deg);
+    return 0.75 + 3.7e-3 * n * waves + std::ceil(waves / together) * walk <
+           2.4 + 17e-6 * n * d.Ap + more * (0.08e-6 * n * d.Ap) + std::min(more, kHeavy - 12.0) * 7e-3 +
+               (J.max_deg > kHeavy ? 3.3 : 0.0);
 }
 
 cudaError_t launch_resident64(const SolveDims &d, const DevCsr &J, Work &w, int32_t step0, int32_t nsteps, bool first,
@@ -227,8 +236,7 @@ cudaError_t launch_resident64(const SolveDims &d, const DevCsr &J, Work &w, int3
     const size_t smem = smem64(d.n);
     cudaError_t e = cudaFuncSetAttribute(k_res64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int threads = (int)std::min<int64_t>(1024, std::max<int64_t>(64, (d.n + 31) / 32 * 32));
-    return launch(k_res64, dim3((unsigned)d.A), dim3((unsigned)threads), smem, s, d.pdl, P);
+    return launch(k_res64, dim3((unsigned)d.A), dim3((unsigned)threads64(d.n)), smem, s, d.pdl, P);
 }
 
 }  // namespace sbx
