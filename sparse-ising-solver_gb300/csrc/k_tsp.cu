@@ -26,6 +26,8 @@
 #include "common.cuh"
 #include "engine.h"
 
+#include <algorithm>
+
 namespace sbx {
 
 namespace {
@@ -132,9 +134,17 @@ __global__ void __launch_bounds__(H == 1 ? 512 : 1024) k_tsp_resident(const TspP
         prv = P.prev[ag];
     }
     __syncthreads();
-    float i2r[CPT];   // the linear field of this thread's cities
+    // the linear field of this thread's cities (all 32: from shared memory where
+    // it is used, their registers are spent)
+    [[maybe_unused]] float i2r[CPT > 8 ? 1 : CPT];
+    if constexpr (CPT <= 8) {
 #pragma unroll
-    for (int j = 0; j < CPT; j++) i2r[j] = s_I2[k0 + j];
+        for (int j = 0; j < CPT; j++) i2r[j] = s_I2[k0 + j];
+    }
+    auto field = [&](int j) {
+        if constexpr (CPT <= 8) return i2r[j];
+        else return s_I2[k0 + j];
+    };
 
     const bool whole = k0 + CPT <= N;   // warp-uniform: no city past N
     // the parts that sum this row and its column: another for the next warp
@@ -200,7 +210,7 @@ __global__ void __launch_bounds__(H == 1 ? 512 : 1024) k_tsp_resident(const TspP
                                                      __ffma2_rn(qc, cs2, __fmul2_rn(qb, rs2)));
                         const float2 i1 = __fmul2_rn(m1005, jx);
                         const float2 x0 = make_float2(xo[q], xo[q + 1]), y0 = make_float2(yr[q], yr[q + 1]);
-                        float2 y = __ffma2_rn(cxi, __ffma2_rn(bt, make_float2(i2r[q], i2r[q + 1]),
+                        float2 y = __ffma2_rn(cxi, __ffma2_rn(bt, make_float2(field(q), field(q + 1)),
                                                               __fmul2_rn(two, i1)), y0);
                         y = make_float2(rnd<T>(y.x), rnd<T>(y.y));
                         float2 x = __ffma2_rn(cdt, y, x0);
@@ -324,18 +334,15 @@ cudaError_t launch_res(const TspP &P, const DevTsp &t, int ka, cudaStream_t s, b
     return cudaLaunchKernelEx(&cfg, k_tsp_resident<T, NP, H>, P, D, ka);
 }
 
-// Eight cities a thread (four parts of 32, two of 16) where the CTA's threads
-// allow it; more agents a CTA (only when asked for) take fewer parts.
+// Eight cities a thread: two parts of 16, whose rows always fit, and four of 32
+// where the CTA's 1,024 threads allow it; more agents a CTA (only when asked
+// for) take whole rows (17 cities, 30 agents a CTA: 5.6 us a step, two parts of
+// 16 cities 6.3 to 6.9).
 template <class T>
 cudaError_t launch_np(const TspP &P, const DevTsp &t, int ka, cudaStream_t s, bool pdl)
 {
-    const int R = part_threads(P.N, ka);
-    if (P.N <= 16) {
-        if (2 * R <= 1024) return launch_res<T, 16, 2>(P, t, ka, s, pdl);
-        return launch_res<T, 16, 1>(P, t, ka, s, pdl);
-    }
-    if (4 * R <= 1024) return launch_res<T, 32, 4>(P, t, ka, s, pdl);
-    if (2 * R <= 1024) return launch_res<T, 32, 2>(P, t, ka, s, pdl);
+    if (P.N <= 16) return launch_res<T, 16, 2>(P, t, ka, s, pdl);
+    if (4 * part_threads(P.N, ka) <= 1024) return launch_res<T, 32, 4>(P, t, ka, s, pdl);
     return launch_res<T, 32, 1>(P, t, ka, s, pdl);
 }
 
@@ -348,11 +355,13 @@ int tsp_pick_ka(const SolveDims &d, const DevTsp &t, int requested)
     const int kmax = 512 / t.N;   // registers: <= 512 threads of ~128 registers
     if (kmax < 1) return 0;
     if (requested > 0) return requested <= kmax ? requested : 0;
-    // one CTA an SM, as long as its rows can be split in eight-city parts
-    int ka = (d.A + nsm - 1) / nsm;
-    if (ka < 1) ka = 1;
-    while (ka > 1 && (t.N <= 16 ? 2 : 4) * part_threads(t.N, ka) > 1024) ka--;
-    return ka;
+    // one CTA an SM in as few even waves as leave its rows in eight-city parts
+    // (29 cities x 2,500 agents: three waves of six 7.9 us a step, three of the
+    // most a CTA so holds, eight, 9.9)
+    for (int waves = 1;; waves++) {
+        const int ka = std::max(1, (d.A + waves * nsm - 1) / (waves * nsm));
+        if (ka == 1 || (t.N <= 16 ? 2 : 4) * part_threads(t.N, ka) <= 1024) return ka;
+    }
 }
 
 cudaError_t launch_tsp_resident(const SolveDims &d, const DevTsp &t, Work &w, int ka,
