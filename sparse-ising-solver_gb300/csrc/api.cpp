@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <numeric>
 #include <map>
 #include <set>
@@ -1333,10 +1334,44 @@ void free_bres(DevBres &B)
     B = DevBres();
 }
 
+// Microseconds of the other steps of a batch class of +-1 weights, fitted on
+// GB300 as build_bres's (mean errors 7 to 10%): streaming, from the agents that
+// its tile holds a row; the plane kernel; and the resident batch, whose CTAs
+// hold whole bins.
+double stream_us(const BatchClass &c, const SolveDims &d)
+{
+    const bool half = prec_bytes(d.prec) == 2;
+    const double n = (double)c.J.n, deg = (double)c.J.nnz / n, cells = 1e-6 * n * tile_agents(d);
+    if (half) return 2.45 + 0.011 * deg + cells * (deg <= 4 ? 1.45 : 1.70 + 0.0176 * deg);
+    return 2.28 + 0.0113 * deg + cells * (deg <= 4 ? 2.53 : 2.87 + 0.0233 * deg);
+}
+double plane_us(const BatchClass &c, const SolveDims &d)
+{
+    const double n = (double)c.J.n, deg = (double)c.J.nnz / n;
+    return 3.26 + 0.0425 * deg + (c.probs.size() > 1 ? 1.28 : 0) + 1e-3 * n * d.W * (0.047 + 0.48e-3 * deg);
+}
+double resident_batch_us(const BatchClass &c, int64_t max_rows)
+{
+    std::vector<int64_t> ns, fill;   // first fit, as build_rb packs
+    for (const sbx_problem *q : c.probs) ns.push_back(q->J.n);
+    std::sort(ns.begin(), ns.end(), std::greater<int64_t>());
+    for (int64_t n : ns) {
+        size_t b = 0;
+        while (b < fill.size() && fill[b] + n > max_rows) b++;
+        if (b == fill.size()) fill.push_back(0);
+        fill[b] += n;
+    }
+    const int64_t nsm = std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
+    const double waves = (double)(((int64_t)fill.size() * (c.Ap / 4) + nsm - 1) / nsm);
+    const double deg = (double)c.J.nnz / (double)c.J.n;
+    return waves * (0.73 + 1e-3 * (double)*std::max_element(fill.begin(), fill.end()) * (0.52 + 0.091 * deg));
+}
+
 // Pack a class for the on-chip batch kernel; leaves bres.rows null when an
-// instance does not fit or stepping launch by launch is faster.  A bin's cluster is the smallest that holds it and,
-// when the class alone cannot fill the GPU, splits it down to an SM's share.
-int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32)
+// instance does not fit or the step that would run instead (other_us) is as
+// fast.  A bin's cluster is the smallest that holds it and, when the class
+// alone cannot fill the GPU, splits it down to an SM's share.
+int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
 {
     DevBres &B = c.bres[f32];
     free_bres(B);
@@ -1380,25 +1415,31 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32)
         bins[at].inst.push_back((int32_t)i);
         bins[at].rows += n;
     }
-    // Taken where its step is the shorter one (microseconds, both sides fitted
-    // on GB300 on 1 to 512 instances of 100 to 20,000 rows at 32, 64 and 128
-    // agents): a cluster's step is about 2 + 0.085 per slice of its CTAs at
-    // degree 24 (FP32, half the agents: 0.06), and the step per launch about 6 +
-    // 0.06 per thousand rows and 32 agents (FP32: 4 + 0.11).  One instance of
-    // 19,909 rows at 64 agents, 16 bits: 15.5 against 7.5; 32 instances, 154,000
-    // rows: 16.6 against 22.7, FP32 22.5 against 40.2.
+    // Taken where its step is clearly shorter (by 5%, the fits' error) than
+    // other_us, the step that would run instead: microseconds, fitted on GB300
+    // (mean error 9%, FP32 12%) on 950 classes of 1 to 128 instances of 100 to
+    // 15,000 rows at mean degrees 2 to 90 and 32 to 512 agents.  A CTA's step has
+    // a fixed time, one per slice of rows and neighbour, and the latency of a
+    // round's longest row; clusters that share the SMs end a quarter after their
+    // sum.  Us a step, on chip against the other: one graph of 10,000 rows at
+    // degree 10, 64 agents, 16 bits 6.4 against 5.1; 32 graphs of 4,000 to 5,000
+    // rows at degree 20, FP32, 64 agents 22.5 against 40.2.
+    struct Fit {
+        double one, cluster, slice, nbr, round;
+    };
+    static const Fit kFit[2] = {{0.40, 0.86, 0.054, 0.66e-3, 0.0168}, {0.275, 0.77, 0.040, 0.31e-3, 0.025}};
+    const Fit &f = kFit[f32];
+    const double mean_deg = (double)J.nnz / (double)J.n;
     double sum = 0, longest = 0;
     for (const Bin &b : bins) {
         const int C = batch_res_ctas(b.k);
-        int64_t nnz = 0;
-        for (int32_t i : b.inst) nnz += c.probs[(size_t)i]->J.nnz;
-        const double deg = (double)nnz / (double)b.rows;
-        const double t = 2.0 + (f32 ? 0.060 : 0.085) * (double)(((b.rows + 31) / 32 + C - 1) / C) * (0.4 + 0.6 * deg / 24);
+        const double slices = (double)(((b.rows + 31) / 32 + C - 1) / C);
+        const double t = (C == 1 ? f.one : f.cluster) + slices * (f.slice + f.nbr * mean_deg) +
+                         std::ceil(slices / 32) * f.round * mean_deg;
         sum += t * C * groups / nsm;
         longest = std::max(longest, t);
     }
-    if (std::max(longest, 1.1 * sum) > (f32 ? 4.0 : 6.0) + (f32 ? 0.11e-3 : 0.06e-3) * (double)J.n * (c.Ap / 32))
-        return SBX_OK;
+    if (1.05 * std::max(longest, 1.24 * sum) > other_us) return SBX_OK;
     std::stable_sort(bins.begin(), bins.end(),
                      [](const Bin &a, const Bin &b) { return a.k != b.k ? a.k < b.k : a.rows > b.rows; });
     const size_t nb = bins.size();
@@ -1834,9 +1875,9 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
                            (!c.J.unit || c.J.max_deg <= kHeavy) && c.J.n < (int64_t)1 << 30 && nchunks > 0;
         // Each 4-agent CTA re-reads its bin's rows every step and gathers
         // neighbour signs from shared memory, so by itself the resident batch
-        // is taken only for low-degree classes (mean degree <= 8) that neither
-        // the on-chip kernel nor the plane kernel takes (below); measured on
-        // GB300 it trails the streaming kernel at degree ~20.
+        // is taken only for low-degree classes (mean degree <= 8), and there
+        // where neither the on-chip kernel nor streaming is faster (below);
+        // measured on GB300 it trails the streaming kernel at degree ~20.
         const bool low_degree = c.J.nnz <= 8 * c.J.n;
         const bool want_rb = (pr->kernel == SBX_KERNEL_AUTO && low_degree) || pr->kernel == SBX_KERNEL_RESIDENT ||
                              pr->kernel == SBX_KERNEL_RESIDENT_SPLIT;
@@ -1865,18 +1906,24 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         bool use_res = (!use_rb || by_itself) && !tile_pinned && !bsm_threads && !pr->count_mode && pr->kernel == SBX_KERNEL_AUTO &&
                        d.prec != P_F64 && d.fused && !d.trace && nchunks > 0 && c.J.unit &&
                        c.J.max_deg <= kHeavy;
-        if (use_res) {
-            if (!bres.tried && (rc = build_bres(ctx, c, d.prec == P_F32))) return rc;
-            use_res = bres.rows != nullptr;
-            if (use_res) use_rb = false;
+        // by itself at low degree: the streaming step or the resident batch,
+        // whichever is shorter (16 bits, 64 agents, us a step: one torus of 961
+        // rows 2.5 against 1.4, 8 of 2,600 in all 2.7 against 2.8, one of 10,000
+        // 3.4 against 9.0; the plane kernel only by its CTA size)
+        const double rb_us = use_rb && by_itself ? resident_batch_us(c, rb_rows) : 0;
+        const bool rb_slower = use_rb && by_itself && c.J.unit && stream_us(c, d) < rb_us;
+        if (use_res && !bres.tried) {
+            const double other = use_rb ? std::min(rb_us, stream_us(c, d)) : use_bsm ? plane_us(c, d) : stream_us(c, d);
+            if ((rc = build_bres(ctx, c, d.prec == P_F32, other))) return rc;
         }
-        // ... else a step kernel before the resident batch, which they outrun
-        // at low degree (8 tori, 20,434 rows at 64 agents: 17.7 us a step, the
-        // plane kernel 6.3, the streaming step 4.3): the streaming step, unless
-        // a CTA size of the plane kernel is asked for
-        if (use_rb && by_itself && !tile_pinned && bsm_ok(c, d)) {
+        use_res = use_res && bres.rows != nullptr;
+        if (use_res) {
             use_rb = false;
-            use_bsm = bsm_threads;
+        } else if (use_rb && by_itself && !tile_pinned && bsm_threads && bsm_ok(c, d)) {
+            use_rb = false;
+            use_bsm = true;
+        } else if (rb_slower && !tile_pinned && !bsm_threads) {
+            use_rb = false;
         }
         c.J.bsm = nullptr;
         if (use_res) {

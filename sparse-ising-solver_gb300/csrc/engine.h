@@ -178,6 +178,17 @@ struct SolveDims {
                              // its CTA size (512 or 1024); 0: not used
 };
 
+// Agents that a row's lanes of the streaming step hold: the padded ones, up to
+// the widest whole-warp tile in a power of two (rows sharing a warp), past it in
+// whole tiles.
+inline int tile_agents(const SolveDims &d)
+{
+    const int most = prec_bytes(d.prec) == 2 ? 256 : 128;
+    int a = 32;
+    while (a < most && a < d.Ap) a *= 2;
+    return d.Ap > most ? (d.Ap + most - 1) / most * most : a;
+}
+
 // Plan of the batched step kernel with per-instance sign planes in shared
 // memory (k_batch_smem.cu): the rows cut into one contiguous run per CTA,
 // each run into segments at instance boundaries.

@@ -567,13 +567,9 @@ int resident_rs_pick(const SolveDims &d, const DevCsr &J, bool forced, bool tile
     const double n = (double)d.n, deg = (double)J.nnz / n;
     const bool low = J.unit && deg <= 4;   // one block of four neighbours a row
     const double waves = (double)(((d.A + ka - 1) / ka + nsm - 1) / nsm);
-    const int most = half ? 256 : 128;     // agents of a whole-warp row's widest vectors
-    int held_agents = 32;
-    while (held_agents < most && held_agents < d.Ap) held_agents *= 2;
-    if (d.Ap > most) held_agents = (d.Ap + most - 1) / most * most;
     const double res = waves * (f.wave + 1e-3 * (n * (low ? f.row4 : f.row + f.nbr * deg) +
                                                  std::max(0.0, n - kTmRows * kNT) * f.past));
-    const double str = f.step + 1e-6 * n * held_agents * (low ? f.cell4 : f.cell + f.cell_nbr * deg);
+    const double str = f.step + 1e-6 * n * tile_agents(d) * (low ? f.cell4 : f.cell + f.cell_nbr * deg);
     return 1.05 * res < str ? ka : 0;
 }
 
