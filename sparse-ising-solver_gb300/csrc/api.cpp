@@ -20,6 +20,7 @@
 #include <functional>
 #include <numeric>
 #include <map>
+#include <memory>
 #include <set>
 #include <string>
 #include <vector>
@@ -1171,6 +1172,14 @@ int build_class(sbx_ctx *ctx, BatchClass &c)
     return SBX_OK;
 }
 
+// Host threads that place `entries` matrix entries: 17 ns each on one core, a
+// thread's start about 70 us, so the square root of their ratio.
+int place_threads(int64_t entries)
+{
+    const int n = (int)std::sqrt((double)entries / 4096);
+    return n <= 1 ? 1 : std::min(n, host_threads());
+}
+
 // Entries of a slice's rows (row l's left[l] entries at ent + l pos) to their
 // positions in the sliced form: position j of row l at out[(j / 4) 128 + 4 l +
 // j % 4], positions not written keep the padding there.  The kernels gather the
@@ -1259,9 +1268,9 @@ int ensure_sell(sbx_ctx *ctx, DevCsr &J, DevSell &L, int scale)
     };
     for (int64_t s = 0; s < n; s++) hd[s] = (float)degree(s);
     if (J.unit) {
-        parallel(J.nnz > (1 << 16) ? std::min(host_threads(), 8) : 1, [&](int t, int TT) {
+        parallel(place_threads(J.nnz), [&](int t, int TT) {   // slices in turn: the first are the longest
             std::vector<uint16_t> ent;
-            for (int64_t k = nsl * t / TT; k < nsl * (t + 1) / TT; k++) place(k, ent);
+            for (int64_t k = t; k < nsl; k += TT) place(k, ent);
         });
     } else {
         for (int64_t s = 0; s < n; s++) {
@@ -1370,12 +1379,19 @@ double resident_batch_us(const BatchClass &c, int64_t max_rows)
 // Pack a class for the on-chip batch kernel; leaves bres.rows null when an
 // instance does not fit or the step that would run instead (other_us) is as
 // fast.  A bin's cluster is the smallest that holds it and, when the class
-// alone cannot fill the GPU, splits it down to an SM's share.
-int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
+// alone cannot fill the GPU, splits it down to an SM's share.  place: the
+// entries by bank (place_entries), which costs 15 ns each on one core and saves
+// 5 to 20% of a step: it repays itself in 700 to 3,500 steps, so a plan whose
+// solves have come to fewer than kPlaceSteps in all keeps the rows' order (24
+// graphs of 15,000 rows at degree 24: 11.0 ms and 29.7 us a step, or 5.2 ms and
+// 32.6 us).
+constexpr int64_t kPlaceSteps = 1000;
+int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us, bool place)
 {
     DevBres &B = c.bres[f32];
     free_bres(B);
     B.tried = true;
+    B.placed = place;
     const DevCsr &J = c.J;
     const size_t ni = c.probs.size();
     int64_t cap[4];
@@ -1459,10 +1475,11 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
     }
     std::vector<int32_t> off((size_t)slices, 0);
     std::vector<int64_t> blocks(nb, 0);
-    const int T = J.nnz > (1 << 18) ? host_threads() : 1;
+    const int T = place_threads(J.nnz);
+    std::vector<int32_t> inv((size_t)J.n);
     // a bin's slots: its instances' rows by decreasing degree (<= 127), ties
     // in row order; its slices' block counts
-    parallel(T, [&](int t, int TT) {
+    parallel(J.n > (1 << 15) ? T : 1, [&](int t, int TT) {
         for (size_t b = (size_t)t; b < nb; b += (size_t)TT) {
             int64_t at[129] = {0};
             auto deg = [&](int64_t r) { return J.hrowptr[(size_t)r + 1] - J.hrowptr[(size_t)r]; };
@@ -1473,6 +1490,7 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
                 for (int64_t r = c.row_off[(size_t)i], e = r + c.probs[(size_t)i]->J.n; r < e; r++) {
                     const size_t s = (size_t)slot0[b] + (size_t)at[127 - deg(r)]++;
                     perm[s] = (int32_t)r;
+                    inv[(size_t)r] = (int32_t)(s - (size_t)slot0[b]);
                     B.hinst[s] = i;
                     B.hdeg[s] = deg(r);
                 }
@@ -1491,17 +1509,22 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
         total += blocks[b];
     }
     if (total * 32 > INT32_MAX) return SBX_OK;
-    std::vector<uint16_t> col((size_t)std::max<int64_t>(total, 1) * 128);
-    std::vector<int32_t> inv((size_t)J.n);
+    const size_t ncol = (size_t)std::max<int64_t>(total, 1) * 128;
+    const std::unique_ptr<uint16_t[]> col(new uint16_t[ncol]);   // not cleared: every block is filled below
+    for (size_t b = 0; b < nb; b++)
+        for (int64_t k = 0; k <= (rows[b] + 31) / 32; k++) off[(size_t)(slice0[b] + k)] += (int32_t)first[b];
+    // the slices of all bins in turn: one bin alone keeps every thread busy
     parallel(T, [&](int t, int TT) {
-        for (size_t b = (size_t)t; b < nb; b += (size_t)TT) {
-            for (int64_t s = 0; s < rows[b]; s++) inv[(size_t)perm[(size_t)(slot0[b] + s)]] = (int32_t)s;
-            std::fill(col.begin() + (long)(first[b] * 128), col.begin() + (long)((first[b] + blocks[b]) * 128),
-                      (uint16_t)batch_res_entry(bins[b].k, f32, J.allpos, (uint32_t)rows[b], false));
-            int32_t *o = &off[(size_t)slice0[b]];
-            uint16_t ent[32 * 128];   // degree <= 127: at most 128 positions
-            int32_t left[32];
+        uint16_t ent[32 * 128];   // degree <= 127: at most 128 positions
+        int32_t left[32];
+        int64_t turn = 0;
+        for (size_t b = 0; b < nb; b++) {
+            const uint16_t none = (uint16_t)batch_res_entry(bins[b].k, f32, J.allpos, (uint32_t)rows[b], false);
+            const int32_t *o = &off[(size_t)slice0[b]];
             for (int64_t k = 0; 32 * k < rows[b]; k++) {
+                if (turn++ % TT != t) continue;
+                uint16_t *out = &col[(size_t)o[k] * 128];
+                std::fill(out, out + (size_t)(o[k + 1] - o[k]) * 128, none);
                 const int64_t pos = 4 * (o[k + 1] - o[k]);
                 const int m = (int)std::min<int64_t>(32, rows[b] - 32 * k);
                 for (int l = 0; l < m; l++) {
@@ -1512,11 +1535,16 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
                         *v++ = (uint16_t)batch_res_entry(bins[b].k, f32, J.allpos, (uint32_t)inv[(size_t)J.hcol[(size_t)e]],
                                                          J.hval[(size_t)e] < 0);
                 }
-                place_entries(ent, pos, m, left, 0xffffu, &col[(size_t)(first[b] + o[k]) * 128]);
+                if (place) {
+                    place_entries(ent, pos, m, left, 0xffffu, out);
+                    continue;
+                }
+                for (int l = 0; l < m; l++)
+                    for (int32_t j = 0; j < left[l]; j++) out[(j / 4) * 128 + 4 * l + (j & 3)] = ent[l * pos + j];
             }
-            for (int64_t k = 0; k <= (rows[b] + 31) / 32; k++) o[k] += (int32_t)first[b];
         }
     });
+    if (!total) std::fill(col.get(), col.get() + ncol, (uint16_t)0);
     auto put = [&](void **p, const void *src, size_t bytes) {
         cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
         return e == cudaSuccess && bytes ? cudaMemcpy(*p, src, bytes, cudaMemcpyHostToDevice) : e;
@@ -1525,7 +1553,7 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us)
     CK(put((void **)&B.slot0, slot0.data(), 4 * nb));
     CK(put((void **)&B.slice0, slice0.data(), 4 * nb));
     CK(put((void **)&B.off, off.data(), 4 * off.size()));
-    CK(put(&B.col, col.data(), 2 * col.size()));
+    CK(put(&B.col, col.get(), 2 * ncol));
     CK(put((void **)&B.perm, perm.data(), 4 * perm.size()));
     CK(cudaMalloc(&B.cb, sizeof(float) * 2 * std::max<int64_t>(J.n, 1)));
     CK(put((void **)&B.rows, rows.data(), 4 * nb));   // last: the plan is complete
@@ -1912,9 +1940,13 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
         // 3.4 against 9.0; the plane kernel only by its CTA size)
         const double rb_us = use_rb && by_itself ? resident_batch_us(c, rb_rows) : 0;
         const bool rb_slower = use_rb && by_itself && c.J.unit && stream_us(c, d) < rb_us;
-        if (use_res && !bres.tried) {
-            const double other = use_rb ? std::min(rb_us, stream_us(c, d)) : use_bsm ? plane_us(c, d) : stream_us(c, d);
-            if ((rc = build_bres(ctx, c, d.prec == P_F32, other))) return rc;
+        if (use_res) {
+            const int64_t steps = (bres.tried ? bres.steps : 0) + total;   // of the plan's solves, this one's too
+            if (!bres.tried || (bres.rows && !bres.placed && steps >= kPlaceSteps)) {
+                const double other = use_rb ? std::min(rb_us, stream_us(c, d)) : use_bsm ? plane_us(c, d) : stream_us(c, d);
+                if ((rc = build_bres(ctx, c, d.prec == P_F32, other, steps >= kPlaceSteps))) return rc;
+            }
+            bres.steps = steps;
         }
         use_res = use_res && bres.rows != nullptr;
         if (use_res) {

@@ -211,6 +211,8 @@ struct DevBsm {
 // of 4 for bins past 16,383 rows -- each largest first.
 struct DevBres {
     bool tried = false;          // planned (rows is null when the class does not fit)
+    bool placed = false;         // entries placed by bank
+    int64_t steps = 0;           // steps of its solves so far
     int32_t *bins = nullptr, *slot0 = nullptr, *slice0 = nullptr, *rows = nullptr, *off = nullptr;
     void *col = nullptr;         // [blocks][32] of four entries (batch_res_entry)
     void *cb = nullptr;          // per slot: dt * xi0, -degree
