@@ -65,7 +65,8 @@ enum { SBX_DIST_EUC_2D = 0, SBX_DIST_GEO = 1, SBX_DIST_EUC_2D_FLOAT = 2 };
  * its MMAs) gives up at its first check, as a wait
  * that never completes would after its limit.  The kernels flag the error,
  * let their copies in flight land and return; the solve returns SBX_ERR_CUDA
- * and the context stays usable for the next solve. */
+ * and the context stays usable for the next solve.  The on-chip batch kernel
+ * reports that its layout does not fit, and the batch takes another kernel. */
 #define SBX_FLAG_TEST_GIVEUP 16u
 
 typedef struct sbx_ctx sbx_ctx;

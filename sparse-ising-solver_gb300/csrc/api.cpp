@@ -1549,14 +1549,21 @@ int build_bres(sbx_ctx *ctx, BatchClass &c, bool f32, double other_us, bool plac
         cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
         return e == cudaSuccess && bytes ? cudaMemcpy(*p, src, bytes, cudaMemcpyHostToDevice) : e;
     };
-    CK(put((void **)&B.bins, list.data(), 4 * nb));
-    CK(put((void **)&B.slot0, slot0.data(), 4 * nb));
-    CK(put((void **)&B.slice0, slice0.data(), 4 * nb));
-    CK(put((void **)&B.off, off.data(), 4 * off.size()));
-    CK(put(&B.col, col.get(), 2 * ncol));
-    CK(put((void **)&B.perm, perm.data(), 4 * perm.size()));
-    CK(cudaMalloc(&B.cb, sizeof(float) * 2 * std::max<int64_t>(J.n, 1)));
-    CK(put((void **)&B.rows, rows.data(), 4 * nb));   // last: the plan is complete
+    cudaError_t e = put((void **)&B.bins, list.data(), 4 * nb);
+    if (e == cudaSuccess) e = put((void **)&B.slot0, slot0.data(), 4 * nb);
+    if (e == cudaSuccess) e = put((void **)&B.slice0, slice0.data(), 4 * nb);
+    if (e == cudaSuccess) e = put((void **)&B.off, off.data(), 4 * off.size());
+    if (e == cudaSuccess) e = put(&B.col, col.get(), 2 * ncol);
+    if (e == cudaSuccess) e = put((void **)&B.perm, perm.data(), 4 * perm.size());
+    if (e == cudaSuccess) e = cudaMalloc(&B.cb, sizeof(float) * 2 * std::max<int64_t>(J.n, 1));
+    if (e == cudaSuccess) e = put((void **)&B.rows, rows.data(), 4 * nb);   // last: the plan is complete
+    if (e == cudaErrorMemoryAllocation) {   // no room for the plan: another kernel
+        cudaGetLastError();
+        free_bres(B);
+        B.tried = true;
+        return SBX_OK;
+    }
+    CK(e);
     return SBX_OK;
 }
 
@@ -2030,6 +2037,11 @@ int solve_batch(sbx_ctx *ctx, int32_t count, sbx_problem *const *problems, const
             CK(cudaMemcpyAsync(cutv.data(), ctx->w.cut, sizeof(double) * nvals, cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(ctl, ctx->w.ctl, sizeof ctl, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        if (use_res && ctl[CTL_ERR] == kErrMisfit) {   // never expected: the whole batch again, this class without it
+            free_bres(bres);
+            bres.tried = true;
+            return solve_batch(ctx, count, problems, agents, pr, targets, res, agent_values, batch_time_us);
+        }
         if (ctl[CTL_ERR]) return fail(ctx, SBX_ERR_CUDA, "a bounded wait in the step kernel gave up");
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

@@ -110,7 +110,9 @@ struct DevCsr {
 };
 
 // Control words shared by the kernels of one solve.
-// CTL_ERR: a kernel gave up a bounded wait (set, never cleared by kernels).
+// CTL_ERR: a kernel gave up a bounded wait (1), or the on-chip batch kernel's
+// layout does not fit (kErrMisfit); set, never cleared by kernels.
+constexpr int kErrMisfit = 2;
 enum Ctl { CTL_STEP = 0, CTL_STOP = 1, CTL_WINDOWS = 2, CTL_NBIF = 3, CTL_TRACED = 4, CTL_ERR = 5, CTL_N = 8 };
 
 // One window of a traced solve: SB steps run, best cut over the agents of

@@ -55,6 +55,7 @@ struct BresP {
     int32_t *ctl;
     int32_t Ap, W, groups, nsteps;
     uint32_t smem;                       // bytes of dynamic shared memory
+    int32_t misfit;                      // test only: the layout is taken not to fit
 };
 
 // agents of a cluster: 64 bytes of x and y a row
@@ -282,11 +283,14 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
     const uint32_t pb = ((uint32_t)(R + 1) * RB + 15) & ~15u;   // bytes of a sign plane
     // chunks before, between and after the planes
     const uint32_t q0 = (kPlane - kFirst) / kChunk, q1 = (kPlane - pb) / kChunk, q2 = (P.smem - 2 * kPlane - pb) / kChunk;
-    // Never expected, the host leaves room: the layout does not fit.  The
-    // CTAs of a cluster agree before any of them leaves.
+    // Never expected: the layout does not fit.  It assumes that a CTA's shared
+    // window starts at a multiple of 16 MB and dynamic shared memory below
+    // kFirst in it, which no document promises.  The CTAs of a cluster agree
+    // before any of them leaves; the host then takes another kernel.
     __shared__ uint32_t s_bad;
     if (tid == 0)
-        s_bad = so > kFirst || pb > kPlane || 2 * kPlane + pb > P.smem || mine - kTmRows * (kNT / 32) > (int)(q0 + q1 + q2);
+        s_bad = P.misfit || so > kFirst || pb > kPlane || 2 * kPlane + pb > P.smem ||
+                mine - kTmRows * (kNT / 32) > (int)(q0 + q1 + q2);
     step_barrier<C>();
     uint32_t bad = 0;
     if (C == 1) bad = s_bad;
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
             bad |= v;
         }
     if (bad) {
-        if (tid == 0) atomicExch(&P.ctl[CTL_ERR], 1);
+        if (tid == 0) atomicExch(&P.ctl[CTL_ERR], kErrMisfit);
         step_barrier<C>();
         return;
     }
@@ -589,6 +593,7 @@ cudaError_t launch_batch_res(const SolveDims &d, const DevBres &B, bool allpos, 
     P.groups = (agents + ka - 1) / ka;   // groups of padded agents alone stay as they began
     P.nsteps = d.steps_run;
     P.smem = smem_bytes();
+    P.misfit = d.giveup;
     // the cluster sizes on streams of their own, largest first: the smaller
     // ones' CTAs fill the SMs that whole clusters leave
     cudaError_t e = cudaEventRecord(fork, s);
