@@ -628,11 +628,12 @@ int pick_tile(sbx_ctx *ctx, SolveDims &d, const DevCsr &J, const sbx_params *pr,
     }
     cudaStream_t s = ctx->stream;
     Work &w = ctx->w;
-    // Every candidate over an eighth of 2 ms of launches, then those within a
-    // quarter of the fastest over 2 ms, best of two rounds: most of the up to
-    // 24 candidates are far off, and timing all of them at length was most of
-    // a first solve (R-MAT 2^16 x 256, 1,000 steps: 176 ms, now 46; 20,000
-    // rows x 200 in FP32: 75, now 29; the same tiles chosen).
+    // Every candidate over an eighth of 2 ms of launches, then the four fastest
+    // of those within a quarter of the first over 2 ms, best of two rounds: most
+    // of the up to 40 candidates are far off, and timing all of them at length
+    // was most of a first solve (R-MAT 2^16 x 256, 1,000 steps: 176 ms, now 46;
+    // 20,000 rows of degree 8 x 608, FP64, where all are near: 70 ms with every
+    // near one, now 50).
     CK(launch_plain_steps(d, J, w, 1, s));
     CK(cudaEventRecord(ctx->ev0, s));
     CK(launch_plain_steps(d, J, w, 1, s));
@@ -643,9 +644,14 @@ int pick_tile(sbx_ctx *ctx, SolveDims &d, const DevCsr &J, const sbx_params *pr,
     const int reps = std::max(3, std::min(64, (int)(2.0 / std::max(one, 1e-3f))));
     std::vector<float> best(cands.size(), 1e30f);
     float least = 1e30f;
+    float limit = 1e30f;
     for (int round = 0; round < 3; round++) {
         const int count = round ? reps : std::max(3, reps / 8);
-        const float limit = round ? 1.25f * least : 1e30f;
+        if (round == 1) {
+            std::vector<float> sorted(best);
+            std::sort(sorted.begin(), sorted.end());
+            limit = std::min(1.25f * least, sorted[std::min<size_t>(3, sorted.size() - 1)]);
+        }
         for (size_t i = 0; i < cands.size(); i++) {
             if (round && best[i] > limit) continue;
             apply(cands[i]);
