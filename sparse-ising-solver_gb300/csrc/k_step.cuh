@@ -1142,12 +1142,12 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
     if (P.niso && !Q.order) return cudaErrorInvalidValue;
     // light rows by their records, where they end the row items: in the
     // heavy-row kernels, and in the others when they are at least half of the
-    // rows (20,000 rows of mean degree 8, 31% of them light, 128 agents: 10.5 us
-    // a step by records, 9.7 without; 30,000 of degree 3, nearly all light:
-    // 11.0 against 11.6)
+    // rows of a state past 12 MB (FP32, 128 agents, us a step by records and
+    // without: 30,000 rows of degree 3, nearly all light, 10.9 and 11.4; 6,000 of
+    // degree 2 4.44 and 4.12; 20,000 of degree 8, 31% light, 10.5 and 9.7)
     const bool stage = LR == 32 && !WIN && KIND != K_XY && !RAG && d.tst != 0 && J.unit;
     if (LR == 32 && KIND != K_XY && J.unit && J.light && Q.order && P.niso == J.niso && !stage &&
-        (big || 2 * (int64_t)J.nlight >= d.n - J.niso)) {
+        (big || (2 * (int64_t)J.nlight >= d.n - J.niso && 2.0 * sizeof(T) * d.n * d.Ap > 12e6))) {
         Q.light = J.light;
         Q.nlight = J.nlight;
     }

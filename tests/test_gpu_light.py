@@ -43,10 +43,11 @@ def test_segments_of_light_rows(ctx, prec, lanes, n, segments):
 @pytest.mark.parametrize("prec", [sbx.F64, sbx.F32, sbx.F16])
 @pytest.mark.parametrize("degree", [1.0, 3.0, 6.5, 9.0])
 @pytest.mark.parametrize("fused", [1, 0])
-@pytest.mark.parametrize("agents", [32, 256, 300])
+@pytest.mark.parametrize("agents", [32, 256, 300, 1536])
 def test_records_by_the_share_of_light_rows(ctx, prec, degree, fused, agents):
     # no heavy row: records where at least half of the rows are light (here up
-    # to a mean degree of about 6.5), the row pointers otherwise
+    # to a mean degree of about 6.5) in a state past 12 MB, the row pointers
+    # otherwise
     g = sbx.gen_er(2500, degree / 2499, pm1=True, seed=int(10 * degree))
     prob = ctx.problem(g)
     base = dict(dt=0.5, steps=2000, run_steps=200, agents=agents, seed=5, precision=prec, fused=fused,
