@@ -345,22 +345,25 @@ __device__ __forceinline__ void count_bits_s(const StepP &P, const uint32_t *Sq,
     const uint32_t *cwp = P.colw + e0 + sl;   // this lane's column words, from one base
     // past a row's end: the zero row (word 0, weight sign clear), so those
     // terms vanish without a test per word
-    auto columns = [&](int32_t cb, uint32_t (&cw)[T]) {
-#pragma unroll
-        for (int t = 0; t < T; t++) cw[t] = cb + t * LR + sl < dw ? __ldg(cwp + cb + t * LR) : P.zrow;
-    };
     uint32_t nextcw[T];
-    if (AHEAD) columns(0, nextcw);
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int t = 0; t < T; t++) nextcw[t] = t * LR + sl < dw ? __ldg(cwp + t * LR) : P.zrow;
+    }
     for (int32_t cb = 0; cb < dmax; cb += 32) {
         uint32_t mycw[T];
-        if (AHEAD) {
-            // the next block's column words are on their way while this one's
-            // sign words are gathered
 #pragma unroll
-            for (int t = 0; t < T; t++) mycw[t] = nextcw[t];
-            columns(cb + 32, nextcw);
-        } else {
-            columns(cb, mycw);
+        for (int t = 0; t < T; t++) {
+            if constexpr (AHEAD) {
+                // the next block's column words are on their way while this
+                // one's sign words are gathered
+                mycw[t] = nextcw[t];
+                const int32_t idx = cb + 32 + t * LR + sl;
+                nextcw[t] = idx < dw ? __ldg(cwp + cb + 32 + t * LR) : P.zrow;
+            } else {
+                const int32_t idx = cb + t * LR + sl;
+                mycw[t] = idx < dw ? __ldg(cwp + cb + t * LR) : P.zrow;
+            }
         }
         uint32_t w[T * KPL];
 #pragma unroll
@@ -676,10 +679,11 @@ template <int V> __device__ __forceinline__ uint32_t sign_bits16(const uint32_t 
 // registers), 5 otherwise (heavy-row kernels: 6 spilled more and ran 2%
 // slower on R-MAT 2^20, 7 ran 11% slower).
 // RAG: the lanes of a row's last segment hold more agents than the row has.
-// LT: light rows are walked by their records; a variant of its own because
-// their loop costs the others registers (FP32, four agents a lane, bit planes:
-// 64 against 56, 5 to 10% of a step at degree 12 to 24).
-template <class T, int V, int KIND, bool WIN, int WM, bool BIG, int LR, int CM, int ST, bool RAG, bool LT>
+// LT: light rows are walked by their records, whole rows a warp (1) or single
+// segments (2); variants of their own because the loop costs the others
+// registers (FP32, four agents a lane, bit planes: 64 against 56, 5 to 10% of a
+// step at degree 12 to 24), and choosing the walk in it 1 to 2% of R-MAT's.
+template <class T, int V, int KIND, bool WIN, int WM, bool BIG, int LR, int CM, int ST, bool RAG, int LT>
 __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P, const int offset)
 {
     static_assert(LR == 32 || !BIG, "heavy rows are counted by whole warps");
@@ -838,44 +842,38 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
     };
 
     // Light rows (at most kLight neighbours): one record of eight words a row
-    // -- row, degree, columns -- loaded two items ahead and its x, y one ahead,
-    // so that a row's state and all its sign words are requested at once.
-    // Through the order, the row pointers and the columns it is four dependent
-    // loads, and rows of two neighbours (most of R-MAT's) took three times
-    // their bytes' time.  An item is a segment of a row, as below (whole rows a
-    // warp left a small graph's many segments to as few warps as it has light
-    // rows: a star of 300 rows at 1,024 agents, FP64, 22.6 us a step).
+    // -- row, degree, columns -- loaded an item ahead, so that a row's x, y and
+    // all its sign words are requested at once.  Through the order, the row
+    // pointers and the columns it is four dependent loads, and rows of two
+    // neighbours (most of R-MAT's) took three times their bytes' time.  A warp
+    // takes whole rows, or single segments when there are few rows for the warps
+    // (a star of 300 rows at 1,024 agents, FP64: 8.5 us a step, by rows 22.6).
     if constexpr (LT) {
         // from the last warp down: the row items' remainder is the first warps'
-        const int32_t nl = P.nlight, dg = (int32_t)(nw / nit), di = (int32_t)nw - dg * nit;
-        int32_t g = (int32_t)(nw - 1 - w0) / nit, it = (int32_t)(nw - 1 - w0) - g * nit;
-        auto advance = [&](int32_t &gg, int32_t &ii) {
-            gg += dg;
-            ii += di;
-            if (ii >= nit) {
-                ii -= nit;
-                gg++;
-            }
+        const int32_t nw32 = (int32_t)nw;
+        constexpr bool split = LT == 2;
+        const int32_t nl = split ? P.nlight * nit : P.nlight;
+        auto record = [&](int32_t i) {
+            return i < nl ? __ldg(&P.light[(int64_t)(split ? i / nit : i) * 8 + (lane & 7)]) : 0u;
         };
-        auto record = [&](int32_t i) { return i < nl ? __ldg(&P.light[(int64_t)i * 8 + (lane & 7)]) : 0u; };
-        // x, y of segment i of a record's row
+        auto first = [&](int32_t i) -> int { return split ? i % nit : 0; };   // the item's first segment
+        // x, y of segment i of a record's row, one item ahead of their use
         auto state = [&](uint32_t rec, int i, RawT &xr, RawT &yr) {
             const int a1 = i * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
             const int64_t base = (int64_t)__shfl_sync(FULL, rec, 0) * P.Ap + a0;
             xr = vload_s<T, V>(xp + base, cs);
             yr = vload_s<T, V>(yp + base, cs);
         };
-        int32_t g1 = g, it1 = it;
-        advance(g1, it1);
-        uint32_t rec = record(g), rec1 = record(g1);
+        int32_t g = (int32_t)(nw - 1 - w0), it = first(g);
+        uint32_t rec = record(g), rec1 = record(g + nw32), rec2;
         RawT xr, yr;
         if (g < nl) state(rec, it, xr, yr);
         while (g < nl) {
-            int32_t g2 = g1, it2 = it1;
-            advance(g2, it2);
-            const uint32_t rec2 = record(g2);
+            const bool end = split || it + 1 == nit;   // warp-uniform
+            const bool more = !end || g + nw32 < nl;
+            if (end) rec2 = record(g + 2 * nw32);
             RawT xn = xr, yn = yr;
-            if (g1 < nl) state(rec1, it1, xn, yn);
+            if (more) state(end ? rec1 : rec, end ? first(g + nw32) : it + 1, xn, yn);
             const int32_t r = (int32_t)__shfl_sync(FULL, rec, 0), deg = (int32_t)__shfl_sync(FULL, rec, 1);
             const int a1 = it * 32 * V + lane * V, a0 = RAG ? min(a1, P.Ap - V) : a1;
             const int q = a0 >> 5, off = a0 & 31;
@@ -901,12 +899,14 @@ __global__ void __launch_bounds__(256, (CM && !BIG) ? 4 : 5) k_row(const StepP P
             finish(r, q, off, base, !RAG || a1 == a0, xr, yr, tv, row_c0(r), wp_old);
             xr = xn;
             yr = yn;
-            rec = rec1;
-            rec1 = rec2;
-            g = g1;
-            it = it1;
-            g1 = g2;
-            it1 = it2;
+            if (end) {
+                g += nw32;
+                rec = rec1;
+                rec1 = rec2;
+                it = first(g);
+            } else {
+                it++;
+            }
         }
     }
 
@@ -1141,13 +1141,16 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
     // isolated rows (P.niso, left to k_iso) are the end of the degree order
     if (P.niso && !Q.order) return cudaErrorInvalidValue;
     // light rows by their records, where they end the row items: in the
-    // heavy-row kernels, and in the others when they are at least half of the
-    // rows of a state past 12 MB (FP32, 128 agents, us a step by records and
-    // without: 30,000 rows of degree 3, nearly all light, 10.9 and 11.4; 6,000 of
-    // degree 2 4.44 and 4.12; 20,000 of degree 8, 31% light, 10.5 and 9.7)
+    // heavy-row kernels -- by segments when they are few for the GPU's warps
+    // (five CTAs of eight an SM) -- and in the others when they are enough, at
+    // least half of the rows, and of a state past 12 MB (FP32, 128 agents, us a
+    // step by records and without: 30,000 rows of degree 3, nearly all light, 10.9
+    // and 11.4; 6,000 of degree 2 4.44 and 4.12; 20,000 of degree 8, 31% light,
+    // 10.5 and 9.7)
     const bool stage = LR == 32 && !WIN && KIND != K_XY && !RAG && d.tst != 0 && J.unit;
+    const bool split = nit > 1 && J.nlight < 4 * 40 * std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
     if (LR == 32 && KIND != K_XY && J.unit && J.light && Q.order && P.niso == J.niso && !stage &&
-        (big || (2 * (int64_t)J.nlight >= d.n - J.niso && 2.0 * sizeof(T) * d.n * d.Ap > 12e6))) {
+        (big || (!split && 2 * (int64_t)J.nlight >= d.n - J.niso && 2.0 * sizeof(T) * d.n * d.Ap > 12e6))) {
         Q.light = J.light;
         Q.nlight = J.nlight;
     }
@@ -1164,38 +1167,44 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
         if (big) {
             if constexpr (can_st) {
                 if (st) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 1, false, 0>, d, items, bt, smem_st, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1, false, 0>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
-            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG, KIND != K_XY>, d, items, bt, smem, s, Q, offset);
-            return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, RAG, KIND != K_XY>, d, items, bt, smem, s, Q, offset);
+            if constexpr (KIND != K_XY && !RAG)
+                if (!split) {
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, false, 1>, d, items, bt, smem, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, false, 1>, d, items, bt, smem, s, Q, offset);
+                }
+            constexpr int lt = KIND != K_XY ? 2 : 0;
+            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG, lt>, d, items, bt, smem, s, Q, offset);
+            return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, RAG, lt>, d, items, bt, smem, s, Q, offset);
         }
     } else {
         if (big) return cudaErrorInvalidValue;
     }
-    if (KIND == K_XY) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
+    if (KIND == K_XY) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG, 0>, d, items, bt, smem, s, Q, offset);
     if (J.unit) {
         if constexpr (KIND != K_XY) {
             if constexpr (can_st) {
                 if (st) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 1, false, false>, d, items, bt, smem_st, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 1, false, 0>, d, items, bt, smem_st, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 1, false, 0>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
             if constexpr (LR == 32)
                 if (Q.nlight) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, 32, 1, 0, RAG, true>, d, items, bt, smem, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, 32, 0, 0, RAG, true>, d, items, bt, smem, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, 32, 1, 0, RAG, 1>, d, items, bt, smem, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, 32, 0, 0, RAG, 1>, d, items, bt, smem, s, Q, offset);
                 }
-            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
+            if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 1, 0, RAG, 0>, d, items, bt, smem, s, Q, offset);
         }
-        return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, false, LR, 0, 0, RAG, 0>, d, items, bt, smem, s, Q, offset);
     }
     if constexpr (sizeof(T) == 8)
-        return launch_grid(k_row<T, V, KIND, WIN, W_F64, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_F64, false, LR, 0, 0, RAG, 0>, d, items, bt, smem, s, Q, offset);
     else
-        return launch_grid(k_row<T, V, KIND, WIN, W_F32, false, LR, 0, 0, RAG, false>, d, items, bt, smem, s, Q, offset);
+        return launch_grid(k_row<T, V, KIND, WIN, W_F32, false, LR, 0, 0, RAG, 0>, d, items, bt, smem, s, Q, offset);
 }
 
 template <class T, int V, int LR, int KIND, bool WIN>
