@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "engine.h"
 
+#include <algorithm>
 #include <cstring>
 
 namespace sbx {
@@ -240,8 +241,9 @@ cudaError_t launch_t(void *x, void *y, int32_t Ap, int tsp, int64_t L, int shift
 // serial FP64 divisions.
 int rand_chunk_shift(int64_t outputs)
 {
+    const int64_t fill = 640 * (int64_t)std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
     int s = 6;
-    while (s > 0 && (outputs / kRound >> s) < 152 * 640) s--;
+    while (s > 0 && (outputs / kRound >> s) < fill) s--;
     return s;
 }
 int64_t rand_round() { return kRound; }
