@@ -48,8 +48,8 @@ enum { SBX_F32 = 0, SBX_BF16 = 1, SBX_F16 = 2, SBX_F64 = 3 };
  * 8 agents per CTA split between tensor memory and shared memory, for graphs
  * too large for the former (AUTO also takes it for FP32 state, 4 agents).  For
  * batches, RESIDENT and RESIDENT_SPLIT ask for the resident batch kernel; AUTO
- * may take the on-chip one, which a result shows as staging 3.  TENSOR (TSP, 16-bit state, 3 <= N <= 32) is the
- * resident TSP kernel with the distance product on the tensor cores
+ * may take the on-chip one, which a result shows as staging 3.  TENSOR (TSP,
+ * 16-bit state, 3 <= N <= 32) is the resident TSP kernel with the distance product on the tensor cores
  * (tcgen05): AUTO's choice for BF16 and FP16 TSP states that fit it. */
 enum { SBX_KERNEL_AUTO = 0, SBX_KERNEL_STREAM = 1, SBX_KERNEL_RESIDENT = 2, SBX_KERNEL_RESIDENT_SPLIT = 3,
        SBX_KERNEL_TENSOR = 4 };
@@ -93,8 +93,12 @@ typedef struct sbx_params {
      * tile computes identical results. */
     int32_t lane_agents;    /* agents per lane: 1, 2, 4 or 8 (16-bit states) */
     int32_t row_lanes;      /* lanes per row: 32, or 16/8/4 (several rows per
-                               warp; then lane_agents * row_lanes = padded agents).
-                               With 32 the last lanes of a row may hold no agents */
+                               warp).  A tile asked for by lane_agents or
+                               row_lanes holds the padded agents exactly: 32 *
+                               lane_agents divides them, or lane_agents *
+                               row_lanes are they.  The autotuner may also leave
+                               a row's last lanes without agents; a result that
+                               shows such a tile cannot be asked for */
     int32_t block_threads;  /* threads per CTA: 128 or 256 */
     int32_t count_mode;     /* +-1 weights: 1 byte counters per lane, 2 bit
                                planes per sign word (neighbours split across
@@ -125,13 +129,21 @@ typedef struct sbx_result {
     int64_t bifurcated;     /* agents whose bifurcated flag is set */
     int64_t valid;          /* TSP: agents holding a valid tour */
     int32_t best_agent;     /* first agent reaching max (MaxCut) / min (TSP) */
-    int32_t kernel_used;    /* the SBX_KERNEL_* that ran */
+    int32_t kernel_used;    /* the SBX_KERNEL_* family that ran.  AUTO's forms
+                               of a family are not all to be asked for: FP64
+                               RESIDENT and FP32 RESIDENT_SPLIT are refused.  The
+                               on-chip batch kernel, which has no family of its
+                               own, is known by staging 3; kernel_used is then
+                               RESIDENT for a class of mean degree <= 8 and
+                               STREAM above, as batches of that degree have
+                               always reported */
     int32_t agents_per_block;
     int32_t lane_agents;    /* streaming tile used (0 for other kernels; the
                                on-chip batch kernel: agents of a cluster) */
     int32_t row_lanes;
     int32_t block_threads;
-    int32_t count_mode;     /* as above; the batch kernels report 4 */
+    int32_t count_mode;     /* as above; the plane and the on-chip batch kernel
+                               report 4 (asked for, it selects the former) */
     int32_t staging;        /* as above; 3: a batch's state stayed on chip for
                                the whole solve */
     double kernel_ms;       /* SBX_FLAG_PROFILE: summed hot-kernel time */

@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(kNT, 1) k_batch_res(const BresP P)
     }
     T *xg = (T *)P.x, *yg = (T *)P.y;
 
-    // All of the SM's tensor memory: 1,024 threads of 64 registers leave room
-    // for no second CTA that would wait for it.
+    // All of the SM's tensor memory: 1,024 threads of 55 registers and more
+    // leave room for no second CTA that would wait for it.
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
                      "r"(512u));

@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(kNT, 1) k_resident_rs(const RsP P)
         return;
     }
 
-    // All of the SM's tensor memory: 1,024 threads of 64 registers leave room
-    // for no second CTA that would wait for it.
+    // All of the SM's tensor memory: 1,024 threads of 55 registers and more
+    // leave room for no second CTA that would wait for it.
     const int warp = tid >> 5;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),

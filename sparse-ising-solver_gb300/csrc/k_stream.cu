@@ -170,10 +170,10 @@ StepP make_step(const SolveDims &d, const DevCsr &J, Work &w)
     P.allpos = J.allpos ? 1 : 0;
     P.bits_min = d.tcm == 2 ? kBitsMin : INT32_MAX;
     P.niso = 0;
-    P.light = nullptr;   // set per kernel (step_vl)
+    P.light = nullptr;   // set per kernel (step_vlr)
     P.nlight = 0;
     P.nchunks = J.nchunks;
-    P.order = nullptr;   // set per kernel (step_vl)
+    P.order = nullptr;   // set per kernel (step_vlr)
     P.row0 = 0;
     P.c0r32 = J.c0r32;
     P.c0r64 = J.c0r64;

@@ -10,8 +10,8 @@
 // Options after the positional arguments (all optional):
 //   --seed=N         srand seed (default: time(0), as the reference)
 //   --precision=P    f32 (default) | bf16 | f16 | f64
-//   --kernel=K       auto (default) | stream | resident | split (registers +
-//                    shared memory, 16-bit fused state) | tensor (TSP, 16-bit
+//   --kernel=K       auto (default) | stream | resident | split (tensor memory
+//                    + shared memory, 16-bit fused state) | tensor (TSP, 16-bit
 //                    state: the distance product on the tensor cores)
 //   --period=N       steps per window (default: the reference's)
 //   --device=N       CUDA device (default 0)
