@@ -80,19 +80,27 @@ def restart_copies(rows_missed, rows_total):
 # (the command is in the source string); the resident kernels' launch covers
 # the whole solve.
 TRAFFIC = {
-    "torus": (43.17e6, "ncu -k regex:k_resident_rs -c 1: bench.py --workload torus "
+    "torus": (43.17e6, "ncu --clock-control none -k regex:k_resident_rs -c 1: bench.py --workload torus "
                        "--profile 2000 --kernel split (one 2,000-step launch)"),
     # per SB step: the k_row launch plus 1/100 of the isolated rows' k_iso
-    "rmat20": (9.792e8, "ncu -k regex:k_row|k_iso: bench.py --workload rmat20 "
+    "rmat20": (9.792e8, "ncu --clock-control none -k regex:k_row|k_iso: bench.py --workload rmat20 "
                         "--profile 100 (k_row launch + k_iso / 100)"),
-    # the state is read and written once a solve: per step of a solve of 100
-    "batch512": (8.80e6, "ncu -k regex:k_batch_res -c 4: bench.py --workload batch512 "
-                         "--profile 100 (the four launches / 100 steps)"),
+    # the state is read and written once a solve, whatever its steps: the four
+    # launches' 880 MB, per launch
+    "batch512": (2.20e8, "ncu --clock-control none -k regex:k_batch_res -c 4: bench.py --workload batch512 "
+                         "--profile 100 (mean of the four launches of a solve)"),
     # the whole 2,000-step solve is one launch; per launch of the bench's
     # 20,000-step solve the state read once is the same
-    "tsp30": (3.870e6, "ncu --set full -k regex:k_tsp_tc -c 1: bench.py --workload tsp30 "
+    "tsp30": (3.870e6, "ncu --set full --clock-control none -k regex:k_tsp_tc -c 1: bench.py --workload tsp30 "
                        "--profile 2000 --kernel tensor --precision bf16 (one launch)"),
 }
+
+
+def on_chip(roof, step_us):
+    """A kernel whose state stays on chip is bound by issue, not by HBM: its
+    algorithmic bytes per second are no fraction of a roofline, only what a
+    kernel that streams the state would have to move."""
+    roof.update(bound="issue", effective_hbm_frac=roof["frac"], frac=None, step_us=step_us)
 
 
 def load_peaks():
@@ -693,6 +701,8 @@ def main():
                     "traffic_source": tr[1] if tr else None, "peak_kind": peak_kind,
                     "kernel": kname, "bytes_per_launch": bytes_per_launch,
                     "launch_us": per_launch_s * 1e6, "launches": rp["kernel_launches"]}
+            if rp["kernel_used"] != sbx.KERNEL_STREAM:
+                on_chip(roof, per_launch_s * 1e6 * rp["kernel_launches"] / rp["steps_run"])
 
     ref_gpu = None
     if rank == 0 and world == 1 and wl["kind"] == "tsp":
@@ -963,11 +973,15 @@ def run_batch(args, wl, rank, world, local):
         roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": tr[0] if tr else None,
                 "traffic_source": tr[1] if tr else None, "peak_kind": peak_kind,
-                "kernel": ("k_batch_res (the whole solve in up to four launches; state on chip, "
-                           "effective bytes of one SB step)") if rp[0]["staging"] == 3 else
-                          "step kernel, one launch per SB step over all instances",
+                "kernel": "step kernel, one launch per SB step over all instances",
                 "bytes_per_launch": b_step, "launch_us": per_launch_s * 1e6,
                 "launches": rp[0]["kernel_launches"]}
+        if rp[0]["staging"] == 3:   # the whole solve in up to four launches
+            per = rp[0]["steps_run"] / rp[0]["kernel_launches"]
+            roof.update(kernel="k_batch_res (the whole solve in up to four launches side by side; state on "
+                               "chip, effective bytes)",
+                        bytes_per_launch=b_step * per, launch_us=per_launch_s * 1e6 * per)
+            on_chip(roof, per_launch_s * 1e6)
     # the same instances in FP16 state, and in FP32 from other seeds (the
     # seed-to-seed spread of the best cut that any other trajectory shows)
     spread = {}
