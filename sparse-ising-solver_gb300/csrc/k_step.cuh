@@ -1141,14 +1141,15 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
     // isolated rows (P.niso, left to k_iso) are the end of the degree order
     if (P.niso && !Q.order) return cudaErrorInvalidValue;
     // light rows by their records, where they end the row items: in the
-    // heavy-row kernels -- by segments when they are few for the GPU's warps
-    // (five CTAs of eight an SM) -- and in the others when they are enough, at
+    // heavy-row kernels -- by segments when they are fewer than the GPU's warps
+    // (five CTAs of eight an SM; R-MAT 2^14 at 200 agents, FP32: 11.8 us a step
+    // by rows, 12.4 by segments) -- and in the others when they are enough, at
     // least half of the rows, and of a state past 12 MB (FP32, 128 agents, us a
     // step by records and without: 30,000 rows of degree 3, nearly all light, 10.9
     // and 11.4; 6,000 of degree 2 4.44 and 4.12; 20,000 of degree 8, 31% light,
     // 10.5 and 9.7)
     const bool stage = LR == 32 && !WIN && KIND != K_XY && !RAG && d.tst != 0 && J.unit;
-    const bool split = nit > 1 && J.nlight < 4 * 40 * std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
+    const bool split = nit > 1 && J.nlight < 40 * std::max(1, dev_attr(cudaDevAttrMultiProcessorCount));
     if (LR == 32 && KIND != K_XY && J.unit && J.light && Q.order && P.niso == J.niso && !stage &&
         (big || (!split && 2 * (int64_t)J.nlight >= d.n - J.niso && 2.0 * sizeof(T) * d.n * d.Ap > 12e6))) {
         Q.light = J.light;
@@ -1171,10 +1172,10 @@ cudaError_t step_vlr(const SolveDims &d, const DevCsr &J, const StepP &P, int of
                     return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 1, false, 0>, d, items, bt, smem_st, s, Q, offset);
                 }
             }
-            if constexpr (KIND != K_XY && !RAG)
+            if constexpr (KIND != K_XY)
                 if (!split) {
-                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, false, 1>, d, items, bt, smem, s, Q, offset);
-                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, false, 1>, d, items, bt, smem, s, Q, offset);
+                    if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG, 1>, d, items, bt, smem, s, Q, offset);
+                    return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 0, 0, RAG, 1>, d, items, bt, smem, s, Q, offset);
                 }
             constexpr int lt = KIND != K_XY ? 2 : 0;
             if (cm) return launch_grid(k_row<T, V, KIND, WIN, W_UNIT, true, 32, 1, 0, RAG, lt>, d, items, bt, smem, s, Q, offset);
